@@ -268,13 +268,38 @@ int pick_kmax(SweepParams& p) {
     return 8;
 }
 
-int auto_plane_chunks(int tiles, int nplanes) {
-    const int target = num_sms() * 6;         // ~3 waves of 2 resident CTAs per SM
-    if (tiles >= target || nplanes < 8) return 1;
-    int c = (target + tiles - 1) / tiles;
-    const int maxc = nplanes / 4;             // keep >= 4 planes per chunk
-    if (c > maxc) c = maxc;
-    return c < 1 ? 1 : c;
+// CTAs of a tile shape that fit on one SM together: the kernels' launch bounds, and the shared
+// memory of Geom<r, th> (228 KB per SM, 1 KB of it reserved per CTA).
+static int resident_ctas(int r, int th) {
+    const size_t JP = TW + 2 * ((r + 3) & ~3) + 4, HR = th + 2 * r;
+    const size_t smem = HR * JP * 8 + HR * TW * 16 + (size_t)6 * th * TW * 4 + sizeof(Coef) * MVS_MAX_SOURCES + 1024;
+    const int fit = (int)((size_t)228 * 1024 / smem), bound = th == 16 ? 3 : (th == 32 ? 2 : 1);
+    return fit < 1 ? 1 : (fit < bound ? fit : bound);
+}
+
+// Plane chunks of a launch: `tiles` x chunks CTAs of about equal work run `slots` at a time, so the
+// launch takes ceil(tiles chunks / slots) rounds of (planes per chunk + overhead). The overhead of
+// a chunk - the tile's set-up, its record's write and the merge's read of it - measures about half
+// a plane of work. Of equal estimates the fewest chunks. (640 x 480, 4 sources, 128 planes: the
+// fixed rule of ~900 CTAs gave 6 chunks of 22 planes in 4 rounds = 88 planes where 65 are the even
+// share; 13 chunks of 10 planes take 7 rounds = 70.) Launches of many rounds keep one chunk: there
+// the rounds blur and records of large images cost more than the last round's idle SMs.
+int auto_plane_chunks(int tiles, int nplanes, int slots) {
+    if (tiles < 1 || nplanes < 2 || tiles >= 6 * slots) return 1;
+    int best = 1;
+    double cost = 0.0;
+    for (int c = 1; c <= nplanes; ++c) {
+        const int ppc = (nplanes + c - 1) / c, used = (nplanes + ppc - 1) / ppc;
+        if (used != c) continue;
+        const long long rounds = ((long long)tiles * c + slots - 1) / slots;
+        const double t = (double)rounds * (ppc + (c > 1 ? 0.5 : 0.0));
+        if (c == 1 || t < cost) {
+            best = c;
+            cost = t;
+        }
+        if (rounds > 16) break;
+    }
+    return best;
 }
 
 mvs_status sweep_range(const mvs_sweep_args* a, int i0, int i1, float* rec_ws, int nchunks, cudaStream_t st) {
@@ -315,7 +340,8 @@ size_t sweep_scratch_bytes(const mvs_sweep_args* a, int* nchunks_out) {
     const int tiles = ((a->W + TW - 1) / TW) * ((a->H + th - 1) / th);
     const int nplanes = a->i1 - a->i0;
     const int per_call = nplanes < MVS_MAX_PLANES_PER_CALL ? nplanes : MVS_MAX_PLANES_PER_CALL;
-    int nch = a->plane_chunks > 0 ? a->plane_chunks : auto_plane_chunks(tiles, per_call);
+    int nch = a->plane_chunks > 0 ? a->plane_chunks
+                                 : auto_plane_chunks(tiles, per_call, num_sms() * resident_ctas(a->r, th));
     if (nch > per_call) nch = per_call < 1 ? 1 : per_call;
     *nchunks_out = nch;
     if (nch <= 1) return 0;

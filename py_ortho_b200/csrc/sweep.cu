@@ -99,7 +99,7 @@ __global__ void finalize_kernel(int H, int W, int kind, int n, int t0, const flo
 template <int R, int KMAX, bool PLANES, bool F16, bool X64, bool CMP, int TH>
 static mvs_status launch_sweep(const SweepParams& p, dim3 grid, cudaStream_t st) {
     auto kern = sweep_kernel<R, KMAX, PLANES, F16, X64, CMP, TH>;
-    const size_t smem = Geom<R, TH>::smem_bytes() + (CMP ? Geom<R, TH>::count_bytes() : 0);
+    const size_t smem = Geom<R, TH>::smem_bytes(WinnerState<R, KMAX, TH>::PLANES) + (CMP ? Geom<R, TH>::count_bytes() : 0);
     // the attribute is per function and per device: set it for the current device every time
     MVS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
              "sweep: shared memory attribute");
@@ -270,9 +270,10 @@ int pick_kmax(SweepParams& p) {
 
 // CTAs of a tile shape that fit on one SM together: the kernels' launch bounds, and the shared
 // memory of Geom<r, th> (228 KB per SM, 1 KB of it reserved per CTA).
-static int resident_ctas(int r, int th) {
+static int resident_ctas(int r, int th, int kk) {
     const size_t JP = TW + 2 * ((r + 3) & ~3) + 4, HR = th + 2 * r;
-    const size_t smem = HR * JP * 8 + HR * TW * 16 + (size_t)6 * th * TW * 4 + sizeof(Coef) * MVS_MAX_SOURCES + 1024;
+    const size_t smem = HR * JP * 8 + HR * TW * 16 + (size_t)(th == TH_DEFAULT && kk <= 2 && (r == 4 || r == 5) ? 5 : 6) * th * TW * 4 +
+                        sizeof(Coef) * MVS_MAX_SOURCES + 1024;
     const int fit = (int)((size_t)228 * 1024 / smem), bound = th == 16 ? 3 : (th == 32 ? 2 : 1);
     return fit < 1 ? 1 : (fit < bound ? fit : bound);
 }
@@ -341,7 +342,7 @@ size_t sweep_scratch_bytes(const mvs_sweep_args* a, int* nchunks_out) {
     const int nplanes = a->i1 - a->i0;
     const int per_call = nplanes < MVS_MAX_PLANES_PER_CALL ? nplanes : MVS_MAX_PLANES_PER_CALL;
     int nch = a->plane_chunks > 0 ? a->plane_chunks
-                                 : auto_plane_chunks(tiles, per_call, num_sms() * resident_ctas(a->r, th));
+                                 : auto_plane_chunks(tiles, per_call, num_sms() * resident_ctas(a->r, th, a->top_k));
     if (nch > per_call) nch = per_call < 1 ? 1 : per_call;
     *nchunks_out = nch;
     if (nch <= 1) return 0;

@@ -112,10 +112,21 @@ struct Geom {
     static constexpr size_t count_bytes() {      // compensated mode: uint8 horizontal window counts
         return ((size_t)HR * TW + 15) & ~(size_t)15;
     }
-    static constexpr size_t smem_bytes() {       // sJ, sI, sH, winner state (6 planes), sC
-        return (size_t)HR * JP * 4 * 2 + (size_t)HR * TW * 16 + (size_t)6 * TH * TW * 4 +
+    static constexpr size_t smem_bytes(int winner_planes = 6) {       // sJ, sI, sH, winner state, sC
+        return (size_t)HR * JP * 4 * 2 + (size_t)HR * TW * 16 + (size_t)winner_planes * TH * TW * 4 +
                sizeof(Coef) * MVS_MAX_SOURCES;
     }
+};
+
+// Planes of the winner state in shared memory: best, prev, s_prev_best, s_next_best, idx and, unless
+// FIRST_TO_REC, a chunk record's first score, which then goes to the record when it is formed. At
+// R = 4 and 5 leaving that plane out lets two CTAs share an SM (1003 x 749, R = 5, float64 sums: 8.0
+// -> 6.7 ms); elsewhere it changes no occupancy, and the store inside the loop costs registers
+// (R = 3: 101.9 -> 114.6 ms).
+template <int R, int KMAX, int TH>
+struct WinnerState {
+    static constexpr bool FIRST_TO_REC = TH == TH_DEFAULT && KMAX == 2 && (R == 4 || R == 5);
+    static constexpr int PLANES = FIRST_TO_REC ? 5 : 6;
 };
 
 // Largest shared-memory footprint over radii 0..RMAX (a persistent CTA serves any of them).
@@ -231,31 +242,147 @@ __device__ __forceinline__ float sample_plane_inside(const Coef& c, const void* 
     return fmaf(val, 0.0f, val);   // finite: val; inf: NaN; NaN: NaN
 }
 
-// Ray path sample: per-pixel inverse depth and world ray, FP64 projection with radial
-// distortion and FP64 bilinear, as _sweep.h:49-80.
-__device__ __forceinline__ float sample_ray(const SweepParams& p, const SrcGeo& g, int i, int gx, int gy) {
-    const float inv = hyp_value(p, i, gx, gy);
-    const long long HW = (long long)p.H * p.W, o = (long long)gy * p.W + gx;
-    const double d = 1.0 / (double)inv;
-    const double rx = __ldg(p.ray + o), ry = __ldg(p.ray + HW + o), rz = __ldg(p.ray + 2 * HW + o);
-    const double X = g.b[0] + d * ((g.m[0] * rx + g.m[1] * ry) + g.m[2] * rz);
-    const double Y = g.b[1] + d * ((g.m[3] * rx + g.m[4] * ry) + g.m[5] * rz);
-    const double Z = g.b[2] + d * ((g.m[6] * rx + g.m[7] * ry) + g.m[8] * rz);
-    if (!(Z > 1e-6)) return qnan();
-    const double nx = X / Z, ny = Y / Z;
-    const double r2 = nx * nx + ny * ny;
-    const double dd = g.f * (1.0 + r2 * (g.k1 + r2 * (g.k2 + r2 * g.k3)));
-    const double u = dd * nx + g.cx, v = dd * ny + g.cy;
-    // NaN u / v (NaN hypotheses) count as invalid; the reference leaves them undefined
-    if (!(u >= 0.0 && v >= 0.0 && u <= (double)g.w - 1.001 && v <= (double)g.h - 1.001)) return qnan();
-    const int x0 = (int)u, y0 = (int)v;
-    const double fx = u - (double)x0, fy = v - (double)y0;
-    const long long so = (long long)y0 * g.w + x0;
-    MVS_BOUND(so >= 0 && so + g.w + 1 < (long long)g.h * g.w);
-    const double a00 = tap<false>(g.img, so), a01 = tap<false>(g.img, so + 1);
-    const double a10 = tap<false>(g.img, so + g.w), a11 = tap<false>(g.img, so + g.w + 1);
-    const double val = (a00 * (1.0 - fx) + a01 * fx) * (1.0 - fy) + (a10 * (1.0 - fx) + a11 * fx) * fy;
-    return isfinite(val) ? (float)val : qnan();
+// ---- ray path: per-pixel inverse depth and world ray, FP64 projection with radial distortion and
+// FP64 bilinear (_sweep.h:49-80). The reference's point is X = b + (1 / inv) R ray; only its ratios
+// enter, so it is formed times inv, X = inv b + R ray, with no reciprocal of the depth, and x / z and
+// y / z share one reciprocal of z. What bounds it on an SM is the FP64 pipe (64 lanes a clock, ~40
+// operations a sample) and the conversion unit (16 lanes a clock: 3 ray components, 4 taps, the
+// inverse depth and the result), so the integer tap position comes from an addition rounded toward
+// -inf instead of two conversions, and the bounds are compared as integers.
+
+// 1 / z by two Newton-Raphson steps on the hardware's approximation (relative error ~2^-20 ->
+// 2^-40 -> the last bit or so). 0, inf and NaN give NaN.
+__device__ __forceinline__ double rcp_newton(double z) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));
+    double e = __fma_rn(-z, r, 1.0);
+    r = __fma_rn(r, e, r);
+    e = __fma_rn(-z, r, 1.0);
+    return __fma_rn(r, e, r);
+}
+
+// The source position of one sample: offset of the top-left tap (0 when invalid) and the fractions.
+struct RayTap {
+    double fx, fy;
+    long long o;
+    bool ok;
+};
+
+template <bool PINHOLE>
+__device__ __forceinline__ RayTap ray_tap(const SrcGeo& g, float inv, float rx, float ry, float rz) {
+    // inv = +-inf is depth 0: the point is b, whatever the (finite) ray
+    const bool at_centre = fabsf(inv) == INFINITY;
+    const float m = at_centre ? 0.f : 1.f, af = at_centre ? 1.f : inv;
+    const double a = (double)af, dx = (double)__fmul_rn(rx, m), dy = (double)__fmul_rn(ry, m),
+                 dz = (double)__fmul_rn(rz, m);
+    const double X = __fma_rn(a, g.b[0], __fma_rn(g.m[2], dz, __fma_rn(g.m[1], dy, __dmul_rn(g.m[0], dx))));
+    const double Y = __fma_rn(a, g.b[1], __fma_rn(g.m[5], dz, __fma_rn(g.m[4], dy, __dmul_rn(g.m[3], dx))));
+    const double Z = __fma_rn(a, g.b[2], __fma_rn(g.m[8], dz, __fma_rn(g.m[7], dy, __dmul_rn(g.m[6], dx))));
+    const double iz = rcp_newton(Z);
+    const double nx = __dmul_rn(X, iz), ny = __dmul_rn(Y, iz);
+    double dd = g.f;   // a pinhole's factor f (1 + r2 (0 + r2 (0 + r2 0))) is exactly f
+    if (!PINHOLE) {
+        const double r2 = __fma_rn(nx, nx, __dmul_rn(ny, ny));
+        dd = __dmul_rn(g.f, __fma_rn(r2, __fma_rn(r2, __fma_rn(r2, g.k3, g.k2), g.k1), 1.0));
+    }
+    const double u = __fma_rn(dd, nx, g.cx), v = __fma_rn(dd, ny, g.cy);
+    // camera depth Z / inv > 1e-6: Z - 1e-6 inv has the sign of inv
+    const double t = __fma_rn(-1e-6, a, Z);
+    RayTap s;
+    s.ok = (__double2hiint(t) ^ __double2hiint(a)) >= 0 && af != 0.f;
+    // 0 <= u <= w - 1.001 on the bit patterns as unsigned integers: a negative or NaN u is above
+    // every limit (NaN hypotheses count as invalid; the reference leaves them undefined)
+    s.ok = s.ok && (unsigned long long)__double_as_longlong(u) <= (unsigned long long)__double_as_longlong((double)g.w - 1.001) &&
+           (unsigned long long)__double_as_longlong(v) <= (unsigned long long)__double_as_longlong((double)g.h - 1.001);
+    // floor: u + 1.5 * 2^52 rounded toward -inf holds floor(u) in its low word
+    const double tu = __dadd_rd(u, 6755399441055744.0), tv = __dadd_rd(v, 6755399441055744.0);
+    s.fx = __dsub_rn(u, __dsub_rn(tu, 6755399441055744.0));
+    s.fy = __dsub_rn(v, __dsub_rn(tv, 6755399441055744.0));
+    s.o = s.ok ? (long long)__double2loint(tv) * g.w + __double2loint(tu) : 0;
+    MVS_BOUND(s.o >= 0 && s.o + g.w + 1 < (long long)g.h * g.w);
+    return s;
+}
+
+__device__ __forceinline__ float ray_value(const RayTap& s, float t00, float t01, float t10, float t11) {
+    const double gx = __dsub_rn(1.0, s.fx), gy = __dsub_rn(1.0, s.fy);
+    const double top = __fma_rn((double)t01, s.fx, __dmul_rn((double)t00, gx));
+    const double bot = __fma_rn((double)t11, s.fx, __dmul_rn((double)t10, gx));
+    const float val = (float)__fma_rn(bot, s.fy, __dmul_rn(top, gy));
+    return s.ok && isfinite(val) ? val : qnan();
+}
+
+// Stage A of the ray path: a thread keeps halo column c and rows seg, seg + SEG, ... as in the plane
+// path, and its share of the 2R right-hand columns; `inv` holds its samples' inverse depths for
+// this hypothesis (NaN: no sample), in registers because every source uses them (reloading base
+// and step per source: 4000 x 3000, R = 3, 22.7 against 15.1 ms). GROUP samples are in flight
+// together. Against one sample at a time with four conversions more and two divisions:
+// depth_map's three sweeps take 29.5 -> 15.1 ms at 4000 x 3000 (8 sources, R = 3), 5.0 -> 2.5 ms at
+// 1600 x 1200 (4 sources, R = 5), 0.99 -> 0.19 ms at 320 x 240 (most of it more, smaller chunks).
+template <int R, int TH>
+struct RayShare {
+    static constexpr int NT = TileShape<TH>::NT, SEG = TileShape<TH>::SEG, HR = Geom<R, TH>::HR;
+    static constexpr int MR = (HR + SEG - 1) / SEG;                        // samples in the own column
+    static constexpr int XW = R > 0 ? 2 * R : 1, XS = 2 * R * HR, PX = (XS + NT - 1) / NT;
+    static constexpr int NS = MR + PX;
+    // halo position of sample k; false: a surplus sample (past the tile)
+    static __device__ __forceinline__ bool at(int k, int tid, int& hy, int& hc) {
+        if (k < MR) {
+            hy = tid / TW + k * SEG;
+            hc = tid % TW;
+            return (k + 1) * SEG <= HR || hy < HR;
+        }
+        const int e = tid + (k - MR) * NT;
+        hy = e / XW;
+        hc = TW + (e - hy * XW);
+        return (k - MR + 1) * NT <= XS || e < XS;
+    }
+};
+
+template <int R, int TH, bool PINHOLE>
+__device__ __forceinline__ void stage_a_ray(const SweepParams& p, const SrcGeo& g, const float (&inv)[RayShare<R, TH>::NS],
+                                            int tx, int ty, int tid, float* sJ, bool& any_invalid, bool& any_valid) {
+    using S = RayShare<R, TH>;
+    using G = Geom<R, TH>;
+    constexpr int GROUP = 4;
+    const long long HW = (long long)p.H * p.W;
+    const float* img = reinterpret_cast<const float*>(g.img);
+    const float* img1 = img + g.w;
+#pragma unroll
+    for (int k0 = 0; k0 < S::NS; k0 += GROUP) {
+        RayTap tap[GROUP];
+        float t00[GROUP], t01[GROUP], t10[GROUP], t11[GROUP];
+#pragma unroll
+        for (int q = 0; q < GROUP; ++q) {
+            if (k0 + q >= S::NS) continue;
+            int hy, hc;
+            S::at(k0 + q, tid, hy, hc);
+            // out-of-image and surplus samples (inv = NaN) read a ray of the image
+            const int gy = min(max(ty - R + hy, 0), p.H - 1), gx = min(max(tx - R + hc, 0), p.W - 1);
+            const float* r = p.ray + ((long long)gy * p.W + gx);
+                        tap[q] = ray_tap<PINHOLE>(g, inv[k0 + q], __ldg(r), __ldg(r + HW), __ldg(r + 2 * HW));
+        }
+#pragma unroll
+        for (int q = 0; q < GROUP; ++q) {
+            if (k0 + q >= S::NS) continue;
+            const float *a = img + tap[q].o, *b = img1 + tap[q].o;
+            t00[q] = __ldg(a);
+            t01[q] = __ldg(a + 1);
+            t10[q] = __ldg(b);
+            t11[q] = __ldg(b + 1);
+        }
+#pragma unroll
+        for (int q = 0; q < GROUP; ++q) {
+            if (k0 + q >= S::NS) continue;
+            const float J = ray_value(tap[q], t00[q], t01[q], t10[q], t11[q]);
+            int hy, hc;
+            if (S::at(k0 + q, tid, hy, hc)) {
+                MVS_BOUND(hy * G::JP + (G::RA - R) + hc < G::HR * G::JP);
+                any_invalid |= J != J;
+                any_valid |= J == J;
+                sJ[hy * G::JP + (G::RA - R) + hc] = J;
+            }
+        }
+    }
 }
 
 // The plane map of one (hypothesis, source, tile), composed in FP64 and rounded once (Coef),
@@ -764,6 +891,7 @@ template <int R, int KMAX, bool PLANES, bool F16, bool WIDE = false, bool REF_TM
           bool CMP = false, int TH = TH_DEFAULT>
 __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb, int chunk, float* smem) {
     using G = Geom<R, TH>;
+    using WS = WinnerState<R, KMAX, TH>;
     constexpr int NT = TileShape<TH>::NT, SEG = TileShape<TH>::SEG;
     constexpr int K = G::K, RA = G::RA, HR = G::HR, HC = G::HC, JP = G::JP, P = G::P, NSEG = G::NSEG,
                   NIN = G::NIN;
@@ -799,9 +927,9 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
     }
 
     // winner-take-all state of the tile's pixels: touched once per hypothesis, so it lives in
-    // shared memory (planes: best, prev, s_prev_best, s_next_best, first score, idx bits)
+    // shared memory (planes: best, prev, s_prev_best, s_next_best, idx bits, first score)
     float* sW = reinterpret_cast<float*>(sH + HR * TW);
-    Coef* sC = reinterpret_cast<Coef*>(sW + 6 * TH * TW);
+    Coef* sC = reinterpret_cast<Coef*>(sW + WS::PLANES * TH * TW);
     const int c = tid % TW, seg = tid / TW;
     const float fcol = (float)c, fseg = (float)seg;
     const int gx = tx + c;
@@ -822,8 +950,8 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
         sW[TH * TW + w] = load ? p.prev[o] : -2.f;
         sW[2 * TH * TW + w] = load ? p.spb[o] : -2.f;
         sW[3 * TH * TW + w] = load ? p.snb[o] : -2.f;
-        sW[4 * TH * TW + w] = -2.f;
-        sW[5 * TH * TW + w] = __int_as_float(load ? p.idx[o] : -1);
+        sW[4 * TH * TW + w] = __int_as_float(load ? p.idx[o] : -1);
+        if constexpr (!WS::FIRST_TO_REC) sW[5 * TH * TW + w] = -2.f;
     }
     const int nsrc = p.n_src, kk = p.kk;
     const bool bottom = KMAX > 2 && p.topk_bottom != 0;   // the 2-entry list is always a top list
@@ -908,6 +1036,8 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
         }
     }
 
+    __shared__ unsigned s_reach[2][NT / 32];
+    int vote_slot = 0;
     for (int i = pa; i < pb; ++i) {
         float topk[ROWS][KMAX];
         float total[ROWS];
@@ -923,6 +1053,17 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
                 const int sg_ = tid >> 2;
                 make_coef_group(sC[sg_ < nsrc ? sg_ : 0], p.src[sg_ < nsrc ? sg_ : 0], p.planes[i - p.i0], tx - R,
                                 ty - R, HC, HR, sg_ < nsrc);
+            }
+        }
+        // ray path: the inverse depths of the thread's samples, shared by the sources
+        float inv[PLANES ? 1 : RayShare<R, TH>::NS];
+        if constexpr (!PLANES) {
+#pragma unroll
+            for (int k = 0; k < RayShare<R, TH>::NS; ++k) {
+                int hy, hc;
+                const bool own = RayShare<R, TH>::at(k, tid, hy, hc);
+                const int hgy = ty - R + hy, hgx = tx - R + hc;
+                inv[k] = own && hgy >= 0 && hgy < H && hgx >= 0 && hgx < W ? hyp_value(p, i, hgx, hgy) : qnan();
             }
         }
         // sC ready; first hypothesis: the tile's set-up of sI, sJ and sW too. (Between sources no
@@ -942,7 +1083,7 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
             // ---- A: warp the source into the halo tile
             const void* img = p.src[s].img;
             const int sw = p.src[s].w, sh = p.src[s].h;
-            bool any_invalid = false;
+            bool any_invalid = false, all_valid;
             if constexpr (PLANES) {
                 const Coef cf = sC[s];
                 constexpr int PER = (HR * HC + NT - 1) / NT;
@@ -1015,18 +1156,32 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
                     }
                 }
             } else {
-                any_invalid = true;
-                for (int e = tid; e < HR * HC; e += NT) {
-                    const int hy = e / HC, hc = e - hy * HC;
-                    const int gy = ty - R + hy, gxx = tx - R + hc;
-                    float J = qnan();
-                    if (gy >= 0 && gy < H && gxx >= 0 && gxx < W) J = sample_ray(p, p.src[s], i, gxx, gy);
-                    sJ[hy * JP + (RA - R) + hc] = CMP ? __fsub_rn(J, pv) : J;
+                static_assert(!CMP, "compensated sums run on the plane path");
+                const SrcGeo& g = p.src[s];
+                bool any_valid = false;
+                if (g.k1 == 0.0 && g.k2 == 0.0 && g.k3 == 0.0)
+                    stage_a_ray<R, TH, true>(p, g, inv, tx, ty, tid, sJ, any_invalid, any_valid);
+                else
+                    stage_a_ray<R, TH, false>(p, g, inv, tx, ty, tid, sJ, any_invalid, any_valid);
+                // a source that no sample reached: NCC -1 everywhere, as in the plane path. (The next
+                // stage A may write sJ at once: nothing reads it.) The votes alternate between two
+                // words, so a thread that runs ahead does not overwrite the one still being read.
+                const unsigned vote = (__any_sync(0xffffffffu, any_valid) ? 1u : 0u);
+                if ((tid & 31) == 0) s_reach[vote_slot][tid >> 5] = vote;
+                all_valid = !__syncthreads_or(any_invalid);
+                unsigned reach = 0;
+#pragma unroll
+                for (int w = 0; w < NT / 32; ++w) reach |= s_reach[vote_slot][w];
+                vote_slot ^= 1;
+                if (!reach) {
+#pragma unroll
+                    for (int j = 0; j < ROWS; ++j) topk_insert<KMAX>(topk[j], total[j], -1.f, bottom, nlist);
+                    continue;
                 }
             }
             // every sample of this (hypothesis, source) valid -> the count is k^2 everywhere and
             // stages B and C skip it (block-wide vote; uniform branch)
-            const bool all_valid = !__syncthreads_or(any_invalid);
+            if constexpr (PLANES) all_valid = !__syncthreads_or(any_invalid);
             // ---- B: horizontal window sums of (V, J, J^2, J I), one 16-column row segment per
             // thread: products once per input, running sums along the segment
             if constexpr (CMP) {
@@ -1078,16 +1233,29 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
             const int w = (seg * ROWS + j) * TW + c;
             MVS_BOUND(w < TH * TW);
             float best = sW[w], prv = sW[TH * TW + w];
-            const int id = __float_as_int(sW[5 * TH * TW + w]);
+            const int id = __float_as_int(sW[4 * TH * TW + w]);
             if (id == i - 1) sW[3 * TH * TW + w] = sc;
             if (sc > best) {
                 sW[w] = sc;
                 sW[2 * TH * TW + w] = prv;
                 sW[3 * TH * TW + w] = -2.f;
-                sW[5 * TH * TW + w] = __int_as_float(i);
+                sW[4 * TH * TW + w] = __int_as_float(i);
             }
             sW[TH * TW + w] = sc;
-            if (i == pa) sW[4 * TH * TW + w] = sc;
+            if constexpr (!WS::FIRST_TO_REC) {
+                if (i == pa) sW[5 * TH * TW + w] = sc;
+            }
+        }
+        if constexpr (WS::FIRST_TO_REC) {
+            if (to_rec && i == pa) {   // the prev plane holds the chunk's first scores now
+#pragma unroll 1
+                for (int j = 0; j < ROWS; ++j) {
+                    const int gy = ty + seg * ROWS + j;
+                    if (gx < W && gy < H)
+                        p.rec[(4LL * p.nchunks + chunk) * H * W + (long long)gy * W + gx] =
+                            sW[(TH + seg * ROWS + j) * TW + c];
+                }
+            }
         }
     }
 
@@ -1103,16 +1271,16 @@ __device__ void sweep_tile(const SweepParams& p, int tx, int ty, int pa, int pb,
             p.prev[o] = sW[TH * TW + w];
             p.spb[o] = sW[2 * TH * TW + w];
             p.snb[o] = sW[3 * TH * TW + w];
-            p.idx[o] = __float_as_int(sW[5 * TH * TW + w]);
+            p.idx[o] = __float_as_int(sW[4 * TH * TW + w]);
         } else {
             const long long HW = (long long)H * W;
             const long long plane = (long long)p.nchunks * HW;
             float* rc = p.rec + (long long)chunk * HW + o;
             rc[0] = sW[w];
-            rc[plane] = sW[5 * TH * TW + w];
+            rc[plane] = sW[4 * TH * TW + w];
             rc[2 * plane] = sW[2 * TH * TW + w];
             rc[3 * plane] = sW[3 * TH * TW + w];
-            rc[4 * plane] = sW[4 * TH * TW + w];
+            if constexpr (!WS::FIRST_TO_REC) rc[4 * plane] = sW[5 * TH * TW + w];
             rc[5 * plane] = sW[TH * TW + w];
         }
     }

@@ -66,3 +66,55 @@ def test_automatic_chunks_keep_the_bits(w, h, n):
     b = dense.sweep(*t, s, geo, hyp, 2, 2, state=b)
     for x, y in zip(a, b):
         assert same_bits(x.cpu().numpy(), y.cpu().numpy())
+
+
+@pytest.mark.parametrize("r", [0, 1, 3, 4, 5, 7])
+def test_special_inverse_depths(r):
+    """The per-pixel path's inverse depths at the ends of their range, against the oracle's
+    per-hypothesis scores (float64 window sums, which track it to ~1e-7; bar: tests_support):
+    infinite (depth 0: the reference's own centre as the source sees it), negative, tiny, huge;
+    0 and NaN have no valid sample, so every score is -1."""
+    from py_ortho_b200 import _lib as L, dense
+    from tests_support import SCORE_ABS, random_sweep_case
+    rng = np.random.default_rng(40 + r)
+    H, W, n = 45, 71, 3
+    ref, srcs, ray, geo, _ = random_sweep_case(rng, H, W, n, 2, nan_frac=0.0)
+    geo[:, 11] = (0.5, -0.5, 2.0)                  # b_z: in front, behind, in front
+    geo[2, 13:16] = 0.0                            # one pinhole source
+    base = rng.uniform(0.02, 0.2, (H, W)).astype(np.float32)
+    special = [base, np.full_like(base, np.inf), np.full_like(base, -np.inf), -base, np.full_like(base, 1e-30),
+               np.full_like(base, 1e30), np.zeros_like(base), np.full_like(base, np.nan)]
+    mixed = np.stack(special)[rng.integers(0, len(special) - 2, (H, W)), np.arange(H)[:, None], np.arange(W)[None]]
+    mu, sd = O.ref_stats(ref, r)
+    t = [_dev(a) for a in (ref, mu, sd, ray)]
+    s = [_dev(a) for a in srcs]
+    for k, inv in enumerate(special + [mixed]):
+        st = dense.sweep(*t, s, geo, dense.Hypotheses.maps_(_dev(inv[None])), r, 2, precision=L.PREC_FP64_SUMS)
+        got = st[1].cpu().numpy()
+        if k in (6, 7):
+            assert np.all(got == -1.0), k
+            continue
+        full = O.sweep(ref, srcs, ray, geo, [np.ascontiguousarray(inv)], r, 2, keep_scores=True)
+        assert np.abs(got - full["scores"][0]).max() <= SCORE_ABS, k
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (3, 200), (31, 33), (32, 64), (65, 129), (130, 31), (257, 300)])
+def test_window_statistics_at_tile_edges(h, w):
+    """The window mean and deviation bit for bit against the oracle: sizes around the 32-row /
+    32-column steps, radii inside and beyond the row pass's ring (15), windows larger than the image,
+    NaN and infinite pixels."""
+    from py_ortho_b200 import fast
+    rng = np.random.default_rng(h * 1000 + w)
+    a = rng.normal(0, 1, (h, w)).astype(np.float32)
+    b = a.copy()
+    b[rng.random((h, w)) < 0.01] = np.nan
+    b[h // 2, w // 2] = np.inf
+    for img in (a, b):
+        with np.errstate(invalid="ignore"):
+            for r in (0, 1, 5, 14, 15, 16, 40):
+                mu, sd = O.ref_stats(img, r)
+                gm, gs = fast.ref_stats(img, r)
+                nan = np.isnan(mu), np.isnan(sd)
+                assert np.array_equal(np.isnan(gm), nan[0]) and np.array_equal(np.isnan(gs), nan[1]), r
+                assert same_bits(gm[~nan[0]], mu[~nan[0]]) and same_bits(gs[~nan[1]], sd[~nan[1]]), r
+                assert same_bits(fast.box_zero_mean(img, r)[~nan[0]], mu[~nan[0]]), r

@@ -21,30 +21,159 @@ void clear_error() { g_err[0] = 0; }
 // difference c[y+k] - c[y]; then the same along each row; times float32(1/k^2). The two
 // cumulative sums are sequential float32 sums, so each column / row is one thread (the lead and
 // lag values c[y+k], c[y] follow the identical add sequence, so no table is stored).
-__device__ __forceinline__ float box_in(const float* a, long long o, int sq) {
-    const float v = a[o];
-    return sq ? __fmul_rn(v, v) : v;
-}
 
-__global__ void box_col_kernel(int H, int W, const float* __restrict__ a, int r, int sq, float* __restrict__ out) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+// Column pass: blockIdx.y selects the quantity (a into out0, or with sq the squares; the statistics
+// run both at once). One chain of additions per column leaves two warps per SM at 4000 columns, so
+// the time is memory latency: BOX_U rows are loaded ahead of the BOX_U being summed (no load waits
+// on a branch or on another load). Both quantities at 4000 x 3000: 2254 us with two launches of one
+// load per step, 926 us with loads behind bounds tests, 176 us so; at 640 x 480 152 -> 31 us.
+constexpr int BOX_U = 32;
+
+__global__ void __launch_bounds__(32) box_col_kernel(int H, int W, const float* __restrict__ a, int r, int sq0,
+                                                     float* __restrict__ out0, float* __restrict__ out1) {
+    const int x = blockIdx.x * 32 + threadIdx.x;
     if (x >= W) return;
-    const int k = 2 * r + 1;
-    auto val = [&](int i) -> float {       // padded row i
-        const int ay = i - (r + 1);
-        return (ay < 0 || ay >= H) ? 0.f : box_in(a, (long long)ay * W + x, sq);
-    };
-    float lag = val(0), lead = val(0);
-    for (int i = 1; i <= k; ++i) lead = __fadd_rn(lead, val(i));
-    for (int y = 0; y < H; ++y) {
-        out[(long long)y * W + x] = __fsub_rn(lead, lag);
-        lag = __fadd_rn(lag, val(y + 1));
-        lead = __fadd_rn(lead, val(y + k + 1));
+    const int sq = blockIdx.y ? 1 : sq0;
+    float* out = (blockIdx.y ? out1 : out0) + x;
+    const float* col = a + x;
+    // rows past the image are read from its edge and count as 0 when they are used, so that no load
+    // waits on a branch or on another load's value
+    auto raw = [&](int y) -> float { return __ldg(col + (long long)min(max(y, 0), H - 1) * W); };
+    auto val = [&](float v, int y) -> float { return y >= 0 && y < H ? (sq ? __fmul_rn(v, v) : v) : 0.f; };
+    float lag = 0.f, lead = 0.f;                        // c[y], c[y + k]
+    for (int y = 0; y <= r && y < H; ++y) lead = __fadd_rn(lead, val(raw(y), y));
+    float tail[BOX_U], head[BOX_U];                     // rows y - r and y + r + 1 of the next steps
+#pragma unroll
+    for (int u = 0; u < BOX_U; ++u) {
+        tail[u] = raw(u - r);
+        head[u] = raw(u + r + 1);
+    }
+    for (int y0 = 0; y0 < H; y0 += BOX_U) {
+        float t[BOX_U], h[BOX_U];
+#pragma unroll
+        for (int u = 0; u < BOX_U; ++u) {
+            t[u] = tail[u];
+            h[u] = head[u];
+        }
+#pragma unroll
+        for (int u = 0; u < BOX_U; ++u) {
+            tail[u] = raw(y0 + BOX_U + u - r);
+            head[u] = raw(y0 + BOX_U + u + r + 1);
+        }
+#pragma unroll
+        for (int u = 0; u < BOX_U; ++u) {
+            if (y0 + u < H) out[(long long)(y0 + u) * W] = __fsub_rn(lead, lag);
+            lag = __fadd_rn(lag, val(t[u], y0 + u - r));
+            lead = __fadd_rn(lead, val(h[u], y0 + u + r + 1));
+        }
     }
 }
 
-// one CTA per row: stage the row in shared memory, scan sequentially, write back coalesced
-__global__ void box_row_kernel(int H, int W, int r, float scale, float* __restrict__ io) {
+// Row pass for r <= BOX_ROW_MAX_R, in place: a block takes 32 rows and moves along them by 32 columns.
+// One warp per quantity runs the chains (lane = row) from a ring of 128 columns in shared memory
+// (pitch 129: lane = row and lane = column both touch 32 banks); the other warps bring the columns
+// that come two steps later and write the step before out, so a step costs its chain alone. STATS:
+// the window mean (io0) and the mean of squares (io1), which leaves as sd = sqrt(max(b2 - mu mu,
+// 1e-6)) in float32 (densify.py:328). Both quantities and sd at 4000 x 3000: 797 us as one thread per
+// row and a pass for sd, 411 us with a warp doing all its rows' work, 147 us so; 640 x 480 42 -> 27 us.
+constexpr int BOX_ROW_MAX_R = 15;      // the lead runs r + 1 <= 16 columns past a step: within the next one
+constexpr int BOX_RING = 128, BOX_ROW_WARPS = 8;
+
+template <bool STATS>
+constexpr size_t box_row_smem() {
+    return (size_t)(STATS ? 2 : 1) * 32 * ((BOX_RING + 1) + 2 * 33) * sizeof(float);
+}
+
+template <bool STATS>
+__global__ void __launch_bounds__(32 * BOX_ROW_WARPS) box_row_kernel(int H, int W, int r, float scale,
+                                                                     float* __restrict__ io0, float* __restrict__ io1) {
+    constexpr int NQ = STATS ? 2 : 1, NIO = BOX_ROW_WARPS - NQ, PER = (32 * NQ + NIO - 1) / NIO;
+    extern __shared__ float box_smem[];
+    float (*ring)[32][BOX_RING + 1] = reinterpret_cast<float (*)[32][BOX_RING + 1]>(box_smem);
+    float (*outs)[NQ][32][33] = reinterpret_cast<float (*)[NQ][32][33]>(box_smem + NQ * 32 * (BOX_RING + 1));
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row0 = blockIdx.x * 32;
+    const bool chain = w < NQ;
+    const int rows = min(32, H - row0);
+    // item m of an io warp: row q of quantity k
+    auto item = [&](int m, int& k, int& q) {
+        const int e = (w - NQ) + m * NIO;
+        k = e >> 5;
+        q = e & 31;
+        return e < 32 * NQ;
+    };
+    float next[PER];
+    auto fetch = [&](int x0) {             // columns and rows past the image: read at its edge, kept as 0
+        const long long x = min(x0 + lane, W - 1);
+#pragma unroll
+        for (int m = 0; m < PER; ++m) {
+            int k, q;
+            if (item(m, k, q)) next[m] = (STATS && k ? io1 : io0)[(long long)(row0 + min(q, rows - 1)) * W + x];
+        }
+    };
+    auto keep = [&](int x0) {
+#pragma unroll
+        for (int m = 0; m < PER; ++m) {
+            int k, q;
+            if (item(m, k, q)) ring[k][q][(x0 + lane) & (BOX_RING - 1)] = x0 + lane < W ? next[m] : 0.f;
+        }
+    };
+    auto leave = [&](int x0, int buf) {
+#pragma unroll
+        for (int m = 0; m < PER; ++m) {
+            int k, q;
+            if (item(m, k, q) && q < rows && x0 + lane < W) {
+                float v = outs[buf][k][q][lane];
+                if (STATS && k) {
+                    const float mu = outs[buf][0][q][lane];
+                    v = __fsqrt_rn(max_nan(__fsub_rn(v, __fmul_rn(mu, mu)), 1e-6f));
+                }
+                (STATS && k ? io1 : io0)[(long long)(row0 + q) * W + x0 + lane] = v;
+            }
+        }
+    };
+    for (int e = threadIdx.x; e < NQ * 32 * (BOX_RING + 1); e += 32 * BOX_ROW_WARPS) box_smem[e] = 0.f;
+    __syncthreads();                       // (zeros: the columns before 0)
+    if (!chain) {
+        fetch(0);
+        keep(0);
+        fetch(32);
+        keep(32);
+        fetch(64);
+    }
+    __syncthreads();
+    float lag = 0.f, lead = 0.f;
+    if (chain)
+        for (int x = 0; x <= r; ++x) lead = __fadd_rn(lead, ring[w][lane][x]);
+    int buf = 0;
+    for (int x0 = 0; x0 < W; x0 += 32, buf ^= 1) {
+        if (chain) {
+#pragma unroll
+            for (int h = 0; h < 32; h += 16) {
+                float t[16], n[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    t[u] = ring[w][lane][(x0 + h + u - r) & (BOX_RING - 1)];
+                    n[u] = ring[w][lane][(x0 + h + u + r + 1) & (BOX_RING - 1)];
+                }
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    outs[buf][w][lane][h + u] = __fmul_rn(__fsub_rn(lead, lag), scale);
+                    lag = __fadd_rn(lag, t[u]);
+                    lead = __fadd_rn(lead, n[u]);
+                }
+            }
+        } else {
+            keep(x0 + 64);                 // over the columns of two steps ago
+            fetch(x0 + 96);
+            if (x0 > 0) leave(x0 - 32, buf ^ 1);
+        }
+        __syncthreads();
+    }
+    if (!chain) leave((W - 1) / 32 * 32, buf ^ 1);
+}
+
+// Row pass at any radius: one CTA per row, the row staged in shared memory, one thread's chain.
+__global__ void box_row_wide_kernel(int H, int W, int r, float scale, float* __restrict__ io) {
     extern __shared__ float row[];        // 2 * W
     float* res = row + W;
     const int y = blockIdx.x;
@@ -78,19 +207,38 @@ __global__ void sd_kernel(long long n, const float* __restrict__ mu, float* b2sd
     b2sd[i] = __fsqrt_rn(max_nan(v, 1e-6f));
 }
 
-mvs_status box_zero_mean(int H, int W, const float* a, int r, int sq, float* out, cudaStream_t st) {
-    if (H == 0 || W == 0) return MVS_OK;
-    box_col_kernel<<<(W + 127) / 128, 128, 0, st>>>(H, W, a, r, sq, out);
-    MVS_TRY(check_launch("box column pass"));
+static float box_scale(int r) {
     const int k = 2 * r + 1;
-    const float scale = (float)(1.0 / ((double)k * k));
-    const size_t smem = (size_t)2 * W * sizeof(float);
+    return (float)(1.0 / ((double)k * k));
+}
+
+template <bool STATS>
+static mvs_status box_rows(int H, int W, int r, float* io0, float* io1, cudaStream_t st) {
+    constexpr size_t smem = box_row_smem<STATS>();
     if (smem > 48 * 1024) {
-        MVS_CUDA(cudaFuncSetAttribute(box_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+        MVS_CUDA(cudaFuncSetAttribute(box_row_kernel<STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                  "box: shared memory attribute");
     }
-    box_row_kernel<<<H, 128, smem, st>>>(H, W, r, scale, out);
+    box_row_kernel<STATS><<<(H + 31) / 32, 32 * BOX_ROW_WARPS, smem, st>>>(H, W, r, box_scale(r), io0, io1);
     return check_launch("box row pass");
+}
+
+static mvs_status box_rows_wide(int H, int W, int r, float* io, cudaStream_t st) {
+    const size_t smem = (size_t)2 * W * sizeof(float);
+    if (smem > 48 * 1024) {
+        MVS_CUDA(cudaFuncSetAttribute(box_row_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                 "box: shared memory attribute");
+    }
+    box_row_wide_kernel<<<H, 128, smem, st>>>(H, W, r, box_scale(r), io);
+    return check_launch("box row pass");
+}
+
+mvs_status box_zero_mean(int H, int W, const float* a, int r, int sq, float* out, cudaStream_t st) {
+    if (H == 0 || W == 0) return MVS_OK;
+    box_col_kernel<<<dim3((W + 31) / 32, 1), 32, 0, st>>>(H, W, a, r, sq, out, nullptr);
+    MVS_TRY(check_launch("box column pass"));
+    if (r > BOX_ROW_MAX_R) return box_rows_wide(H, W, r, out, st);
+    return box_rows<false>(H, W, r, out, nullptr, st);
 }
 
 // ---- rays: _fast._undistort (_fast.pyx:145-164) + densify._rays_world (densify.py:288-297)
@@ -353,8 +501,11 @@ extern "C" mvs_status mvs_ref_stats(int32_t H, int32_t W, const float* ref, int3
     if (H == 0 || W == 0) return MVS_OK;
     if (!ref || !mu || !sd || mu == sd || ref == mu || ref == sd) return fail(MVS_ERR_VALUE, "ref_stats: bad pointers");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    MVS_TRY(box_zero_mean(H, W, ref, r, 0, mu, st));
-    MVS_TRY(box_zero_mean(H, W, ref, r, 1, sd, st));
+    box_col_kernel<<<dim3((W + 31) / 32, 2), 32, 0, st>>>(H, W, ref, r, 0, mu, sd);
+    MVS_TRY(check_launch("ref_stats column pass"));
+    if (r <= BOX_ROW_MAX_R) return box_rows<true>(H, W, r, mu, sd, st);
+    MVS_TRY(box_rows_wide(H, W, r, mu, st));
+    MVS_TRY(box_rows_wide(H, W, r, sd, st));
     const long long n = (long long)H * W;
     sd_kernel<<<blocks(n, 256), 256, 0, st>>>(n, mu, sd);
     return check_launch("ref_stats sd");

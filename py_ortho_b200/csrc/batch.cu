@@ -32,9 +32,9 @@ struct JobFin {                        // per-job table of the merge / finalize 
 // One radius of the tile engine as an out-of-line call: the persistent kernel dispatches on the
 // work item's radius, and keeping each instance out of line gives each its own register
 // allocation (inlined together, the largest instance's pressure spilled the others).
-template <int R, int KMAX, bool F16, bool WIDE, int TH>
+template <int R, int KMAX, bool F16, int TH>
 __device__ __noinline__ void batch_tile(const SweepParams& p, int tx, int ty, int pa, int pb, int ch, float* smem) {
-    sweep_tile<R, KMAX, true, F16, WIDE, false, false, false, TH>(p, tx, ty, pa, pb, ch, smem);
+    sweep_tile<R, KMAX, true, F16, false, false, false, TH>(p, tx, ty, pa, pb, ch, smem);
 }
 
 // TH: the plan's tile height (one shape per persistent launch; 64 x TH tiles on 8 TH threads)
@@ -59,17 +59,17 @@ __global__ void __launch_bounds__(TileShape<TH>::NT, TileShape<TH>::MIN_CTAS)
         const int tx = w.y * TW, ty = w.z * TH;
         // the radius is uniform per work item: each case is the single-view instance itself
         switch (p.r) {
-            case 0: batch_tile<0, KMAX, F16, false, TH>(p, tx, ty, pa, pb, ch, smem); break;
-            case 1: batch_tile<1, KMAX, F16, false, TH>(p, tx, ty, pa, pb, ch, smem); break;
-            case 2: batch_tile<2, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
-            case 3: batch_tile<3, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
+            case 0: batch_tile<0, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+            case 1: batch_tile<1, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+            case 2: batch_tile<2, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+            case 3: batch_tile<3, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
             default:
                 if constexpr (RMAX > 3) {
                     switch (p.r) {
-                        case 4: batch_tile<4, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
-                        case 5: batch_tile<5, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
-                        case 6: batch_tile<6, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
-                        default: batch_tile<7, KMAX, F16, true, TH>(p, tx, ty, pa, pb, ch, smem); break;
+                        case 4: batch_tile<4, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+                        case 5: batch_tile<5, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+                        case 6: batch_tile<6, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
+                        default: batch_tile<7, KMAX, F16, TH>(p, tx, ty, pa, pb, ch, smem); break;
                     }
                 }
         }

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(TileShape<TH>::NT, TileShape<TH>::MIN_CTAS)
     extern __shared__ __align__(128) float4 smem4[];
     const int pa = p.i0 + blockIdx.z * p.ppc;
     const int pb = min(p.i1, pa + p.ppc);
-    sweep_tile<R, KMAX, PLANES, F16, true, true, X64, CMP, TH>(p, blockIdx.x * TW, blockIdx.y * TH, pa, pb,
+    sweep_tile<R, KMAX, PLANES, F16, true, X64, CMP, TH>(p, blockIdx.x * TW, blockIdx.y * TH, pa, pb,
                                                      p.rec ? (int)blockIdx.z : -1, reinterpret_cast<float*>(smem4));
 }
 

@@ -30,6 +30,8 @@
 
 namespace mvs {
 
+struct PMStats;
+
 struct PMParams {
     int H, W, S, r, step, top_k, it, colour;
     double cr0, cr1, cr2, geo_w, geo_tol, dmin, dmax, dd_scale, nn_scale;
@@ -54,6 +56,12 @@ struct PMParams {
     int pinhole[MVS_MAX_SOURCES];       // k1 = k2 = k3 = 0
     double par[MVS_MAX_SOURCES * 18];
     double bsrc[MVS_MAX_SOURCES * 3];   // R_s (C_ref - C_s)
+    // float64 kernel: the active pixels of this colour (pass pixel numbers in raster order) and their
+    // count, both on the device; float32 copies of par and bsrc for the window tests
+    const unsigned* list;
+    const unsigned* n_list;
+    const PMStats* stats;
+    float parf[MVS_MAX_SOURCES * 18], bsf[MVS_MAX_SOURCES * 3];
     // float32 lane kernel: per source its 2 x 2 bilinear footprints, quad[y w + x] =
     // (I(y, x), I(y, x + 1), I(y + 1, x), I(y + 1, x + 1)), one 16-byte load per sample
     const float4* quad[MVS_MAX_SOURCES];
@@ -124,15 +132,83 @@ __device__ __forceinline__ double pm_bil(const float* im, int w, int h, double u
     return (a00 * (1.0 - fx) + a01 * fx) * (1.0 - fy) + (a10 * (1.0 - fx) + a11 * fx) * fy;
 }
 
-// _pm_cost (_dense.pyx:461-556). Window samples are the outer loop as in the reference; the
-// sources of a pass (PM_SRC_PASS at a time) are unrolled inside it with their five sums in
-// registers, so each sample's world point (one division) is formed once per pass instead of once
-// per source. Each source's work is branch-free (invalid samples read a safe address and add 0.0,
-// which leaves a sum that started at +0.0 unchanged), so the sources' float64 dependency chains
-// interleave. Every per-source sum still accumulates in window order: no result changes.
-#ifndef PM_SRC_PASS
-#define PM_SRC_PASS 2
+// ---------------------------------------------------------------- float64 evaluation (MVS_PM_FP64)
+//
+// _pm_cost (_dense.pyx:461-556), every value with the reference's bits. What bounds it is the float64
+// pipe (64 lanes a clock per SM), so the work that provably does not reach a result is left out and
+// what is shared is formed once:
+//   * the geometric term comes first: a candidate whose geometric term alone reaches the pixel's
+//     best cost cannot be accepted (the photo term is at least 1 - NCC, see PM_PRUNE), so its windows
+//     are not evaluated;
+//   * per (candidate, source) the window's four corners are mapped in float32: a source that the
+//     whole window misses has NCC -1 (the count gate), one that it hits with a margin needs no
+//     per-sample tests, and its reference sums are the pixel's own, formed once per visit;
+//   * PM_PASS sources share a sample's world point (one division), and x / z, y / z share one
+//     reciprocal; the tap position comes from an addition rounded toward -inf (no conversions);
+//   * only active pixels get a thread (PMParams::list).
+// Each of a source's sums still accumulates in window order.
+
+// Sources per pass over the window (PM_MIN_BLOCKS has the measurements).
+#ifndef PM_PASS
+#define PM_PASS 2
 #endif
+
+// What mvs_pm_refine's preparation finds out about its inputs (float bit patterns, all >= 0).
+struct PMStats {
+    unsigned max_abs;      // largest finite |value| of the reference and the sources
+    unsigned ray_bend;     // largest second difference of the ray grid along rows and columns
+};
+
+__global__ void __launch_bounds__(256) pm_stats_kernel(const float* __restrict__ im, long long n, PMStats* st) {
+    float m = 0.f;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const float v = fabsf(__ldg(im + i));
+        if (v <= 3.402823466e38f) m = fmaxf(m, v);
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&st->max_abs, __float_as_uint(m));
+}
+
+__global__ void __launch_bounds__(256) pm_bend_kernel(const float* __restrict__ ray, int H, int W, PMStats* st) {
+    const long long HW = (long long)H * W;
+    float m = 0.f;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < HW; i += (long long)gridDim.x * 256) {
+        const int y = (int)(i / W), x = (int)(i - (long long)y * W);
+        for (int k = 0; k < 3; ++k) {
+            const float* r = ray + k * HW + i;
+            const float v = __ldg(r);
+            if (!(fabsf(v) <= 3.402823466e38f)) m = INFINITY;
+            if (x > 0 && x < W - 1) {
+                const float d = fabsf((__ldg(r + 1) - v) - (v - __ldg(r - 1)));
+                m = d <= 3.402823466e38f ? fmaxf(m, d) : INFINITY;
+            }
+            if (y > 0 && y < H - 1) {
+                const float d = fabsf((__ldg(r + W) - v) - (v - __ldg(r - W)));
+                m = d <= 3.402823466e38f ? fmaxf(m, d) : INFINITY;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(&st->ray_bend, __float_as_uint(m));
+}
+
+// 1 / z by two Newton-Raphson steps on the hardware's approximation, to the last bit or so.
+__device__ __forceinline__ double pm_rcp(double z) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));
+    double e = __fma_rn(-z, r, 1.0);
+    r = __fma_rn(r, e, r);
+    e = __fma_rn(-z, r, 1.0);
+    return __fma_rn(r, e, r);
+}
+
+// a / b from r ~ 1 / b: Markstein's correction (IBM J. Res. Dev. 34, 1990) - the remainder a - q b is
+// exact in one fused operation, so the result is the correctly rounded quotient except where a / b
+// lies within ~2^-50 ulp of the middle between two doubles. Several numerators share one reciprocal.
+__device__ __forceinline__ double pm_quot(double a, double b, double r) {
+    const double q = __dmul_rn(a, r);
+    return __fma_rn(__fma_rn(-q, b, a), r, q);
+}
 
 // Geometric term of _pm_cost (_dense.pyx:532-555): mean over the sources with depth maps of
 // min(1, |z - d_j| / d_j / geo_tol) at the rounded projection of the window centre.
@@ -162,104 +238,261 @@ __device__ __forceinline__ double pm_geo(const PMParams& c, double d, double rpx
     return geo;
 }
 
-__device__ double pm_cost(const PMParams& c, int y, int x, double d, const double* n, double& ncc_out) {
-    const int H = c.H, W = c.W;
-    const long long HW = (long long)H * W, idx = (long long)y * W + x;
-    const double rpx = __ldg(c.ray + idx), rpy = __ldg(c.ray + HW + idx), rpz = __ldg(c.ray + 2 * HW + idx);
-    const double ndr = n[0] * rpx + n[1] * rpy + n[2] * rpz;
+// A pixel's window, fixed for one visit.
+struct PMPix {
+    int y, x;
+    int a0, a1, b0, b1;            // offsets inside the image: a0, a0 + step, .. <= a1 (rows), b likewise
+    double rpx, rpy, rpz;
+    double si, sii;                // sums of I and I^2 over the finite reference values, in window order
+    int nfin;
+    float dev;                     // bound of a ray's distance from the corners' bilinear interpolation
+    bool prune;
+};
+
+// Float32 corner offsets (ray_corner - ray_p) of the block's pixels: [corner * 3 + component][thread].
+typedef float PMCorners[12][128];
+
+// One candidate's window sums for M consecutive entries of a source list (uniform over the warp's
+// converged lanes): sJ, sJJ, sIJ, and when CHECKED sI, sII and the count of valid samples.
+template <int M, bool CHECKED>
+__device__ __forceinline__ void pm_sums64(const PMParams& c, const PMPix& px, const int (&src)[M], double num,
+                                          const double* n, int& ns, double (&sJ)[M], double (&sJJ)[M], double (&sIJ)[M],
+                                          double (&sI)[M], double (&sII)[M], int (&cnt)[M]) {
+    const long long HW = (long long)c.H * c.W;
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+        sJ[k] = 0.0; sJJ[k] = 0.0; sIJ[k] = 0.0; sI[k] = 0.0; sII[k] = 0.0; cnt[k] = 0;
+    }
+    ns = 0;
+    for (int a = px.a0; a <= px.a1; a += c.step) {
+        const long long row = (long long)(px.y + a) * c.W + px.x;
+        for (int b = px.b0; b <= px.b1; b += c.step) {
+            const long long q = row + b;
+            const float If = __ldg(c.ref + q);
+            if (!(fabsf(If) <= 3.402823466e38f)) continue;
+            const double I = If;
+            const double qx = __ldg(c.ray + q), qy = __ldg(c.ray + HW + q), qz = __ldg(c.ray + 2 * HW + q);
+            const double den = n[0] * qx + n[1] * qy + n[2] * qz;
+            if (CHECKED && den >= -1e-9) continue;
+            const double t = pm_quot(num, den, pm_rcp(den));
+            const double X = c.cr0 + t * qx, Y = c.cr1 + t * qy, Z = c.cr2 + t * qz;
+            ++ns;
+            const double II = I * I;
+#pragma unroll
+            for (int k = 0; k < M; ++k) {
+                const int s = src[k];
+                const double* p = c.par + 18 * s;
+                // _proj
+                const double dx = X - p[9], dy = Y - p[10], dz = Z - p[11];
+                const double xc = p[0] * dx + p[1] * dy + p[2] * dz;
+                const double yc = p[3] * dx + p[4] * dy + p[5] * dz;
+                const double zc = p[6] * dx + p[7] * dy + p[8] * dz;
+                const bool front = !CHECKED || zc > 1e-6;
+                const double zq = front ? zc : 1.0;
+                const double rz = pm_rcp(zq);
+                const double nx = pm_quot(xc, zq, rz), ny = pm_quot(yc, zq, rz);
+                // pinhole source: the reference's factor f (1 + r2 (k1 + r2 (k2 + r2 k3)))
+                // evaluates to exactly f (r2 >= 0 finite, so every product with 0 is +0)
+                double dd = p[12];
+                if (!c.pinhole[s]) {
+                    const double r2 = nx * nx + ny * ny;
+                    dd = p[12] * (1.0 + r2 * (p[13] + r2 * (p[14] + r2 * p[15])));
+                }
+                const double u = dd * nx + p[16], v = dd * ny + p[17];
+                // _bil: floor by an addition rounded toward -inf (the low word of u + 1.5 * 2^52)
+                const int iw = c.iw[s], ih = c.ih[s];
+                bool in = true;
+                double us = u, vs = v;
+                if (CHECKED) {   // NaN u / v count as outside
+                    in = front && u >= 0.0 && v >= 0.0 && u <= (double)iw - 1.001 && v <= (double)ih - 1.001;
+                    us = in ? u : 0.0;
+                    vs = in ? v : 0.0;
+                }
+                const double tu = __dadd_rd(us, 6755399441055744.0), tv = __dadd_rd(vs, 6755399441055744.0);
+                int x0 = __double2loint(tu), y0 = __double2loint(tv);
+                if (!CHECKED) {
+                    // a no-op for the lanes whose window is inside; the others' sums are not used
+                    x0 = (int)min((unsigned)x0, (unsigned)(iw - 2));
+                    y0 = (int)min((unsigned)y0, (unsigned)(ih - 2));
+                }
+                const double fx = us - __dsub_rn(tu, 6755399441055744.0), fy = vs - __dsub_rn(tv, 6755399441055744.0);
+                MVS_BOUND((long long)y0 * iw + x0 >= 0 && (long long)y0 * iw + x0 + iw + 1 < (long long)iw * ih);
+                const float* im = c.img[s] + ((long long)y0 * iw + x0);
+                const double a00 = __ldg(im), a01 = __ldg(im + 1), a10 = __ldg(im + iw), a11 = __ldg(im + iw + 1);
+                const double J = (a00 * (1.0 - fx) + a01 * fx) * (1.0 - fy) + (a10 * (1.0 - fx) + a11 * fx) * fy;
+                if (CHECKED) {
+                    const bool ok = in && isfinite(J);
+                    sI[k] += ok ? I : 0.0;
+                    sJ[k] += ok ? J : 0.0;
+                    sII[k] += ok ? II : 0.0;
+                    sJJ[k] += ok ? J * J : 0.0;
+                    sIJ[k] += ok ? I * J : 0.0;
+                    cnt[k] += ok ? 1 : 0;
+                } else {
+                    sJ[k] += J;
+                    sJJ[k] += J * J;
+                    sIJ[k] += I * J;
+                }
+            }
+        }
+    }
+}
+
+// Where the window of plane (d, n) maps to in source s: +1 every sample inside with a margin (and in
+// front, and counted), -1 every sample outside, 0 neither shown. The window's rays are within `dev` of
+// the bilinear interpolation of its corner rays and the plane's map is projective, so undistorted
+// image points lie in the box of the corners' points, widened by the effect of `dev` and of float32
+// rounding; a distorted source's factor 1 + r2 (..) is bounded by its terms' absolute values.
+__device__ __forceinline__ int pm_where(const PMParams& c, const PMPix& px, const PMCorners& cor, int s, float num,
+                                        float n0, float n1, float n2, float ndr) {
+    const float* p = c.parf + 18 * s;
+    const float* bs = c.bsf + 3 * s;
+    const float rx = (float)px.rpx, ry = (float)px.rpy, rz = (float)px.rpz;
+    float M[3][3], cen[3], big = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float b = bs[i], p0 = p[3 * i], p1 = p[3 * i + 1], p2 = p[3 * i + 2];
+        M[i][0] = fmaf(b, n0, num * p0);
+        M[i][1] = fmaf(b, n1, num * p1);
+        M[i][2] = fmaf(b, n2, num * p2);
+        cen[i] = fmaf(b, ndr, num * fmaf(p0, rx, fmaf(p1, ry, p2 * rz)));
+        big = fmaxf(big, fabsf(b * ndr));
+    }
+    big += fabsf(num) * (fabsf(rx) + fabsf(ry) + fabsf(rz));
+    const float zc = cen[2];                              // camera depth is zc / ndr: < 0 in front
+    if (!(zc < -1e-20f)) return 0;
+    const float iz = __fdividef(1.0f, zc);
+    float xlo = INFINITY, xhi = -INFINITY, ylo = INFINITY, yhi = -INFINITY;
+    bool good = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float w0 = cor[3 * k][threadIdx.x], w1 = cor[3 * k + 1][threadIdx.x], w2 = cor[3 * k + 2][threadIdx.x];
+        const float v0 = fmaf(M[0][0], w0, fmaf(M[0][1], w1, fmaf(M[0][2], w2, cen[0])));
+        const float v1 = fmaf(M[1][0], w0, fmaf(M[1][1], w1, fmaf(M[1][2], w2, cen[1])));
+        const float v2 = fmaf(M[2][0], w0, fmaf(M[2][1], w1, fmaf(M[2][2], w2, cen[2])));
+        const float den = fmaf(n0, w0, fmaf(n1, w1, fmaf(n2, w2, ndr)));
+        good = good && den < -1e-4f - 4.f * px.dev && v2 < 1e-2f * den && v2 < 0.5f * zc;
+        const float r = __fdividef(1.0f, v2);
+        xlo = fminf(xlo, v0 * r);
+        xhi = fmaxf(xhi, v0 * r);
+        ylo = fminf(ylo, v1 * r);
+        yhi = fmaxf(yhi, v1 * r);
+    }
+    const float ax = fmaxf(fabsf(xlo), fabsf(xhi)), ay = fmaxf(fabsf(ylo), fabsf(yhi));
+    // errors of the box, in image units of the undistorted plane: `dev` through the map (its change
+    // over the window is at most 2 x, by v2 < zc / 2), float32 rounding of the composed map
+    const float m2 = fabsf(M[2][0]) + fabsf(M[2][1]) + fabsf(M[2][2]);
+    const float m0 = fabsf(M[0][0]) + fabsf(M[0][1]) + fabsf(M[0][2]), m1 = fabsf(M[1][0]) + fabsf(M[1][1]) + fabsf(M[1][2]);
+    const float ex = -iz * (4.f * (m0 + ax * m2) * px.dev + 4e-6f * big * (1.f + ax));
+    const float ey = -iz * (4.f * (m1 + ay * m2) * px.dev + 4e-6f * big * (1.f + ay));
+    const float f = p[12], cx = p[16], cy = p[17];
+    float sd = 0.f;
+    if (!c.pinhole[s]) {
+        const float r2 = (ax + ex) * (ax + ex) + (ay + ey) * (ay + ey);
+        sd = 1.001f * r2 * (fabsf(p[13]) + r2 * (fabsf(p[14]) + r2 * fabsf(p[15])));
+    }
+    good = good && sd < 0.5f && f > 0.f && ex * f < 8.f && ey * f < 8.f;
+    xlo -= ex; xhi += ex; ylo -= ey; yhi += ey;
+    const float ulo = fmaf(f, xlo * (xlo < 0.f ? 1.f + sd : 1.f - sd), cx), uhi = fmaf(f, xhi * (xhi > 0.f ? 1.f + sd : 1.f - sd), cx);
+    const float vlo = fmaf(f, ylo * (ylo < 0.f ? 1.f + sd : 1.f - sd), cy), vhi = fmaf(f, yhi * (yhi > 0.f ? 1.f + sd : 1.f - sd), cy);
+    const float w = (float)c.iw[s], h = (float)c.ih[s];
+    const float m = 0.5f + 2e-5f * (f + fabsf(cx) + fabsf(cy) + w + h);
+    if (!good) return 0;                                  // NaN anywhere above fails a test
+    if (uhi < -m || vhi < -m || ulo > w + m || vlo > h + m) return -1;
+    return ulo > m && vlo > m && uhi < w - 1.001f - m && vhi < h - 1.001f - m ? 1 : 0;
+}
+
+// NCC of one source from its window sums (_dense.pyx:505-528).
+__device__ __forceinline__ double pm_ncc64(int ns, int cnt, double sI, double sJ, double sII, double sJJ, double sIJ) {
+    if (ns < 4 || (double)cnt < 0.7 * (double)ns) return -1.0;
+    const double dc = (double)cnt;
+    const double mi = sI / dc, mj = sJ / dc;
+    const double vi = sII / dc - mi * mi;
+    const double vj = sJJ / dc - mj * mj;
+    const double cv = sIJ / dc - mi * mj;
+    return (vi < 1e-8 || vj < 1e-8) ? 0.0 : cv / sqrt(vi * vj);
+}
+
+template <int M>
+__device__ __forceinline__ void pm_batch64(const PMParams& c, const PMPix& px, unsigned group, bool checked,
+                                           unsigned in, unsigned out, double num, const double* n, double* ncc) {
+    int src[M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) {
+        src[k] = __ffs(group) - 1;
+        group &= group - 1;
+    }
+    double sJ[M], sJJ[M], sIJ[M], sI[M], sII[M];
+    int ns, cnt[M];
+    bool redo = checked;
+    if (!checked) {
+        pm_sums64<M, false>(c, px, src, num, n, ns, sJ, sJJ, sIJ, sI, sII, cnt);
+        // a non-finite source value in the window poisons the sums
+#pragma unroll
+        for (int k = 0; k < M; ++k) redo = redo || (((in >> src[k]) & 1u) && !isfinite(sJJ[k]));
+        ns = px.nfin;
+#pragma unroll
+        for (int k = 0; k < M; ++k) {
+            sI[k] = px.si;
+            sII[k] = px.sii;
+            cnt[k] = px.nfin;
+        }
+    }
+    if (redo) pm_sums64<M, true>(c, px, src, num, n, ns, sJ, sJJ, sIJ, sI, sII, cnt);
+#pragma unroll
+    for (int k = 0; k < M; ++k)
+        ncc[src[k]] = !checked && ((out >> src[k]) & 1u) ? -1.0 : pm_ncc64(ns, cnt[k], sI[k], sJ[k], sII[k], sJJ[k], sIJ[k]);
+}
+
+// The cost of plane (d, n), or +inf where it provably is not below `best` (a candidate that the
+// caller then does not accept). best = +inf: always evaluated.
+__device__ double pm_cost(const PMParams& c, const PMPix& px, const PMCorners& cor, double d, const double* n, double best,
+                          double& ncc_out) {
+    const double ndr = n[0] * px.rpx + n[1] * px.rpy + n[2] * px.rpz;
     if (ndr >= -1e-6 || d <= 0.0) {
         ncc_out = 0.0;   // unused by the caller for cost 10 (never accepted over a real cost)
         return 10.0;
     }
+    const double gterm = c.geo_w * pm_geo(c, d, px.rpx, px.rpy, px.rpz);
+    // PM_PRUNE: the NCC of values up to 6 in magnitude exceeds 1 by less than 1e-3 through rounding
+    // (window sums of < 1000 samples carry < 1e-12; the variances are at least 1e-8), so the cost
+    // is at least gterm - 1e-3
+    if (px.prune && gterm - 1e-3 >= best) {
+        ncc_out = 0.0;
+        return __longlong_as_double(0x7ff0000000000000LL);
+    }
     const double num = d * ndr;
+    const unsigned all = (1u << c.S) - 1u;
+    unsigned in = 0, out = 0;
+    for (int s = 0; s < c.S; ++s) {
+        const int w = pm_where(c, px, cor, s, (float)num, (float)n[0], (float)n[1], (float)n[2], (float)ndr);
+        in |= w > 0 ? 1u << s : 0u;
+        out |= w < 0 ? 1u << s : 0u;
+    }
     double ncc[MVS_MAX_SOURCES];
-    int nsamp = 0;
-    for (int s0 = 0; s0 < c.S; s0 += PM_SRC_PASS) {
-        double sI[PM_SRC_PASS], sJ[PM_SRC_PASS], sII[PM_SRC_PASS], sJJ[PM_SRC_PASS], sIJ[PM_SRC_PASS];
-        int cnt[PM_SRC_PASS];
-#pragma unroll
-        for (int k = 0; k < PM_SRC_PASS; ++k) {
-            sI[k] = 0.0; sJ[k] = 0.0; sII[k] = 0.0; sJJ[k] = 0.0; sIJ[k] = 0.0; cnt[k] = 0;
-        }
-        const int npass = min(PM_SRC_PASS, c.S - s0);
-        int ns = 0;
-        for (int a = -c.r; a <= c.r; a += c.step) {
-            const int yy = y + a;
-            if (yy < 0 || yy >= H) continue;
-            for (int b = -c.r; b <= c.r; b += c.step) {
-                const int xx = x + b;
-                if (xx < 0 || xx >= W) continue;
-                const long long q = (long long)yy * W + xx;
-                const double I = __ldg(c.ref + q);
-                if (!isfinite(I)) continue;
-                const double qx = __ldg(c.ray + q), qy = __ldg(c.ray + HW + q), qz = __ldg(c.ray + 2 * HW + q);
-                const double den = n[0] * qx + n[1] * qy + n[2] * qz;
-                if (den >= -1e-9) continue;
-                const double t = num / den;
-                const double X = c.cr0 + t * qx, Y = c.cr1 + t * qy, Z = c.cr2 + t * qz;
-                ++ns;
-                const double II = I * I;
-#pragma unroll
-                for (int k = 0; k < PM_SRC_PASS; ++k) {
-                    if (k < npass) {
-                        const int s = s0 + k;
-                        const double* p = c.par + 18 * s;
-                        // _proj
-                        const double dx = X - p[9], dy = Y - p[10], dz = Z - p[11];
-                        const double xc = p[0] * dx + p[1] * dy + p[2] * dz;
-                        const double yc = p[3] * dx + p[4] * dy + p[5] * dz;
-                        const double zc = p[6] * dx + p[7] * dy + p[8] * dz;
-                        const bool front = zc > 1e-6;
-                        const double zq = front ? zc : 1.0;
-                        const double nx = xc / zq, ny = yc / zq;
-                        // pinhole source: the reference's factor f (1 + r2 (k1 + r2 (k2 + r2 k3)))
-                        // evaluates to exactly f (r2 >= 0 finite, so every product with 0 is +0)
-                        double dd = p[12];
-                        if (!c.pinhole[s]) {
-                            const double r2 = nx * nx + ny * ny;
-                            dd = p[12] * (1.0 + r2 * (p[13] + r2 * (p[14] + r2 * p[15])));
-                        }
-                        const double u = dd * nx + p[16], v = dd * ny + p[17];
-                        // _bil with its bounds (NaN u / v count as outside)
-                        const int iw = c.iw[s], ih = c.ih[s];
-                        const bool in = front && u >= 0.0 && v >= 0.0 && u <= (double)iw - 1.001 && v <= (double)ih - 1.001;
-                        const double us = in ? u : 0.0, vs = in ? v : 0.0;
-                        const int x0 = (int)us, y0 = (int)vs;
-                        const double fx = us - (double)x0, fy = vs - (double)y0;
-                        MVS_BOUND((long long)y0 * iw + x0 >= 0 && (long long)y0 * iw + x0 + iw + 1 < (long long)iw * ih);
-                        const float* im = c.img[s] + ((long long)y0 * iw + x0);
-                        const double a00 = __ldg(im), a01 = __ldg(im + 1), a10 = __ldg(im + iw), a11 = __ldg(im + iw + 1);
-                        const double J = (a00 * (1.0 - fx) + a01 * fx) * (1.0 - fy) + (a10 * (1.0 - fx) + a11 * fx) * fy;
-                        const bool ok = in && isfinite(J);
-                        sI[k] += ok ? I : 0.0;
-                        sJ[k] += ok ? J : 0.0;
-                        sII[k] += ok ? II : 0.0;
-                        sJJ[k] += ok ? J * J : 0.0;
-                        sIJ[k] += ok ? I * J : 0.0;
-                        cnt[k] += ok ? 1 : 0;
-                    }
-                }
+    for (int s = 0; s < c.S; ++s) ncc[s] = -1.0;
+    // the converged lanes walk the same source lists: the sources inside (or outside) for every lane
+    // without tests, then those that some lane has to test
+    const unsigned lanes = __activemask();
+    const unsigned need = __reduce_or_sync(lanes, all & ~out), test = __reduce_or_sync(lanes, all & ~out & ~in);
+    for (int checked = 0; checked < 2; ++checked) {
+        unsigned list = checked ? need & test : need & ~test;
+        while (list) {
+            const int m = min(__popc(list), PM_PASS);
+            unsigned group = 0;
+            for (int k = 0; k < m; ++k) {
+                group |= list & (0u - list);
+                list &= list - 1;
             }
-        }
-        nsamp = ns;   // identical for every pass
-#pragma unroll
-        for (int k = 0; k < PM_SRC_PASS; ++k) {
-            const int s = s0 + k;
-            if (k < npass) {
-                if (ns < 4 || (double)cnt[k] < 0.7 * (double)ns) {
-                    ncc[s] = -1.0;
-                } else {
-                    const double dc = (double)cnt[k];
-                    const double mi = sI[k] / dc, mj = sJ[k] / dc;
-                    const double vi = sII[k] / dc - mi * mi;
-                    const double vj = sJJ[k] / dc - mj * mj;
-                    const double cv = sIJ[k] / dc - mi * mj;
-                    ncc[s] = (vi < 1e-8 || vj < 1e-8) ? 0.0 : cv / sqrt(vi * vj);
-                }
-            }
+#if PM_PASS >= 4
+            if (m == 4) pm_batch64<4>(c, px, group, checked, in, out, num, n, ncc);
+            else if (m == 3) pm_batch64<3>(c, px, group, checked, in, out, num, n, ncc);
+            else
+#endif
+            if (m == 2) pm_batch64<2>(c, px, group, checked, in, out, num, n, ncc);
+            else pm_batch64<1>(c, px, group, checked, in, out, num, n, ncc);
         }
     }
-    (void)nsamp;
     // descending insertion sort (S <= 16), then the mean of the first top_k
     for (int a = 1; a < c.S; ++a) {
         const double tmp = ncc[a];
@@ -275,14 +508,16 @@ __device__ double pm_cost(const PMParams& c, int y, int x, double d, const doubl
     for (int a = 0; a < kk; ++a) photo = photo + ncc[a];
     photo = photo / (double)kk;
     ncc_out = photo;
-    return (1.0 - photo) + c.geo_w * pm_geo(c, d, rpx, rpy, rpz);
+    return (1.0 - photo) + gterm;
 }
 
-// 8 resident blocks of 128 threads per SM (64 registers): the float64 chains are latency-bound,
-// so occupancy beats the spills (measured on B200, 2000 x 1500, 8 sources, 2 iterations: 2 sources
-// per pass and 8 blocks 224 ms; 6 blocks 240 ms; 8 sources per pass at 168 registers 334 ms)
+// Resident blocks of 128 threads per SM. Propagation + trials of a 1600 x 1200 repair (4 sources, 5 x 5
+// samples, a third of the pixels active, geometric term) / of 5 views of 800 x 600 (ms): 2 sources a
+// pass with 5 blocks (96 registers) 8.0 / 24.7, 6 blocks 8.3 / 26.1, 8 blocks 7.7 / 27.2; 4 sources a
+// pass with 5 blocks 11.5 / 37.7 (spills), 4 blocks 12.5 / 38.7. One thread per pixel, all windows
+// and tests, three divisions a sample: 36.0 / 54.2.
 #ifndef PM_MIN_BLOCKS
-#define PM_MIN_BLOCKS 8
+#define PM_MIN_BLOCKS 5
 #endif
 // Pixel of pass number t (raster order of the colour's pixels): false past the image.
 __device__ __forceinline__ bool pm_pixel(const PMParams& c, long long t, int& y, int& x) {
@@ -298,6 +533,7 @@ __device__ __forceinline__ bool pm_pixel(const PMParams& c, long long t, int& y,
 template <typename CostFn>
 __device__ __forceinline__ void pm_trials(const PMParams& c, unsigned st, float& dcur, float* ncur, double& best,
                                           double& sc, unsigned long long& changed, CostFn&& cost) {
+#pragma unroll 1
     for (int tr = 0; tr < 2; ++tr) {
         const double u0 = xs_draw(st);
         const double u1 = xs_draw(st);
@@ -314,7 +550,7 @@ __device__ __forceinline__ void pm_trials(const PMParams& c, unsigned st, float&
         nb[1] = nb[1] / nn;
         nb[2] = nb[2] / nn;
         double ph;
-        const double cst = cost(dp, nb, ph);
+        const double cst = cost(dp, nb, best, ph);
         if (cst < best) {
             best = cst;
             sc = ph;
@@ -339,34 +575,72 @@ __device__ __forceinline__ void pm_finish(const PMParams& c, long long idx, floa
     if (changed && c.changed) atomicAdd(c.changed, changed);
 }
 
-// PHASE 0: current plane and propagation; PHASE 1: the random trials.
+// PHASE 0: current plane and propagation; PHASE 1: the random trials. One thread per active pixel.
 template <int PHASE>
 __global__ void __launch_bounds__(128, PM_MIN_BLOCKS) pm_kernel(const __grid_constant__ PMParams c) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int y, x;
-    const bool in = pm_pixel(c, t, y, x);
+    __shared__ PMCorners cor;
+    const unsigned slot = blockIdx.x * 128u + threadIdx.x;
+    if (slot >= *c.n_list) return;
+    const long long t = c.list[slot];
+    PMPix px;
+    if (!pm_pixel(c, t, px.y, px.x)) return;          // (list entries are pixels)
+    const int y = px.y, x = px.x;
     const long long HW = (long long)c.H * c.W, idx = (long long)y * c.W + x;
-    if (!in || !c.active[idx]) {
-        if (PHASE == 0 && t < (long long)c.H * ((c.W + 1) / 2)) c.flags[t] = 0;
-        return;
+    unsigned flag = 0;
+    if (PHASE == 1) {
+        flag = c.flags[t];
+        if (!(flag & 1u)) {                           // no draws: the visit ends with propagation's result
+            pm_finish(c, idx, c.depth[idx], c.pbest[t], c.psc[t], flag >> 1);
+            return;
+        }
     }
-    auto cost = [&](double d, const double* nb, double& ph) { return pm_cost(c, y, x, d, nb, ph); };
+    {
+        // the window clipped to the image, its corner rays and its reference sums
+        const int r = c.r, st = c.step, m = 2 * r / st;
+        px.a0 = y - r < 0 ? -r + (r - y + st - 1) / st * st : -r;
+        px.b0 = x - r < 0 ? -r + (r - x + st - 1) / st * st : -r;
+        px.a1 = min(-r + m * st, c.H - 1 - y);
+        px.b1 = min(-r + m * st, c.W - 1 - x);
+        const float rx = __ldg(c.ray + idx), ry = __ldg(c.ray + HW + idx), rz = __ldg(c.ray + 2 * HW + idx);
+        px.rpx = rx; px.rpy = ry; px.rpz = rz;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int yy = k < 2 ? max(y - r, 0) : min(y + r, c.H - 1), xx = (k & 1) ? min(x + r, c.W - 1) : max(x - r, 0);
+            const long long q = (long long)yy * c.W + xx;
+            cor[3 * k][threadIdx.x] = __ldg(c.ray + q) - rx;
+            cor[3 * k + 1][threadIdx.x] = __ldg(c.ray + HW + q) - ry;
+            cor[3 * k + 2][threadIdx.x] = __ldg(c.ray + 2 * HW + q) - rz;
+        }
+        px.si = px.sii = 0.0;
+        px.nfin = 0;
+        for (int a = px.a0; a <= px.a1; a += st)
+            for (int b = px.b0; b <= px.b1; b += st) {
+                const float If = __ldg(c.ref + (long long)(y + a) * c.W + x + b);
+                if (!(fabsf(If) <= 3.402823466e38f)) continue;
+                const double I = If;
+                px.si += I;
+                px.sii += I * I;
+                ++px.nfin;
+            }
+        // piecewise linear interpolation between points 2 r apart is off by at most r^2 / 2 second
+        // differences per direction
+        px.dev = (float)(r * r) * __uint_as_float(c.stats->ray_bend);
+        px.prune = __uint_as_float(c.stats->max_abs) <= 6.f && (m + 1) * (m + 1) <= 400;
+    }
+    auto cost = [&](double d, const double* nb, double bound, double& ph) { return pm_cost(c, px, cor, d, nb, bound, ph); };
     float dcur = c.depth[idx];
     float ncur[3] = {c.normal[idx], c.normal[HW + idx], c.normal[2 * HW + idx]};
     double best, sc, ncc;
     unsigned long long changed = 0;
     if (PHASE == 1) {
-        const unsigned f = c.flags[t];
         best = c.pbest[t];
         sc = c.psc[t];
-        changed = f >> 1;
-        if (f & 1u) {
-            pm_trials(c, c.pstate[t], dcur, ncur, best, sc, changed, cost);
-            c.depth[idx] = dcur;
-            c.normal[idx] = ncur[0];
-            c.normal[HW + idx] = ncur[1];
-            c.normal[2 * HW + idx] = ncur[2];
-        }
+        changed = flag >> 1;
+        pm_trials(c, c.pstate[t], dcur, ncur, best, sc, changed, cost);
+        c.depth[idx] = dcur;
+        c.normal[idx] = ncur[0];
+        c.normal[HW + idx] = ncur[1];
+        c.normal[2 * HW + idx] = ncur[2];
         pm_finish(c, idx, dcur, best, sc, changed);
         return;
     }
@@ -376,32 +650,38 @@ __global__ void __launch_bounds__(128, PM_MIN_BLOCKS) pm_kernel(const __grid_con
     // cost of the pixel's current plane: reused from its previous visit when that visit kept the
     // plane it started with (the cost was then computed from these very float32 values)
     const double cached = c.cost_cache ? c.cost_cache[idx] : __longlong_as_double(0x7ff8000000000000LL);
-    if (isfinite(dcur) && cached == cached) {
+    const bool fresh = isfinite(dcur) && !(cached == cached);
+    best = 1e9;
+    sc = -1.0;
+    if (isfinite(dcur) && !fresh) {
         best = cached;
         sc = c.score_cache[idx];
-    } else if (isfinite(dcur)) {
-        const double n[3] = {ncur[0], ncur[1], ncur[2]};
-        best = pm_cost(c, y, x, (double)dcur, n, ncc);
-        sc = ncc;
-    } else {
-        best = 1e9;
-        sc = -1.0;
     }
-    const double rx = __ldg(c.ray + idx), ry = __ldg(c.ray + HW + idx), rz = __ldg(c.ray + 2 * HW + idx);
-    for (int k = 0; k < 8; ++k) {
-        const int yn = y + offy[k], xn = x + offx[k];
-        if (yn < 0 || xn < 0 || yn >= H || xn >= W) continue;
-        const long long nidx = (long long)yn * W + xn;
-        const float dnb = c.depth[nidx];
-        if (!isfinite(dnb)) continue;
-        const double nb[3] = {c.normal[nidx], c.normal[HW + nidx], c.normal[2 * HW + nidx]};
-        const double dn = nb[0] * __ldg(c.ray + nidx) + nb[1] * __ldg(c.ray + HW + nidx) + nb[2] * __ldg(c.ray + 2 * HW + nidx);
-        const double ndr = nb[0] * rx + nb[1] * ry + nb[2] * rz;
-        if (ndr >= -1e-6) continue;
-        const double dp = (double)dnb * dn / ndr;
-        if (dp < c.dmin || dp > c.dmax) continue;
-        const double cst = pm_cost(c, y, x, dp, nb, ncc);
-        if (cst < best) {
+    // one call of the cost in the code: k = -1 is the pixel's own plane
+#pragma unroll 1
+    for (int k = fresh ? -1 : 0; k < 8; ++k) {
+        double dp, nb[3];
+        if (k < 0) {
+            dp = (double)dcur;
+            nb[0] = ncur[0]; nb[1] = ncur[1]; nb[2] = ncur[2];
+        } else {
+            const int yn = y + offy[k], xn = x + offx[k];
+            if (yn < 0 || xn < 0 || yn >= H || xn >= W) continue;
+            const long long nidx = (long long)yn * W + xn;
+            const float dnb = c.depth[nidx];
+            if (!isfinite(dnb)) continue;
+            nb[0] = c.normal[nidx]; nb[1] = c.normal[HW + nidx]; nb[2] = c.normal[2 * HW + nidx];
+            const double dn = nb[0] * __ldg(c.ray + nidx) + nb[1] * __ldg(c.ray + HW + nidx) + nb[2] * __ldg(c.ray + 2 * HW + nidx);
+            const double ndr = nb[0] * px.rpx + nb[1] * px.rpy + nb[2] * px.rpz;
+            if (ndr >= -1e-6) continue;
+            dp = (double)dnb * dn / ndr;
+            if (dp < c.dmin || dp > c.dmax) continue;
+        }
+        const double cst = cost(dp, nb, k < 0 ? __longlong_as_double(0x7ff0000000000000LL) : best, ncc);
+        if (k < 0) {
+            best = cst;
+            sc = ncc;
+        } else if (cst < best) {
             best = cst;
             sc = ncc;
             dcur = (float)dp;
@@ -496,6 +776,45 @@ __global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_state_kernel(const unsigned 
     if (threadIdx.x == 0) base = jump8(J, rng[cur], boff[blockIdx.x]);
     __syncthreads();
     if (t < n) pstate[t] = f ? jump8(J, base, excl) : 0u;
+}
+
+// The active pixels of a colour: per block of PM_SCAN_BLOCK pass pixels their number, and (after
+// pm_offsets_kernel) their pass pixel numbers in raster order.
+__device__ __forceinline__ bool pm_is_active(const unsigned char* active, int H, int W, int colour, long long t) {
+    const int half_w = (W + 1) / 2;
+    if (t >= (long long)H * half_w) return false;
+    const int y = (int)(t / half_w), x = 2 * (int)(t - (long long)y * half_w) + ((y + colour) & 1);
+    return x < W && active[(long long)y * W + x];
+}
+__global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_active_count_kernel(const unsigned char* active, int H, int W,
+                                                                        int colour, unsigned* bsum) {
+    const long long t = (long long)blockIdx.x * PM_SCAN_BLOCK + threadIdx.x;
+    const int cnt = __syncthreads_count(pm_is_active(active, H, W, colour, t));
+    if (threadIdx.x == 0) bsum[blockIdx.x] = (unsigned)cnt;
+}
+// One block: counts -> exclusive offsets in place, and their total.
+__global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_offsets_kernel(unsigned* bsum, int nb, unsigned* total_out) {
+    const int per = (nb + PM_SCAN_BLOCK - 1) / PM_SCAN_BLOCK;
+    const int beg = min(nb, (int)threadIdx.x * per), end = min(nb, beg + per);
+    unsigned s = 0;
+    for (int i = beg; i < end; ++i) s += bsum[i];
+    unsigned total = 0;
+    unsigned run = block_exclusive_scan(s, total);
+    for (int i = beg; i < end; ++i) {
+        const unsigned v = bsum[i];
+        bsum[i] = run;
+        run += v;
+    }
+    if (threadIdx.x == 0) *total_out = total;
+}
+__global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_active_list_kernel(const unsigned char* active, int H, int W,
+                                                                       int colour, const unsigned* boff,
+                                                                       unsigned* list) {
+    const long long t = (long long)blockIdx.x * PM_SCAN_BLOCK + threadIdx.x;
+    const bool f = pm_is_active(active, H, W, colour, t);
+    unsigned total;
+    const unsigned excl = block_exclusive_scan(f ? 1u : 0u, total);
+    if (f) list[boff[blockIdx.x] + excl] = (unsigned)t;
 }
 
 __global__ void pm_rng_init_kernel(unsigned* rng, const unsigned* from, unsigned seed) {
@@ -995,7 +1314,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
     }
     const double rx = rpx, ry = rpy, rz = rpz;
     // cost of a candidate: _pm_cost's 10 for an invalid plane, else (1 - photo) + geo_w * geo
-    auto cost = [&](double d, const double* nb, double& photo) -> double {
+    auto cost = [&](double d, const double* nb, double, double& photo) -> double {
         const double ndr = nb[0] * rx + nb[1] * ry + nb[2] * rz;
         if (ndr >= -1e-6 || d <= 0.0) {
             photo = 0.0;
@@ -1030,7 +1349,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
         sc = c.score_cache[idx];
     } else if (isfinite(dcur)) {
         const double n[3] = {ncur[0], ncur[1], ncur[2]};
-        best = cost((double)dcur, n, ph);
+        best = cost((double)dcur, n, 0.0, ph);
         sc = ph;
     } else {
         best = 1e9;
@@ -1245,7 +1564,7 @@ __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
     wn.sii = sii;
     wn.allfin = kc == (float)nw;
     const double rx = rpx, ry = rpy, rz = rpz;
-    auto cost = [&](double d, const double* nb, double& photo) -> double {
+    auto cost = [&](double d, const double* nb, double, double& photo) -> double {
         const double ndr = nb[0] * rx + nb[1] * ry + nb[2] * rz;
         if (ndr >= -1e-6 || d <= 0.0) {
             photo = 0.0;
@@ -1343,12 +1662,16 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
     // float32 evaluation needs pinhole sources (the local map is a homography)
     bool fast = a->precision == MVS_PM_FP32;
     for (int s = 0; s < a->S && fast; ++s) fast = p.pinhole[s] != 0;
-    if (fast) {
+    {
         for (int s = 0; s < a->S; ++s) {
             const double* q = a->par + 18 * s;
             // b_s = R_s (C_ref - C_s)
             const double e0 = a->Cr[0] - q[9], e1 = a->Cr[1] - q[10], e2 = a->Cr[2] - q[11];
-            for (int i = 0; i < 3; ++i) p.bsrc[3 * s + i] = q[3 * i] * e0 + q[3 * i + 1] * e1 + q[3 * i + 2] * e2;
+            for (int i = 0; i < 3; ++i) {
+                p.bsrc[3 * s + i] = q[3 * i] * e0 + q[3 * i + 1] * e1 + q[3 * i + 2] * e2;
+                p.bsf[3 * s + i] = (float)p.bsrc[3 * s + i];
+            }
+            for (int k = 0; k < 18; ++k) p.parf[18 * s + k] = (float)q[k];
         }
     }
     // scratch, one stream-ordered allocation: per pass pixel the propagation result, its flag and
@@ -1359,8 +1682,10 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
     const bool use_cache = a->iters > 1;
     auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
     const size_t o_best = 0, o_sc = o_best + up(n * 8), o_state = o_sc + up(n * 8), o_flags = o_state + up(n * 4);
-    const size_t o_bsum = o_flags + up(n), o_rng = o_bsum + up((size_t)nb * 4), o_cache = o_rng + 256;
-    const size_t o_quad = o_cache + up(use_cache ? (size_t)HW * 2 * sizeof(double) : 0);
+    // (float64: flags and list for each colour)
+    const size_t flag_bytes = up(n), o_bsum = o_flags + (fast ? 1 : 2) * flag_bytes, o_rng = o_bsum + up((size_t)nb * 4), o_cache = o_rng + 256;
+    const size_t o_list = o_cache + up(use_cache ? (size_t)HW * 2 * sizeof(double) : 0);
+    const size_t list_bytes = fast ? 0 : up((size_t)n * 4), o_quad = o_list + 2 * list_bytes;
     size_t quad_bytes = 0;
     if (fast)
         for (int s = 0; s < a->S; ++s) quad_bytes += up((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
@@ -1388,6 +1713,25 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
             const long long ns = (long long)a->src_w[s] * a->src_h[s];
             const int qb = (int)std::min<long long>((ns + 255) / 256, 148LL * 8);
             pm_quad_kernel<<<qb, 256, 0, st>>>(a->src[s], a->src_w[s], a->src_h[s], q);
+        }
+    }
+    unsigned char* flags = reinterpret_cast<unsigned char*>(scratch + o_flags);
+    if (!fast) {
+        // pixels that are not active never draw; the input facts and both colours' active pixels
+        cudaMemsetAsync(flags, 0, 2 * flag_bytes, st);
+        PMStats* stats = reinterpret_cast<PMStats*>(rng + 8);
+        cudaMemsetAsync(stats, 0, sizeof(PMStats), st);
+        p.stats = stats;
+        const unsigned sb = 148 * 8;
+        pm_bend_kernel<<<sb, 256, 0, st>>>(a->ray, a->H, a->W, stats);
+        pm_stats_kernel<<<sb, 256, 0, st>>>(a->ref, HW, stats);
+        for (int s = 0; s < a->S; ++s)
+            pm_stats_kernel<<<sb, 256, 0, st>>>(a->src[s], (long long)a->src_w[s] * a->src_h[s], stats);
+        for (int colour = 0; colour < 2; ++colour) {
+            unsigned* list = reinterpret_cast<unsigned*>(scratch + o_list + colour * list_bytes);
+            pm_active_count_kernel<<<nb, PM_SCAN_BLOCK, 0, st>>>(a->active, a->H, a->W, colour, bsum);
+            pm_offsets_kernel<<<1, PM_SCAN_BLOCK, 0, st>>>(bsum, nb, rng + 4 + colour);
+            pm_active_list_kernel<<<nb, PM_SCAN_BLOCK, 0, st>>>(a->active, a->H, a->W, colour, bsum, list);
         }
     }
     const PMJump& J = stream_tables().J;
@@ -1449,6 +1793,11 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
         p.nn_scale = 0.3 / (double)(git + 1);
         for (int colour = 0; colour < 2 && status == MVS_OK; ++colour) {
             p.colour = colour;
+            if (!fast) {
+                p.flags = flags + colour * flag_bytes;
+                p.list = reinterpret_cast<unsigned*>(scratch + o_list + colour * list_bytes);
+                p.n_list = rng + 4 + colour;
+            }
             p.win_smem = (unsigned)smem;
             if (fast) lane_kernel[0]<<<grid, block, smem, st>>>(p);
             else pm_kernel<0><<<grid, 128, 0, st>>>(p);

@@ -63,7 +63,8 @@ struct PMParams {
     const PMStats* stats;
     float parf[MVS_MAX_SOURCES * 18], bsf[MVS_MAX_SOURCES * 3];
     // float32 lane kernel: per source its 2 x 2 bilinear footprints, quad[y w + x] =
-    // (I(y, x), I(y, x + 1), I(y + 1, x), I(y + 1, x + 1)), one 16-byte load per sample
+    // (I(y, x), I(y + 1, x), I(y, x + 1), I(y + 1, x + 1)), one 16-byte load per sample whose halves
+    // are the operands of the packed interpolation along x
     const float4* quad[MVS_MAX_SOURCES];
 };
 
@@ -764,18 +765,53 @@ __global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_scan_kernel(unsigned* bsum, 
 }
 
 // Per drawing pixel: the stream state before its first draw (0 for pixels that do not draw; a
-// xorshift32 state is never 0).
+// xorshift32 state is never 0). The jump of a pixel splits into the jump to its warp's first draw, which
+// the lanes of the first warp form for all 32 warps at once, and at most 31 pixels within the warp,
+// from nibble tables in shared memory (8 words read per matrix product instead of 32 masks and
+// xors): every pixel jumping by its block-wide number took 388 us a pass at 4000 x 3000.
 __global__ void __launch_bounds__(PM_SCAN_BLOCK) pm_state_kernel(const unsigned char* flags, long long n,
                                                                   const unsigned* boff, const unsigned* rng, int cur,
                                                                   const __grid_constant__ PMJump J, unsigned* pstate) {
-    const long long t = (long long)blockIdx.x * PM_SCAN_BLOCK + threadIdx.x;
-    const unsigned f = t < n ? (flags[t] & 1u) : 0u;
-    unsigned total;
-    const unsigned excl = block_exclusive_scan(f, total);
+    __shared__ unsigned tab[5][8][16];      // t[j] applied to nibble q of a state
+    __shared__ unsigned wcount[32], wbase[32];
     __shared__ unsigned base;
-    if (threadIdx.x == 0) base = jump8(J, rng[cur], boff[blockIdx.x]);
+    const long long t = (long long)blockIdx.x * PM_SCAN_BLOCK + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool f = t < n && (flags[t] & 1u);
+    const unsigned draw = __ballot_sync(0xffffffffu, f);
+    if (lane == 0) wcount[w] = __popc(draw);
+    if (threadIdx.x < 5 * 8 * 16) {
+        const int j = threadIdx.x / 128, q = (threadIdx.x / 16) % 8, v = threadIdx.x % 16;
+        unsigned r = 0;
+        for (int b = 0; b < 4; ++b)
+            if (v & (1 << b)) r ^= J.t[j].col[4 * q + b];
+        tab[j][q][v] = r;
+    }
+    if (threadIdx.x == PM_SCAN_BLOCK - 1) base = jump8(J, rng[cur], boff[blockIdx.x]);
     __syncthreads();
-    if (t < n) pstate[t] = f ? jump8(J, base, excl) : 0u;
+    if (w == 0) {                           // exclusive prefix of the warps' draws, and their states
+        unsigned inc = wcount[lane];
+        const unsigned own = inc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        wbase[lane] = jump8(J, base, inc - own);
+    }
+    __syncthreads();
+    if (t >= n) return;
+    unsigned s = wbase[w];
+    const unsigned k = __popc(draw & ((1u << lane) - 1u));
+#pragma unroll
+    for (int j = 0; j < 5; ++j)
+        if (k & (1u << j)) {
+            unsigned r = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) r ^= tab[j][q][(s >> (4 * q)) & 15u];
+            s = r;
+        }
+    pstate[t] = f ? s : 0u;
 }
 
 // The active pixels of a colour: per block of PM_SCAN_BLOCK pass pixels their number, and (after
@@ -831,7 +867,7 @@ __global__ void __launch_bounds__(256) pm_quad_kernel(const float* __restrict__ 
         const int y = (int)(i / w), x = (int)(i - (long long)y * w);
         const long long r0 = (long long)y * w, r1 = (long long)min(y + 1, h - 1) * w;
         const int x1 = min(x + 1, w - 1);
-        quad[i] = make_float4(__ldg(im + r0 + x), __ldg(im + r0 + x1), __ldg(im + r1 + x), __ldg(im + r1 + x1));
+        quad[i] = make_float4(__ldg(im + r0 + x), __ldg(im + r1 + x), __ldg(im + r0 + x1), __ldg(im + r1 + x1));
     }
 }
 
@@ -857,13 +893,12 @@ __global__ void __launch_bounds__(256) pm_quad_kernel(const float* __restrict__ 
 // Float32 costs differ from the float64 ones by ~1e-7 (measured 99.9th percentile 2e-6), so the
 // strict '<' can decide near-ties differently; the float64 mode is the bit-exact reference.
 
-// Resident blocks of 256 threads per SM for the lane kernel (propagation; trials). On B200, 2 iterations
-// of a 2000 x 1500, 8-source case with one 16-byte footprint load per sample: 5 / 5 blocks (48
-// registers, spills) 54.4 ms, 4 / 5 55.2 ms, 4 / 4 (64 registers) 55.5 ms, 4 / 3 57.4 ms, 3 / 4
-// 58.6 ms. (With four scalar tap loads 4 blocks had been best: 58.7 ms against 61.7 ms at 3 and
-// 64.5 ms at 5; rolling or partly unrolling a window row's samples was slower.)
+// Resident blocks of 256 threads per SM for the lane kernel (propagation; trials). Propagation of 4
+// iterations at 4000 x 3000, 8 sources, 7 x 7: 252 ms with single samples at 5 blocks (48 registers), in
+// pairs 239 ms at 5, 232 ms at 4 (64 registers), 248 ms at 3. What bounds it is latency at that
+// occupancy: issue slots alone would take ~100 ms, the footprints' L1 wavefronts ~50 ms.
 #ifndef PM_LANE_MIN_BLOCKS
-#define PM_LANE_MIN_BLOCKS 5
+#define PM_LANE_MIN_BLOCKS 4
 #endif
 #ifndef PM_LANE_MIN_BLOCKS_TRIALS
 #define PM_LANE_MIN_BLOCKS_TRIALS PM_LANE_MIN_BLOCKS
@@ -885,30 +920,79 @@ __device__ __forceinline__ unsigned pmf_floor_bits(float x, float& f) {   // |x|
     return (unsigned)__float_as_int(t);
 }
 
+__device__ __forceinline__ float2 pm_dup(float x) { return make_float2(x, x); }
+// a - b elementwise with one rounding (b (-1) + a)
+__device__ __forceinline__ float2 pm_sub2(float2 a, float2 b) { return __ffma2_rn(b, pm_dup(-1.0f), a); }
+// The hardware's approximation of 1 / x for normal x (the bits of __fdividef(1, x) there)
+__device__ __forceinline__ float pm_rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // A pixel's window as the cost code reads it: sample (row, k) = e-th of the window as
 // (ray_q - ray_p, I_q - mI) with I = NaN where there is no sample (outside the image or a
-// non-finite reference value), and the ray offsets of the clipped window's four corners.
+// non-finite reference value), and the ray offsets of the clipped window's four corners. PAIRS:
+// samples (row, 2 m) and (row, 2 m + 1) come as packed pairs of each component, for the packed
+// arithmetic of pm_window_sums (an odd side's last pair has a surplus second sample).
 //   PMWinStaged: staged once per visit in shared memory by the pixel's lane group;
+//   PMWinPairs:  the same for a side known at compile time, pair by pair (32 bytes: x x y y z z I I);
 //   PMWinTile:   read from the warp's shared tile of raw rays and reference values (one lane per
-//                pixel), the offsets formed on each read - the same float32 operations, so the
-//                same values (positions outside the image hold masked samples either way).
+//                pixel; one plane per component, so that a pair of columns is one 8-byte load and the
+//                lanes' loads are contiguous), the offsets formed on each read - the same float32
+//                operations, so the same values (positions outside the image hold masked samples
+//                either way). PAIRS at step 1, where a lane's columns start on an even one.
 struct PMWinStaged {
+    static constexpr bool PAIRS = false;
     const float4* w;      // NW samples, then the 4 corners
     __device__ __forceinline__ float4 at(int, int, int e) const { return w[e]; }
     __device__ __forceinline__ float4 corner(int k4, int nw) const { return w[nw + k4]; }
+    __device__ __forceinline__ void pair(int, int, float2&, float2&, float2&, float2&) const {}
 };
+template <int NSIDE>
+struct PMWinPairs {
+    static constexpr bool PAIRS = true;
+    static constexpr int NP = (NSIDE + 1) / 2;                 // pairs per row
+    // float4 entries per pixel: the pairs, the 4 corners, one more (an odd number of 16-byte units
+    // puts the 4 pixels of a warp on different banks)
+    static constexpr int ENTRIES = 2 * NSIDE * NP + 4 + 1;
+    const float4* w;
+    static __device__ __forceinline__ int slot(int row, int k) { return (row * NP + (k >> 1)) * 8 + (k & 1); }
+    __device__ __forceinline__ float4 at(int row, int k, int) const {
+        const float* f = reinterpret_cast<const float*>(w) + slot(row, k);
+        return make_float4(f[0], f[2], f[4], f[6]);
+    }
+    __device__ __forceinline__ float4 corner(int k4, int) const { return w[2 * NSIDE * NP + k4]; }
+    __device__ __forceinline__ void pair(int row, int m, float2& x, float2& y, float2& z, float2& i) const {
+        const float4 a = w[2 * (row * NP + m)], b = w[2 * (row * NP + m) + 1];
+        x = make_float2(a.x, a.y);
+        y = make_float2(a.z, a.w);
+        z = make_float2(b.x, b.y);
+        i = make_float2(b.z, b.w);
+    }
+};
+template <bool STEP1>
 struct PMWinTile {
-    const float4* t;      // tile entry of the window's first sample (row y - r, column x - r)
+    static constexpr bool PAIRS = STEP1;
+    const float* t;       // x plane at the window's first sample (row y - r, column x - r)
+    int plane;            // entries of one plane (x, y, z, I)
     int rs, cs;           // tile offsets of one window row and one window column
     int cy0, cy1, cx0, cx1;   // tile offsets of the clipped corners' rows and columns
     float rpx, rpy, rpz, mI;
     __device__ __forceinline__ float4 at(int row, int k, int) const {
-        const float4 v = t[row * rs + k * cs];
-        return make_float4(v.x - rpx, v.y - rpy, v.z - rpz, v.w - mI);
+        const float* v = t + row * rs + k * cs;
+        return make_float4(v[0] - rpx, v[plane] - rpy, v[2 * plane] - rpz, v[3 * plane] - mI);
     }
     __device__ __forceinline__ float4 corner(int k4, int) const {
-        const float4 v = t[(k4 < 2 ? cy0 : cy1) + ((k4 & 1) ? cx1 : cx0)];
-        return make_float4(v.x - rpx, v.y - rpy, v.z - rpz, 0.f);
+        const float* v = t + (k4 < 2 ? cy0 : cy1) + ((k4 & 1) ? cx1 : cx0);
+        return make_float4(v[0] - rpx, v[plane] - rpy, v[2 * plane] - rpz, 0.f);
+    }
+    __device__ __forceinline__ void pair(int row, int m, float2& x, float2& y, float2& z, float2& i) const {
+        const float* v = t + row * rs + 2 * m;
+        x = pm_sub2(*reinterpret_cast<const float2*>(v), pm_dup(rpx));
+        y = pm_sub2(*reinterpret_cast<const float2*>(v + plane), pm_dup(rpy));
+        z = pm_sub2(*reinterpret_cast<const float2*>(v + 2 * plane), pm_dup(rpz));
+        i = pm_sub2(*reinterpret_cast<const float2*>(v + 3 * plane), pm_dup(mI));
     }
 };
 
@@ -921,7 +1005,6 @@ struct PMWinT {
     float si, sii;        // sum of (I - mI) and (I - mI)^2 over those samples
     bool allfin;          // every sample has a finite reference value inside the image
 };
-using PMWin = PMWinT<PMWinStaged>;
 
 // One source's window sums. CHECKED: every sample tested as in the reference (camera depth,
 // source bounds, finite value) and the reference sums formed per source; otherwise (the whole
@@ -935,6 +1018,51 @@ __device__ __forceinline__ void pm_window_sums(const Acc& win, int side_rt, cons
                                                float mJ,
                                                float& T1, float& T2, float& X, float& S1, float& S2, float& cnt,
                                                float& ns) {
+    if constexpr (Acc::PAIRS && NSIDE > 0 && !CHECKED) {
+        // two samples at a time in packed float32 (each element rounds as its scalar operation, the
+        // sums still run sample by sample): coordinates, floors and fractions pair up over the
+        // samples, the interpolation along x over a footprint's two rows
+        const float2 A0 = pm_dup(A[0]), A1 = pm_dup(A[1]), A2 = pm_dup(A[2]), a0p = pm_dup(a0);
+        const float2 B0 = pm_dup(B[0]), B1 = pm_dup(B[1]), B2 = pm_dup(B[2]), b0p = pm_dup(b0);
+        const float2 C0 = pm_dup(C[0]), C1 = pm_dup(C[1]), C2 = pm_dup(C[2]), c0p = pm_dup(c0);
+        const float2 bias = pm_dup(12582912.0f), nbias = pm_dup(-12582912.0f);
+#pragma unroll 1
+        for (int row = 0; row < NSIDE; ++row)
+#pragma unroll
+            for (int m = 0; m < (NSIDE + 1) / 2; ++m) {
+                float2 x, y, z, iv;
+                win.pair(row, m, x, y, z, iv);
+                const float2 cq = __ffma2_rn(C0, x, __ffma2_rn(C1, y, __ffma2_rn(C2, z, c0p)));
+                const float2 aq = __ffma2_rn(A0, x, __ffma2_rn(A1, y, __ffma2_rn(A2, z, a0p)));
+                const float2 bq = __ffma2_rn(B0, x, __ffma2_rn(B1, y, __ffma2_rn(B2, z, b0p)));
+                const float2 rc = make_float2(pm_rcp_ftz(cq.x), pm_rcp_ftz(cq.y));
+                const float2 ul = __fmul2_rn(aq, rc), vl = __fmul2_rn(bq, rc);
+                const float2 tu = __fadd2_rd(ul, bias), tv = __fadd2_rd(vl, bias);
+                const float2 fx = pm_sub2(ul, __fadd2_rn(tu, nbias)), fy = pm_sub2(vl, __fadd2_rn(tv, nbias));
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    if (2 * m + q >= NSIDE) continue;
+                    // tap offset (floor(v) + V0) sw + floor(u) + U0 as below
+                    const unsigned xb = __float_as_uint(q ? tu.y : tu.x), yb = __float_as_uint(q ? tv.y : tv.x);
+                    const unsigned o = min(yb * (unsigned)sw + xb + kb, last);
+                    MVS_BOUND(o <= last);
+                    const float4 t = __ldg(qd + o);
+                    const float2 lo = make_float2(t.x, t.y), hi = make_float2(t.z, t.w);
+                    const float2 tb = __ffma2_rn(pm_dup(q ? fx.y : fx.x), pm_sub2(hi, lo), lo);   // (top, bottom)
+                    const float J = fmaf(q ? fy.y : fy.x, tb.y - tb.x, tb.x);
+                    float Jp = J - mJ, Iv = q ? iv.y : iv.x;
+                    if (!ALLFIN) {
+                        const bool ok = Iv == Iv;
+                        Jp = ok ? Jp : 0.f;
+                        Iv = ok ? Iv : 0.f;
+                    }
+                    T1 += Jp;
+                    T2 = fmaf(Jp, Jp, T2);
+                    X = fmaf(Iv, Jp, X);
+                }
+            }
+        return;
+    }
     // rows rolled, the samples of a row unrolled when the side is known (the checked form, rare,
     // stays rolled to keep the instruction footprint small)
     const int side = NSIDE > 0 ? NSIDE : side_rt;
@@ -966,7 +1094,7 @@ __device__ __forceinline__ void pm_window_sums(const Acc& win, int side_rt, cons
         MVS_BOUND(o <= last);
         const float fx = ul - fu, fy = vl - fv;
         const float4 q4 = __ldg(qd + o);
-        const float t00 = q4.x, t01 = q4.y, t10 = q4.z, t11 = q4.w;
+        const float t00 = q4.x, t01 = q4.z, t10 = q4.y, t11 = q4.w;
         const float top = fmaf(fx, t01 - t00, t00), bot = fmaf(fx, t11 - t10, t10);
         const float J = fmaf(fy, bot - top, top);
         if (CHECKED) ok = ok && fabsf(J) <= 3.4e38f;
@@ -1075,7 +1203,7 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
             const int o = min(max(yi * sw + xi, 0), last);
             const float fx = ul - fu, fy = vl - fv;
             const float4 q4 = __ldg(qd + o);
-            const float t00 = q4.x, t01 = q4.y, t10 = q4.z, t11 = q4.w;
+            const float t00 = q4.x, t01 = q4.z, t10 = q4.y, t11 = q4.w;
             const float top = fmaf(fx, t01 - t00, t00), bot = fmaf(fx, t11 - t10, t10);
             const float J = fmaf(fy, bot - top, top);
             if (fabsf(J) <= 3.4e38f) mJ = J;
@@ -1218,6 +1346,20 @@ __device__ __forceinline__ double pm_geo_lane(const PMParams& c, double d, doubl
 // Samples along one side of the window: offsets -r, -r + step, ... <= r.
 __host__ __device__ inline int pm_side(int r, int step) { return (2 * r) / step + 1; }
 
+// The lane kernel's staged window: pairs when the side is known at compile time.
+template <int NSIDE>
+struct PMLaneWin {
+    using Acc = PMWinPairs<NSIDE>;
+};
+template <>
+struct PMLaneWin<0> {
+    using Acc = PMWinStaged;
+};
+// float4 entries of one pixel's staged window (nside: the compile-time side or 0; nw: its samples)
+__host__ __device__ constexpr int pm_lane_entries(int nside, int nw) {
+    return nside > 0 ? 2 * nside * ((nside + 1) / 2) + 5 : nw + 4;
+}
+
 // PHASE 0: current plane and propagation; PHASE 1: the random trials.
 template <int L, int NSIDE, int PHASE>
 __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE_MIN_BLOCKS_TRIALS)
@@ -1250,10 +1392,12 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
     // shift of the float32 sums
     const int side = NSIDE > 0 ? NSIDE : pm_side(c.r, c.step);
     const int nw = side * side;
-    float4* win = pm_win + (threadIdx.x / L) * (nw + 4);
-    MVS_BOUND((threadIdx.x / L + 1) * (nw + 4) * sizeof(float4) <= c.win_smem);
+    using Acc = typename PMLaneWin<NSIDE>::Acc;
+    const int entries = pm_lane_entries(NSIDE, nw);
+    float4* win = pm_win + (threadIdx.x / L) * entries;
+    MVS_BOUND((threadIdx.x / L + 1) * entries * sizeof(float4) <= c.win_smem);
     const float rpx = __ldg(c.ray + idx), rpy = __ldg(c.ray + HW + idx), rpz = __ldg(c.ray + 2 * HW + idx);
-    PMWin wn;
+    PMWinT<Acc> wn;
     wn.acc.w = win;
     wn.side = side;
     wn.nw = nw;
@@ -1282,7 +1426,25 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
                     k += 1.f;
                 }
             }
-            win[e] = v;
+            if constexpr (NSIDE > 0) {
+                if (e < nw) {
+                    float* f = reinterpret_cast<float*>(win) + Acc::slot(e / NSIDE, e % NSIDE);
+                    f[0] = v.x;
+                    f[2] = v.y;
+                    f[4] = v.z;
+                    f[6] = v.w;
+                } else {
+                    win[2 * NSIDE * Acc::NP + e - nw] = v;
+                }
+            } else {
+                win[e] = v;
+            }
+        }
+        if constexpr (NSIDE % 2 == 1 && NSIDE > 0) {   // the surplus sample of a row's last pair: the centre ray
+            for (int e = lane; e < NSIDE; e += L) {
+                float* f = reinterpret_cast<float*>(win) + Acc::slot(e, NSIDE);
+                f[0] = f[2] = f[4] = f[6] = 0.f;
+            }
         }
 #pragma unroll
         for (int o = L >> 1; o > 0; o >>= 1) {
@@ -1293,10 +1455,13 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
         const float mI = k > 0.f ? sum / k : 0.f;
         float si = 0.f, sii = 0.f;
         for (int e = lane; e < nw; e += L) {
-            const float I = win[e].w;
+            float* f;
+            if constexpr (NSIDE > 0) f = reinterpret_cast<float*>(win) + Acc::slot(e / NSIDE, e % NSIDE) + 6;
+            else f = &win[e].w;
+            const float I = *f;
             if (I == I) {
                 const float Ip = I - mI;
-                win[e].w = Ip;
+                *f = Ip;
                 si += Ip;
                 sii = fmaf(Ip, Ip, sii);
             }
@@ -1439,12 +1604,12 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
 // kernel's order (L strided partial sums, then its butterfly), so a trial's cost has the lane
 // kernel's bits when top_k <= 2 and no source has a depth map (otherwise the top-k and geometric
 // sums add the same terms in another order).
-// Blocks of 4 warps; resident blocks per SM measured on B200 (2 iterations of a 2000 x 1500,
-// 8-source case, the whole PatchMatch call): 3 (168 registers) 50.9 ms, 4 (128) 50.1 ms, 5 (96,
-// spills) 53.0 ms, 6 (80) 52.6 ms, 8 (64) 57.6 ms; the lane groups' trials 54.0-54.4 ms.
+// Blocks of 4 warps; the trials of 4 iterations at 4000 x 3000, 8 sources: single samples from a tile of
+// 16-byte entries (half of its wavefronts bank conflicts) 88.0 ms at 4 blocks per SM; pairs from
+// planes 84.3 ms at 3 (168 registers), 89.7 ms at 4 (128, spills).
 constexpr int PM_TRIAL_WARPS = 4;   // warps per block
 #ifndef PM_TRIAL_MIN_BLOCKS
-#define PM_TRIAL_MIN_BLOCKS 4
+#define PM_TRIAL_MIN_BLOCKS 3
 #endif
 #ifndef PM_TRIAL_LANE_GROUPS
 #define PM_TRIAL_LANE_GROUPS 0      // 1: the trials on the lane groups' kernel (comparisons)
@@ -1477,7 +1642,7 @@ __device__ __forceinline__ void pm_group_sums(int nw, F&& term, float& a, float&
     b = pb[0];
 }
 
-template <int L, int NSIDE>
+template <int L, int NSIDE, bool STEP1>
 __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
     pm_trial_kernel(const __grid_constant__ PMParams c) {
     extern __shared__ float4 pm_tiles[];
@@ -1490,8 +1655,10 @@ __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
     const int par = (y + c.colour) & 1;
     const int pitch = pm_tile_pitch(r), rows = 2 * r + 1;
     const int xs0 = 2 * k0 + par - r;                                     // image column of tile column 0
-    float4* tile = pm_tiles + (size_t)warp * rows * pitch;
-    MVS_BOUND((size_t)(warp + 1) * rows * pitch * sizeof(float4) <= c.win_smem);
+    // planes of x, y, z and reference value, each rows x pitch (pitch even: column pairs are aligned)
+    const int plane = rows * pitch;
+    float* tile = reinterpret_cast<float*>(pm_tiles + (size_t)warp * plane);
+    MVS_BOUND((size_t)(warp + 1) * plane * sizeof(float4) <= c.win_smem);
     const long long HW = (long long)H * W;
     for (int e = lane; e < rows * pitch; e += 32) {
         const int ty = e / pitch, tx = e - ty * pitch;
@@ -1505,7 +1672,10 @@ __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
             const float I = __ldg(c.ref + q);
             if (fabsf(I) <= 3.4e38f) v.w = I;
         }
-        tile[e] = v;
+        tile[e] = v.x;
+        tile[plane + e] = v.y;
+        tile[2 * plane + e] = v.z;
+        tile[3 * plane + e] = v.w;
     }
     __syncwarp();
     const int k = k0 + lane, x = 2 * k + par;
@@ -1524,12 +1694,13 @@ __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
     const int nw = side * side;
     const float rpx = __ldg(c.ray + idx), rpy = __ldg(c.ray + HW + idx), rpz = __ldg(c.ray + 2 * HW + idx);
     // this pixel's window in the tile: sample (row, col) at w0[row * step * pitch + col * step]
-    const float4* w0 = tile + 2 * lane;
+    const float* w0 = tile + 2 * lane;
+    const float* i0 = w0 + 3 * plane;
     const int rs = step * pitch;
     float sum, kc, si, sii;
     pm_group_sums<L>(nw, [&](int e, float& a, float& b) {
         const int row = e / side, col = e - row * side;
-        const float I = w0[row * rs + col * step].w;
+        const float I = i0[row * rs + col * step];
         if (I == I) {
             a += I;
             b += 1.f;
@@ -1538,15 +1709,16 @@ __global__ void __launch_bounds__(32 * PM_TRIAL_WARPS, PM_TRIAL_MIN_BLOCKS)
     const float mI = kc > 0.f ? sum / kc : 0.f;
     pm_group_sums<L>(nw, [&](int e, float& a, float& b) {
         const int row = e / side, col = e - row * side;
-        const float I = w0[row * rs + col * step].w;
+        const float I = i0[row * rs + col * step];
         if (I == I) {
             const float Ip = I - mI;
             a += Ip;
             b = fmaf(Ip, Ip, b);
         }
     }, si, sii);
-    PMWinT<PMWinTile> wn;
+    PMWinT<PMWinTile<STEP1>> wn;
     wn.acc.t = w0;
+    wn.acc.plane = plane;
     wn.acc.rs = rs;
     wn.acc.cs = step;
     wn.acc.cy0 = (max(y - r, 0) - (y - r)) * pitch;
@@ -1738,7 +1910,7 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
     // float32 lanes: one per source; a block holds as many pixel groups as its staged windows fit
     const int lanes = a->S <= 4 ? 4 : (a->S <= 8 ? 8 : 16);
     const int side = pm_side(a->r, a->step);
-    const size_t win_bytes = (size_t)(side * side + 4) * sizeof(float4);
+    const size_t win_bytes = (size_t)pm_lane_entries(side == 7 || side == 5 ? side : 0, side * side) * sizeof(float4);
     int groups = 256 / lanes;
     while (groups > 1 && (size_t)groups * win_bytes > 96 * 1024) groups >>= 1;
     const int block = fast ? groups * lanes : 128;
@@ -1768,7 +1940,11 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
 #if !PM_TRIAL_LANE_GROUPS
     if (fast && status == MVS_OK && smem_trial <= 227 * 1024) {
 #define PM_PICK_TRIAL(LN)                                                                        \
-    trial_kernel = side == 7 ? pm_trial_kernel<LN, 7> : side == 5 ? pm_trial_kernel<LN, 5> : pm_trial_kernel<LN, 0>;
+    trial_kernel = side == 7 && a->step == 1   ? pm_trial_kernel<LN, 7, true>                       \
+                   : side == 5 && a->step == 1 ? pm_trial_kernel<LN, 5, true>                       \
+                   : side == 7                 ? pm_trial_kernel<LN, 7, false>                      \
+                   : side == 5                 ? pm_trial_kernel<LN, 5, false>                      \
+                                               : pm_trial_kernel<LN, 0, false>;
         if (lanes == 4) { PM_PICK_TRIAL(4) }
         else if (lanes == 8) { PM_PICK_TRIAL(8) }
         else { PM_PICK_TRIAL(16) }

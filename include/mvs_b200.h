@@ -136,6 +136,16 @@ mvs_status mvs_sweep(const mvs_sweep_args* args, void* stream);
  * cudaFree or other allocating routine. */
 mvs_status mvs_sweep_noalloc(const mvs_sweep_args* args, void* stream);
 
+/* mvs_sweep with its plane-chunk scratch given by the caller (256-byte aligned device memory, free
+ * to be used again by work that follows on `stream`): a host process with a caching allocator saves
+ * the driver's allocation per call. mvs_sweep_scratch_bytes: the bytes these arguments need on the
+ * current device (0: none, also for arguments that mvs_sweep rejects); fewer give MVS_ERR_VALUE. */
+size_t mvs_sweep_scratch_bytes(const mvs_sweep_args* args);
+/* The initial winner-take-all state (densify.py:331-335): -2 in the four score planes, idx -1. */
+mvs_status mvs_sweep_state_init(int32_t H, int32_t W, float* best, float* prev, float* s_prev_best,
+                                float* s_next_best, int32_t* idx, void* stream);
+mvs_status mvs_sweep_ws(const mvs_sweep_args* args, void* scratch, size_t scratch_bytes, void* stream);
+
 /* One hypothesis `i` given as an explicit inverse-depth map `inv` (H, W), ray-grid geometry
  * with radial distortion. Replaces _dense.sweep_hypothesis (_dense.pyx:740-838); argument
  * order and meaning as there (srcs: n_src device pointers with their shapes). */
@@ -225,6 +235,10 @@ typedef struct mvs_depth_band_args {
  * values. Allocates its cell table stream-ordered. */
 mvs_status mvs_depth_band(const mvs_depth_band_args* args, void* stream);
 
+/* mvs_depth_band with the cell table's memory given by the caller, as mvs_sweep_ws. */
+size_t mvs_depth_band_scratch_bytes(const mvs_depth_band_args* args);
+mvs_status mvs_depth_band_ws(const mvs_depth_band_args* args, void* scratch, size_t scratch_bytes, void* stream);
+
 /* float32 -> FP16 image conversion for MVS_PREC_FP16 sources (round to nearest; NaN kept). */
 mvs_status mvs_to_fp16(int64_t n, const float* in, void* out_half, void* stream);
 
@@ -280,10 +294,16 @@ typedef struct mvs_pm_args {
  * pass runs propagation for all its pixels in parallel, counts the drawing pixels (a prefix sum
  * in raster order) and jumps the stream to each pixel's offset (GF(2) matrix powers), then runs
  * the trials in parallel. With MVS_PM_FP64 the result is bit-identical to the reference's.
- * Scratch (about 21 bytes per pixel, plus 16 per pixel when iters > 1, plus 16 per source pixel
+ * Scratch (about 21 bytes per pixel, 26 with MVS_PM_FP64, plus 16 per pixel when iters > 1, plus 16 per source pixel
  * with MVS_PM_FP32: each source's 2 x 2 bilinear footprints, one 16-byte load per sample) is
  * allocated stream-ordered per call. */
 mvs_status mvs_pm_refine(const mvs_pm_args* args, void* stream);
+
+/* mvs_pm_refine with its scratch given by the caller (256-byte aligned device memory, free to be used
+ * again by work that follows on `stream`). mvs_pm_scratch_bytes: the bytes these arguments need
+ * (0: none, also for arguments that mvs_pm_refine rejects); fewer give MVS_ERR_VALUE. */
+size_t mvs_pm_scratch_bytes(const mvs_pm_args* args);
+mvs_status mvs_pm_refine_ws(const mvs_pm_args* args, void* scratch, size_t scratch_bytes, void* stream);
 
 /* The xorshift32 state after n steps of the PatchMatch stream from `state` (host; jump-ahead by
  * GF(2) matrix powers, n up to 2^64 - 1). mvs_pm_refine's trials use the same jumps. */

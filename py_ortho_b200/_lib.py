@@ -118,6 +118,9 @@ SIGNATURES = {
     "mvs_tie_depths": (i32, [i32, vp, vp, i32, i32, vp, vp]),
     "mvs_depth_band": (i32, [vp, vp]),
     "mvs_pm_refine": (i32, [vp, vp]),
+    "mvs_sweep_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_sweep_state_init": (i32, [i32, i32, vp, vp, vp, vp, vp, vp]),
+    "mvs_sweep_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_pm_stream_advance": (C.c_uint32, [C.c_uint32, C.c_uint64]),
     "mvs_batch_create": (i32, [vp, i32, vp, vp]),
     "mvs_batch_run": (i32, [vp, i32, vp]),
@@ -131,7 +134,11 @@ SIGNATURES = {
     "mvs_init_normals": (i32, [i32, i32, vp, vp, vp, vp]),
     "mvs_fuse_view": (i32, [vp, vp]),
     "mvs_sample_view": (i32, [vp, vp]),
+    "mvs_depth_band_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_depth_band_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_box_sat_mean": (i32, [i32, i32, i32, vp, i32, vp, vp]),
+    "mvs_pm_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_pm_refine_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_height_score": (i32, [vp, vp]),
     "mvs_sgm": (i32, [i32, i32, i32, vp, C.c_float, C.c_float, vp, vp]),
     "mvs_last_error": (C.c_size_t, [C.c_char_p, C.c_size_t]),
@@ -232,3 +239,22 @@ def host_f64(a) -> np.ndarray:
 
 def host_ptr(a: np.ndarray) -> int:
     return int(a.ctypes.data)
+def call_with_scratch(name: str, args: int, device, stream=None) -> int:
+    """Status of the entry point `name` on `args` (a struct's address), its scratch taken from torch's
+    caching allocator on the stream that the call uses: the driver's stream-ordered pool gives its
+    memory back at every synchronisation, so an allocation per call mapped it anew each time
+    (a 2 GB PatchMatch call ~25 ms, a small sweep ~0.5 ms). The memory is the stream's again when the
+    call returns. Under capture, or when the allocator has no room, the entry point allocates."""
+    lib, sh = load(), stream_handle(stream)
+    need = getattr(lib, "mvs_pm_scratch_bytes" if name == "mvs_pm_refine" else name + "_scratch_bytes")(args)
+    if need and (stream is None or isinstance(stream, torch.cuda.Stream)):
+        with contextlib.nullcontext() if stream is None else torch.cuda.stream(stream):
+            if not torch.cuda.is_current_stream_capturing():
+                try:
+                    ws = torch.empty(need, dtype=torch.uint8, device=device)
+                    return getattr(lib, name + "_ws")(args, ws.data_ptr(), need, sh)
+                except torch.cuda.OutOfMemoryError:
+                    pass
+    return getattr(lib, name)(args, sh)
+
+

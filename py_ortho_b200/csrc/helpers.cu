@@ -588,37 +588,60 @@ extern "C" mvs_status mvs_tie_depths(int32_t n, const double* X, const double* c
     return check_launch("tie_depths");
 }
 
-extern "C" mvs_status mvs_depth_band(const mvs_depth_band_args* a, void* stream) {
-    clear_error();
+static mvs_status check_depth_band(const mvs_depth_band_args* a) {
     if (!a) return fail(MVS_ERR_VALUE, "depth_band: null arguments");
     if (a->H < 0 || a->W < 0 || a->n_pts < 0) return fail(MVS_ERR_VALUE, "depth_band: negative size");
     if (a->block < 1) return fail(MVS_ERR_VALUE, "depth_band: block must be >= 1");
     if (a->H == 0 || a->W == 0) return MVS_OK;
     if (!a->cam || !a->base || !a->step || (a->n_pts >= MVS_BAND_MIN_POINTS && !a->X))
         return fail(MVS_ERR_VALUE, "depth_band: null pointer");
+    return MVS_OK;
+}
+
+extern "C" size_t mvs_depth_band_scratch_bytes(const mvs_depth_band_args* a) {
+    clear_error();
+    if (check_depth_band(a) != MVS_OK) {
+        clear_error();
+        return 0;
+    }
+    if (a->H == 0 || a->W == 0 || a->n_pts < MVS_BAND_MIN_POINTS) return 0;
+    return (size_t)((a->H + a->block - 1) / a->block) * ((a->W + a->block - 1) / a->block) * 20;
+}
+
+extern "C" mvs_status mvs_depth_band_ws(const mvs_depth_band_args* a, void* scratch, size_t scratch_bytes, void* stream) {
+    clear_error();
+    MVS_TRY(check_depth_band(a));
+    if (a->H == 0 || a->W == 0) return MVS_OK;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int gh = (a->H + a->block - 1) / a->block, gw = (a->W + a->block - 1) / a->block;
     const int nb = gh * gw;
     const bool uniform = a->n_pts < MVS_BAND_MIN_POINTS;
-    char* cells = nullptr;
+    unsigned long long *zlo = nullptr, *zhi = nullptr;
+    int* cnt = nullptr;
     if (!uniform) {
-        MVS_CUDA(cudaMallocAsync((void**)&cells, (size_t)nb * 20, st), "depth_band: cell table");
-        unsigned long long* zlo = reinterpret_cast<unsigned long long*>(cells);
-        unsigned long long* zhi = zlo + nb;
-        int* cnt = reinterpret_cast<int*>(zhi + nb);
+        if (!scratch || scratch_bytes < (size_t)nb * 20)
+            return fail(MVS_ERR_VALUE, "depth_band: scratch of %zu bytes below the %zu needed", scratch_bytes, (size_t)nb * 20);
+        zlo = reinterpret_cast<unsigned long long*>(scratch);
+        zhi = zlo + nb;
+        cnt = reinterpret_cast<int*>(zhi + nb);
         TieCam c;
         memcpy(c.c, a->cam, sizeof(c.c));
         band_init_kernel<<<blocks(nb, 256), 256, 0, st>>>(nb, zlo, zhi, cnt);
         band_scatter_kernel<<<blocks(a->n_pts, 256), 256, 0, st>>>(a->n_pts, a->X, c, a->H, a->W, a->block, gw, zlo,
                                                                    zhi, cnt);
     }
-    const unsigned long long* zlo = reinterpret_cast<const unsigned long long*>(cells);
-    const unsigned long long* zhi = uniform ? nullptr : zlo + nb;
-    const int* cnt = uniform ? nullptr : reinterpret_cast<const int*>(zhi + nb);
     band_fill_kernel<<<dim3(blocks(a->W, 256), a->H), 256, 0, st>>>(a->H, a->W, a->block, gh, gw, zlo, zhi, cnt, a->lo,
                                                                    a->hi, a->margin, a->nd, uniform ? 1 : 0, a->base,
                                                                    a->step, a->inv_hi);
-    const mvs_status s = check_launch("depth_band");
+    return check_launch("depth_band");
+}
+
+extern "C" mvs_status mvs_depth_band(const mvs_depth_band_args* a, void* stream) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const size_t need = mvs_depth_band_scratch_bytes(a);
+    void* cells = nullptr;
+    if (need) MVS_CUDA(cudaMallocAsync(&cells, need, st), "depth_band: cell table");
+    const mvs_status s = mvs_depth_band_ws(a, cells, need, stream);
     if (cells) cudaFreeAsync(cells, st);
     return s;
 }

@@ -1796,8 +1796,13 @@ extern "C" uint32_t mvs_pm_stream_advance(uint32_t state, uint64_t n) {
     return state;
 }
 
-extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
-    clear_error();
+namespace {
+
+size_t pm_align(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// MVS_OK and *work = false: nothing to do.
+mvs_status check_pm(const mvs_pm_args* a, bool* work) {
+    *work = false;
     if (!a) return fail(MVS_ERR_VALUE, "pm_refine: null arguments");
     if (a->S == 0 || a->S > MVS_MAX_SOURCES) return MVS_OK;   // the reference returns 0 here
     if (a->S < 0) return fail(MVS_ERR_VALUE, "pm_refine: negative source count");
@@ -1809,6 +1814,86 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
         return fail(MVS_ERR_VALUE, "pm_refine: null pointer");
     if ((long long)a->H * ((a->W + 1) / 2) >= (1LL << 31))
         return fail(MVS_ERR_VALUE, "pm_refine: image of %d x %d pixels is too large", a->W, a->H);
+    for (int s = 0; s < a->S; ++s) {
+        if (!a->src[s]) return fail(MVS_ERR_VALUE, "pm_refine: null source %d", s);
+        if (a->src_h[s] < 2 || a->src_w[s] < 2) return fail(MVS_ERR_VALUE, "pm_refine: source %d smaller than 2x2", s);
+    }
+    if (a->precision != MVS_PM_FP64 && a->precision != MVS_PM_FP32)
+        return fail(MVS_ERR_VALUE, "pm_refine: unknown precision %d", a->precision);
+    *work = true;
+    return MVS_OK;
+}
+
+// Scratch of one call: per pass pixel the propagation result, its flag and stream state; per scan
+// block a count; the stream state (two words, alternating passes), counts and input facts; from the
+// second iteration on, the per-pixel cost cache; float64: both colours' active pixels; float32: the
+// sources' footprints.
+struct PMLayout {
+    bool fast, use_cache;
+    long long n;
+    int nb;
+    size_t flag_bytes, list_bytes;
+    size_t o_best, o_sc, o_state, o_flags, o_bsum, o_rng, o_cache, o_list, o_quad, bytes;
+};
+
+PMLayout pm_layout(const mvs_pm_args* a) {
+    PMLayout l;
+    // float32 evaluation needs pinhole sources (the local map is a homography)
+    l.fast = a->precision == MVS_PM_FP32;
+    for (int s = 0; s < a->S && l.fast; ++s) {
+        const double* q = a->par + 18 * s;
+        l.fast = q[13] == 0.0 && q[14] == 0.0 && q[15] == 0.0;
+    }
+    l.use_cache = a->iters > 1;
+    l.n = (long long)a->H * ((a->W + 1) / 2);
+    l.nb = (int)((l.n + PM_SCAN_BLOCK - 1) / PM_SCAN_BLOCK);
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = o;
+        o += pm_align(bytes);
+        return at;
+    };
+    l.o_best = take(l.n * 8);
+    l.o_sc = take(l.n * 8);
+    l.o_state = take(l.n * 4);
+    l.flag_bytes = pm_align(l.n);
+    l.o_flags = take((l.fast ? 1 : 2) * l.flag_bytes);
+    l.o_bsum = take((size_t)l.nb * 4);
+    l.o_rng = take(256);
+    l.o_cache = take(l.use_cache ? (size_t)a->H * a->W * 2 * sizeof(double) : 0);
+    l.list_bytes = l.fast ? 0 : pm_align((size_t)l.n * 4);
+    l.o_list = take(2 * l.list_bytes);
+    l.o_quad = o;
+    if (l.fast)
+        for (int s = 0; s < a->S; ++s) take((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
+    l.bytes = o;
+    return l;
+}
+
+}  // namespace
+
+extern "C" size_t mvs_pm_scratch_bytes(const mvs_pm_args* a) {
+    clear_error();
+    bool work;
+    if (check_pm(a, &work) != MVS_OK) clear_error();
+    return work ? pm_layout(a).bytes : 0;
+}
+
+extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const size_t need = mvs_pm_scratch_bytes(a);
+    void* scratch = nullptr;
+    if (need) MVS_CUDA(cudaMallocAsync(&scratch, need, st), "pm_refine: scratch");
+    const mvs_status s = mvs_pm_refine_ws(a, scratch, need, stream);
+    if (scratch) cudaFreeAsync(scratch, st);
+    return s;
+}
+
+extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, size_t scratch_bytes, void* stream) {
+    clear_error();
+    bool work;
+    MVS_TRY(check_pm(a, &work));
+    if (!work) return MVS_OK;
     PMParams p;
     memset(&p, 0, sizeof(p));
     p.H = a->H; p.W = a->W; p.S = a->S; p.r = a->r; p.step = a->step; p.top_k = a->top_k;
@@ -1818,8 +1903,6 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
     p.active = a->active;
     p.changed = reinterpret_cast<unsigned long long*>(a->changed);
     for (int s = 0; s < a->S; ++s) {
-        if (!a->src[s]) return fail(MVS_ERR_VALUE, "pm_refine: null source %d", s);
-        if (a->src_h[s] < 2 || a->src_w[s] < 2) return fail(MVS_ERR_VALUE, "pm_refine: source %d smaller than 2x2", s);
         p.img[s] = a->src[s];
         p.dep[s] = a->src_depth[s];
         p.iw[s] = a->src_w[s];
@@ -1829,11 +1912,8 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const long long HW = (long long)a->H * a->W;
-    if (a->precision != MVS_PM_FP64 && a->precision != MVS_PM_FP32)
-        return fail(MVS_ERR_VALUE, "pm_refine: unknown precision %d", a->precision);
-    // float32 evaluation needs pinhole sources (the local map is a homography)
-    bool fast = a->precision == MVS_PM_FP32;
-    for (int s = 0; s < a->S && fast; ++s) fast = p.pinhole[s] != 0;
+    const PMLayout lay = pm_layout(a);
+    const bool fast = lay.fast;
     {
         for (int s = 0; s < a->S; ++s) {
             const double* q = a->par + 18 * s;
@@ -1846,51 +1926,39 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
             for (int k = 0; k < 18; ++k) p.parf[18 * s + k] = (float)q[k];
         }
     }
-    // scratch, one stream-ordered allocation: per pass pixel the propagation result, its flag and
-    // stream state; per scan block a count; the stream state (two words, alternating passes);
-    // from the second iteration on, the per-pixel cost cache
-    const long long n = (long long)a->H * ((a->W + 1) / 2);
-    const int nb = (int)((n + PM_SCAN_BLOCK - 1) / PM_SCAN_BLOCK);
-    const bool use_cache = a->iters > 1;
-    auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-    const size_t o_best = 0, o_sc = o_best + up(n * 8), o_state = o_sc + up(n * 8), o_flags = o_state + up(n * 4);
-    // (float64: flags and list for each colour)
-    const size_t flag_bytes = up(n), o_bsum = o_flags + (fast ? 1 : 2) * flag_bytes, o_rng = o_bsum + up((size_t)nb * 4), o_cache = o_rng + 256;
-    const size_t o_list = o_cache + up(use_cache ? (size_t)HW * 2 * sizeof(double) : 0);
-    const size_t list_bytes = fast ? 0 : up((size_t)n * 4), o_quad = o_list + 2 * list_bytes;
-    size_t quad_bytes = 0;
-    if (fast)
-        for (int s = 0; s < a->S; ++s) quad_bytes += up((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
-    const size_t bytes = o_quad + quad_bytes;
-    char* scratch = nullptr;
-    MVS_CUDA(cudaMallocAsync((void**)&scratch, bytes, st), "pm_refine: scratch");
-    p.pbest = reinterpret_cast<double*>(scratch + o_best);
-    p.psc = reinterpret_cast<double*>(scratch + o_sc);
-    unsigned* pstate = reinterpret_cast<unsigned*>(scratch + o_state);
+    if (!scratch_mem || scratch_bytes < lay.bytes)
+        return fail(MVS_ERR_VALUE, "pm_refine: scratch of %zu bytes below the %zu needed", scratch_bytes, lay.bytes);
+    char* scratch = reinterpret_cast<char*>(scratch_mem);
+    const long long n = lay.n;
+    const int nb = lay.nb;
+    const bool use_cache = lay.use_cache;
+    p.pbest = reinterpret_cast<double*>(scratch + lay.o_best);
+    p.psc = reinterpret_cast<double*>(scratch + lay.o_sc);
+    unsigned* pstate = reinterpret_cast<unsigned*>(scratch + lay.o_state);
     p.pstate = pstate;
-    p.flags = reinterpret_cast<unsigned char*>(scratch + o_flags);
-    unsigned* bsum = reinterpret_cast<unsigned*>(scratch + o_bsum);
-    unsigned* rng = reinterpret_cast<unsigned*>(scratch + o_rng);
+    p.flags = reinterpret_cast<unsigned char*>(scratch + lay.o_flags);
+    unsigned* bsum = reinterpret_cast<unsigned*>(scratch + lay.o_bsum);
+    unsigned* rng = reinterpret_cast<unsigned*>(scratch + lay.o_rng);
     if (use_cache) {
-        p.cost_cache = reinterpret_cast<double*>(scratch + o_cache);
+        p.cost_cache = reinterpret_cast<double*>(scratch + lay.o_cache);
         p.score_cache = p.cost_cache + HW;
         cudaMemsetAsync(p.cost_cache, 0xFF, (size_t)HW * sizeof(double), st);   // all-ones = NaN: recompute
     }
     if (fast) {
-        size_t off = o_quad;
+        size_t off = lay.o_quad;
         for (int s = 0; s < a->S; ++s) {
             float4* q = reinterpret_cast<float4*>(scratch + off);
             p.quad[s] = q;
-            off += up((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
+            off += pm_align((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
             const long long ns = (long long)a->src_w[s] * a->src_h[s];
             const int qb = (int)std::min<long long>((ns + 255) / 256, 148LL * 8);
             pm_quad_kernel<<<qb, 256, 0, st>>>(a->src[s], a->src_w[s], a->src_h[s], q);
         }
     }
-    unsigned char* flags = reinterpret_cast<unsigned char*>(scratch + o_flags);
+    unsigned char* flags = reinterpret_cast<unsigned char*>(scratch + lay.o_flags);
     if (!fast) {
         // pixels that are not active never draw; the input facts and both colours' active pixels
-        cudaMemsetAsync(flags, 0, 2 * flag_bytes, st);
+        cudaMemsetAsync(flags, 0, 2 * lay.flag_bytes, st);
         PMStats* stats = reinterpret_cast<PMStats*>(rng + 8);
         cudaMemsetAsync(stats, 0, sizeof(PMStats), st);
         p.stats = stats;
@@ -1900,7 +1968,7 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
         for (int s = 0; s < a->S; ++s)
             pm_stats_kernel<<<sb, 256, 0, st>>>(a->src[s], (long long)a->src_w[s] * a->src_h[s], stats);
         for (int colour = 0; colour < 2; ++colour) {
-            unsigned* list = reinterpret_cast<unsigned*>(scratch + o_list + colour * list_bytes);
+            unsigned* list = reinterpret_cast<unsigned*>(scratch + lay.o_list + colour * lay.list_bytes);
             pm_active_count_kernel<<<nb, PM_SCAN_BLOCK, 0, st>>>(a->active, a->H, a->W, colour, bsum);
             pm_offsets_kernel<<<1, PM_SCAN_BLOCK, 0, st>>>(bsum, nb, rng + 4 + colour);
             pm_active_list_kernel<<<nb, PM_SCAN_BLOCK, 0, st>>>(a->active, a->H, a->W, colour, bsum, list);
@@ -1970,8 +2038,8 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
         for (int colour = 0; colour < 2 && status == MVS_OK; ++colour) {
             p.colour = colour;
             if (!fast) {
-                p.flags = flags + colour * flag_bytes;
-                p.list = reinterpret_cast<unsigned*>(scratch + o_list + colour * list_bytes);
+                p.flags = flags + colour * lay.flag_bytes;
+                p.list = reinterpret_cast<unsigned*>(scratch + lay.o_list + colour * lay.list_bytes);
                 p.n_list = rng + 4 + colour;
             }
             p.win_smem = (unsigned)smem;
@@ -1995,7 +2063,6 @@ extern "C" mvs_status mvs_pm_refine(const mvs_pm_args* a, void* stream) {
         if (cudaMemcpyAsync(a->rng_state, rng + cur, sizeof(unsigned), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
             status = fail(MVS_ERR_CUDA, "pm_refine: stream state copy");
     }
-    cudaFreeAsync(scratch, st);
     return status;
 }
 

@@ -380,6 +380,45 @@ extern "C" mvs_status mvs_sweep(const mvs_sweep_args* a, void* stream) {
     return s;
 }
 
+extern "C" size_t mvs_sweep_scratch_bytes(const mvs_sweep_args* a) {
+    clear_error();
+    int nch = 1;
+    if (validate_sweep(a) != MVS_OK) {
+        clear_error();
+        return 0;
+    }
+    return a->H == 0 || a->W == 0 || a->i1 == a->i0 ? 0 : sweep_scratch_bytes(a, &nch);
+}
+
+extern "C" mvs_status mvs_sweep_ws(const mvs_sweep_args* a, void* scratch, size_t scratch_bytes, void* stream) {
+    clear_error();
+    MVS_TRY(validate_sweep(a));
+    if (a->H == 0 || a->W == 0 || a->i1 == a->i0) return MVS_OK;
+    return sweep_with_scratch(a, scratch, scratch ? scratch_bytes : 0, reinterpret_cast<cudaStream_t>(stream));
+}
+
+namespace mvs {
+__global__ void __launch_bounds__(256) state_init_kernel(long long n, float* best, float* prev, float* spb, float* snb,
+                                                         int* idx) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    best[i] = prev[i] = spb[i] = snb[i] = -2.f;
+    idx[i] = -1;
+}
+}  // namespace mvs
+
+extern "C" mvs_status mvs_sweep_state_init(int32_t H, int32_t W, float* best, float* prev, float* s_prev_best,
+                                           float* s_next_best, int32_t* idx, void* stream) {
+    clear_error();
+    if (H < 0 || W < 0) return fail(MVS_ERR_VALUE, "state_init: negative shape");
+    if (H == 0 || W == 0) return MVS_OK;
+    if (!best || !prev || !s_prev_best || !s_next_best || !idx) return fail(MVS_ERR_VALUE, "state_init: null pointer");
+    const long long n = (long long)H * W;
+    state_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        n, best, prev, s_prev_best, s_next_best, idx);
+    return check_launch("state init");
+}
+
 extern "C" mvs_status mvs_sweep_hypothesis(int32_t H, int32_t W, const float* ref, const float* mu_i,
                                            const float* sd_i, int32_t n_src, const float* const* srcs,
                                            const int32_t* src_h, const int32_t* src_w, const float* ray,

@@ -188,9 +188,15 @@ def sweep_args(ref, mu, sd, ray, srcs, geo, ref_cam, hyp: Hypotheses, r, top_k, 
 
 def new_state(H: int, W: int, device=None):
     """Initial winner-take-all state (densify.py:331-335): best/prev/spb/snb = -2, idx = -1."""
-    device = device or L.require_cuda()
-    f = [torch.full((H, W), -2.0, dtype=torch.float32, device=device) for _ in range(4)]
-    return (*f, torch.full((H, W), -1, dtype=torch.int32, device=device))
+    device = torch.device(device or L.require_cuda())
+    if device.type != "cuda":
+        f = [torch.full((H, W), -2.0, dtype=torch.float32, device=device) for _ in range(4)]
+        return (*f, torch.full((H, W), -1, dtype=torch.int32, device=device))
+    st = [torch.empty((H, W), dtype=torch.float32, device=device) for _ in range(4)]
+    st.append(torch.empty((H, W), dtype=torch.int32, device=device))
+    with torch.cuda.device(device):
+        L.check(L.load().mvs_sweep_state_init(H, W, *(t.data_ptr() for t in st), L.stream_handle()), "new_state")
+    return tuple(st)
 
 
 def sweep(ref, mu, sd, ray, srcs, geo, hyp: Hypotheses, r: int, top_k: int, state=None, ref_cam=None,
@@ -204,7 +210,7 @@ def sweep(ref, mu, sd, ray, srcs, geo, hyp: Hypotheses, r: int, top_k: int, stat
         state = new_state(H, W, ref.device)
     a, keep = sweep_args(ref, mu, sd, ray, srcs, geo, ref_cam, hyp, r, top_k, state, precision=precision,
                          plane_chunks=plane_chunks, tile_h=tile_h)
-    L.check(L.load().mvs_sweep(C_addr(a), L.stream_handle(stream)), "sweep")
+    L.check(L.call_with_scratch("mvs_sweep", C_addr(a), ref.device, stream), "sweep")
     del keep
     return state
 
@@ -292,7 +298,7 @@ def pm_refine(ref, ray, Cr, srcs: Sequence, src_depths: Sequence, par, depth, no
                     and rng_state.dtype == torch.int32 and rng_state.device == ref_t.device):
                 raise ValueError("pm_refine: rng_state must be a 1-element int32 tensor on the image's device")
             a.rng_state = rng_state.data_ptr()
-        L.check(L.load().mvs_pm_refine(C_addr(a), L.stream_handle()), "pm_refine")
+        L.check(L.call_with_scratch("mvs_pm_refine", C_addr(a), ref_t.device), "pm_refine")
         out = int(changed.item())
         D.close()
         return out

@@ -188,7 +188,7 @@ def _sweep_maps(ref, cam_r, srcs, cams_s, inv_list, opt, ray, block: int = 32):
             first2 = [maps[0]] + ([maps[1]] if i1 > 1 else [])
         hyp = Hypotheses(L.HYP_MAPS, n, maps=maps)
         a, keep = sweep_args(ref_t, mu, sd, ray_t, src_t, geo, None, hyp, r, int(opt.top_k), state, i0=i0, i1=i1)
-        L.check(L.load().mvs_sweep(C_addr(a), L.stream_handle()), "sweep")
+        L.check(L.call_with_scratch("mvs_sweep", C_addr(a), ref_t.device), "sweep")
         del keep
     fin = torch.stack(first2) if len(first2) == 2 else torch.stack([first2[0], first2[0]])
     depth = finalize(Hypotheses(L.HYP_MAPS, n, maps=fin), state)
@@ -246,7 +246,7 @@ def _band_maps(rec, k, cam, shape, rng, nd: int, block: int = 32, margin: float 
     a.lo, a.hi, a.margin = float(rng[0]), float(rng[1]), float(margin)
     a.nd = int(nd)
     a.base, a.step, a.inv_hi = (t.data_ptr() for t in out)
-    L.check(L.load().mvs_depth_band(C_addr(a), L.stream_handle()), "depth_band")
+    L.check(L.call_with_scratch("mvs_depth_band", C_addr(a), dev), "depth_band")
     return tuple(out)
 
 

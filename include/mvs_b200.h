@@ -487,10 +487,48 @@ mvs_status mvs_device_faults(uint32_t* count);
  * for its copy in flight to land and returns with its state untouched. Applies to calls made
  * after it, from any thread. No counterpart in the reference. */
 uint32_t mvs_set_wait_limit(uint32_t iterations);
+/* One photo-consistency evaluation of a height stack: every view's samples (mvs_sample_view on
+ * one-channel images), all window means (mvs_box_sat_mean of the samples, their squares, the valid
+ * masks and the pair products) and mvs_height_score, in three launches and with their values. The grid
+ * must fit the window means' shared memory ((32 + 2 r + 1) (W + 1) doubles within 200 KB, W <= 1024;
+ * D <= 65535), else MVS_ERR_UNSUPPORTED: then call the parts. Scratch (256-byte aligned device
+ * memory, mvs_height_eval_scratch_bytes; 0 for arguments that it rejects) is the caller's. */
+typedef struct mvs_height_eval_args {
+    int32_t V, D, H, W, r, topk;
+    double X0, Y0, gsd;                    /* ground grid, as mvs_sample_view_args               */
+    const float* img[MVS_MAX_SOURCES];     /* per view (img_h, img_w) grey                      */
+    int32_t img_h[MVS_MAX_SOURCES], img_w[MVS_MAX_SOURCES];
+    const double* cams;                    /* HOST (V, 18) R(9) C(3) f k1 k2 k3 cx cy, image pixels */
+    const float* Z;                        /* (D, H, W) heights                                 */
+    const float* cxs;                      /* (W) cell centres, X                               */
+    const float* cys;                      /* (H) cell centres, Y                               */
+    double full, min_texture, full_texture;
+    uint8_t* valid;                        /* out (V, D, H, W)                                  */
+    float* score;                          /* out (D, H, W)                                     */
+    float* st;                             /* out (V, D, H, W), or NULL                         */
+    int32_t* ref;                          /* out (D, H, W), or NULL                            */
+} mvs_height_eval_args;
+size_t mvs_height_eval_scratch_bytes(const mvs_height_eval_args* args);
+mvs_status mvs_height_eval(const mvs_height_eval_args* args, void* scratch, size_t scratch_bytes, void* stream);
+
+/* The refinement around a coarser surface Zc (hc, wc), float32 in NumPy's order (mvs.py:305-340): `up` =
+ * Zc repeated 2 x 2, cropped or edge-padded to (H, W), and stack (K, H, W) = up + offs[k];
+ * mvs_height_pick: the first best of K scores (below `weak`: the middle one), with `parabola` its
+ * vertex: out = (up + offs[b]) + frac * cell; mvs_median3: 3 x 3 median, edge padding. */
+mvs_status mvs_height_stack(int32_t H, int32_t W, int32_t hc, int32_t wc, const float* Zc, int32_t K,
+                            const float* offs, float* up, float* stack, void* stream);
+mvs_status mvs_height_pick(int32_t H, int32_t W, int32_t K, const float* score, const float* up, const float* offs,
+                           float weak, int32_t parabola, float cell, float* out, void* stream);
+mvs_status mvs_median3(int32_t H, int32_t W, const float* a, float* out, void* stream);
+
 
 /* Bounds-checked debug build only (libmvs_b200_debug.so, compiled with MVS_DEBUG_BOUNDS): the
  * number of shared-memory and global indices the tile engine, the batched kernels and PatchMatch
  * used outside their buffers since the last call (synchronises; clears the counts). Release
+/* mvs_sgm with its scratch given by the caller (8 volumes up to 256 hypotheses, else one). */
+size_t mvs_sgm_scratch_bytes(int32_t D, int32_t H, int32_t W);
+mvs_status mvs_sgm_ws(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
+                      void* scratch, size_t scratch_bytes, void* stream);
  * builds return MVS_ERR_UNSUPPORTED. No counterpart in the reference (its Cython kernels are
  * compiled with boundscheck=False). */
 mvs_status mvs_debug_bound_violations(uint32_t* count);

@@ -98,6 +98,14 @@ class BatchJob(C.Structure):
 
 class BatchTuning(C.Structure):
     _fields_ = [("plane_chunk", i32), ("ctas_per_sm", i32), ("tile_h", i32)]
+class HeightEvalArgs(C.Structure):
+    _fields_ = [("V", i32), ("D", i32), ("H", i32), ("W", i32), ("r", i32), ("topk", i32), ("X0", C.c_double),
+                ("Y0", C.c_double), ("gsd", C.c_double), ("img", vp * MAX_SOURCES), ("img_h", i32 * MAX_SOURCES),
+                ("img_w", i32 * MAX_SOURCES), ("cams", vp), ("Z", vp), ("cxs", vp), ("cys", vp), ("full", C.c_double),
+                ("min_texture", C.c_double), ("full_texture", C.c_double), ("valid", vp), ("score", vp), ("st", vp),
+                ("ref", vp)]
+
+
 
 
 # name -> (restype, argtypes); every symbol the header declares
@@ -148,7 +156,14 @@ SIGNATURES = {
     "mvs_version": (C.c_char_p, []),
 }
 
+    "mvs_height_eval_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_height_eval": (i32, [vp, vp, C.c_size_t, vp]),
+    "mvs_height_stack": (i32, [i32, i32, i32, i32, vp, i32, vp, vp, vp, vp]),
+    "mvs_height_pick": (i32, [i32, i32, i32, vp, vp, vp, C.c_float, i32, C.c_float, vp, vp]),
+    "mvs_median3": (i32, [i32, i32, vp, vp, vp]),
 _lib = None
+    "mvs_sgm_scratch_bytes": (C.c_size_t, [i32, i32, i32]),
+    "mvs_sgm_ws": (i32, [i32, i32, i32, vp, C.c_float, C.c_float, vp, vp, C.c_size_t, vp]),
 _lock = threading.Lock()
 
 

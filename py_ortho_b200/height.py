@@ -68,17 +68,20 @@ def _dev():
 
 
 # ------------------------------------------------------------------ kernels
-def sample_view(img: torch.Tensor, cam, X0: float, Y0: float, gsd: float, Z: torch.Tensor):
+def sample_view(img: torch.Tensor, cam, X0: float, Y0: float, gsd: float, Z: torch.Tensor, out=None, valid=None):
     """backend.sample_view (backend.py:67-76): img (h, w, ch) float32 on the device, cam = (R, C, f,
-    k1, k2, k3, cx, cy) in img pixels, Z (H, W) or (D, H, W) heights -> (samples (..., ch), valid)."""
+    k1, k2, k3, cx, cy) in img pixels, Z (H, W) or (D, H, W) heights -> (samples (..., ch), valid),
+    written to `out` and `valid` when given."""
     img = img.contiguous()
     Zs = Z.to(torch.float32).contiguous()
     lead = Zs.shape[:-2]
     D = int(np.prod(lead)) if len(lead) else 1
     H, W = int(Zs.shape[-2]), int(Zs.shape[-1])
     h, w, nch = (int(v) for v in img.shape)
-    out = torch.empty(tuple(Zs.shape) + (nch,), dtype=torch.float32, device=img.device)
-    valid = torch.empty(tuple(Zs.shape), dtype=torch.uint8, device=img.device)
+    if out is None:
+        out = torch.empty(tuple(Zs.shape) + (nch,), dtype=torch.float32, device=img.device)
+    if valid is None:
+        valid = torch.empty(tuple(Zs.shape), dtype=torch.uint8, device=img.device)
     R, C, f, k1, k2, k3, cx, cy = cam
     row = L.host_f64(np.r_[np.asarray(R, np.float64).ravel(), np.asarray(C, np.float64), [f, k1, k2, k3, cx, cy]])
     a = L.SampleViewArgs()
@@ -104,8 +107,11 @@ def sgm(cost: torch.Tensor, P1: float, P2: float) -> torch.Tensor:
     cost = cost.to(torch.float32).contiguous()
     D, H, W = (int(v) for v in cost.shape)
     agg = torch.empty_like(cost)
-    L.check(L.load().mvs_sgm(D, H, W, cost.data_ptr(), float(P1), float(P2), agg.data_ptr(), L.stream_handle()),
-            "sgm")
+    lib = L.load()
+    need = lib.mvs_sgm_scratch_bytes(D, H, W)
+    ws = torch.empty(need, dtype=torch.uint8, device=cost.device)
+    L.check(lib.mvs_sgm_ws(D, H, W, cost.data_ptr(), float(P1), float(P2), agg.data_ptr(), ws.data_ptr(), need,
+                           L.stream_handle()), "sgm")
     return agg
 
 
@@ -261,9 +267,11 @@ def _serpentine(W: int, H: int, T: int):
 
 def _median3(a: torch.Tensor) -> torch.Tensor:
     """3x3 median with edge padding (mvs._median3, mvs.py:64-68): the middle of the 9 sorted shifts."""
-    p = torch.nn.functional.pad(a[None, None], (1, 1, 1, 1), mode="replicate")[0, 0]
-    H, W = a.shape
-    return torch.sort(torch.stack([p[dy:dy + H, dx:dx + W] for dy in range(3) for dx in range(3)]), dim=0).values[4]
+    a = a.contiguous()
+    out = torch.empty_like(a)
+    L.check(L.load().mvs_median3(int(a.shape[0]), int(a.shape[1]), a.data_ptr(), out.data_ptr(), L.stream_handle()),
+            "median3")
+    return out
 
 
 # ------------------------------------------------------------------ one tile on the device
@@ -279,34 +287,72 @@ class _TileSweep:
         ia, ib = np.triu_indices(V, 1)
         self.ia = torch.as_tensor(ia, device=dev)
         self.ib = torch.as_tensor(ib, device=dev)
+        self.centres = {}
 
     def score(self, Z: torch.Tensor, level: int, gsd_l: float, detail: bool = False):
         """Photo-consistency of every cell of the height stack Z (..., HH, WW): the samples of every
-        view, all box means in one call, then the fused per-cell score kernel."""
+        view, all window means, the score (mvs_height_eval; a grid too wide for it in its parts)."""
         t, V, dev, opt = self.t, len(self.views), self.dev, self.opt
+        Z = Z.to(torch.float32).contiguous()
         HH, WW = int(Z.shape[-2]), int(Z.shape[-1])
-        smp, val = [], []
-        for v in self.views:
-            out, ok = sample_view(v.pyr[min(level, len(v.pyr) - 1)], v.cam(level), t.X0, t.Y0, gsd_l, Z)
-            smp.append(out[..., 0])
-            val.append(ok)
-        S = torch.stack(smp)
-        boxes = box(torch.cat([S, S * S, torch.stack(val).to(torch.float32), S[self.ia] * S[self.ib]]), opt.window)
         lead = tuple(Z.shape[:-2])
         score = torch.empty(lead + (HH, WW), dtype=torch.float32, device=dev)
         st = torch.empty((V,) + lead + (HH, WW), dtype=torch.float32, device=dev) if detail else None
         ref = torch.empty(lead + (HH, WW), dtype=torch.int32, device=dev) if detail else None
-        cxs = torch.as_tensor(np.asarray(t.X0 + (np.arange(WW) + 0.5) * gsd_l, np.float32), device=dev)
-        cys = torch.as_tensor(np.asarray(t.Y0 - (np.arange(HH) + 0.5) * gsd_l, np.float32), device=dev)
+        val = torch.empty((V,) + lead + (HH, WW), dtype=torch.uint8, device=dev)
+        cxs, cys = self._centres(HH, WW, gsd_l)
+        imgs = [v.pyr[min(level, len(v.pyr) - 1)] for v in self.views]
+        cams = L.host_f64(np.stack([np.r_[np.asarray(c[0], np.float64).ravel(), np.asarray(c[1], np.float64), c[2:]]
+                                    for c in (v.cam(level) for v in self.views)]))
+        if V > L.MAX_SOURCES:
+            raise ValueError(f"height score: {V} views (at most {L.MAX_SOURCES})")
+        a = L.HeightEvalArgs()
+        a.V, a.D, a.H, a.W, a.r, a.topk = V, int(np.prod(lead)) if lead else 1, HH, WW, int(opt.window), self.topk
+        a.X0, a.Y0, a.gsd = float(t.X0), float(t.Y0), float(gsd_l)
+        for k, im in enumerate(imgs):
+            a.img[k], a.img_h[k], a.img_w[k] = im.data_ptr(), int(im.shape[0]), int(im.shape[1])
+        a.cams, a.Z, a.cxs, a.cys = L.host_ptr(cams), Z.data_ptr(), cxs.data_ptr(), cys.data_ptr()
+        a.full, a.min_texture, a.full_texture = 1.0 - 1e-6, float(opt.min_texture), float(opt.full_texture)
+        a.valid, a.score = val.data_ptr(), score.data_ptr()
+        a.st, a.ref = (st.data_ptr(), ref.data_ptr()) if detail else (0, 0)
+        lib = L.load()
+        need = lib.mvs_height_eval_scratch_bytes(ctypes.addressof(a))
+        ws = torch.empty(need, dtype=torch.uint8, device=dev)
+        status = lib.mvs_height_eval(ctypes.addressof(a), ws.data_ptr(), need, L.stream_handle())
+        if status == L.ERR_UNSUPPORTED:
+            self._score_parts(Z, level, gsd_l, score, st, ref, val, cxs, cys)
+        else:
+            L.check(status, "height score")
+        return (score, st, val, ref.to(torch.int64)) if detail else score
+
+    def _centres(self, HH, WW, gsd_l):
+        """Cell centres of the padded tile at cell size gsd_l (float32, on the device)."""
+        key = (HH, WW, gsd_l)
+        if key not in self.centres:
+            t = self.t
+            xy = np.r_[np.asarray(t.X0 + (np.arange(WW) + 0.5) * gsd_l, np.float32),
+                       np.asarray(t.Y0 - (np.arange(HH) + 0.5) * gsd_l, np.float32)]
+            d = torch.as_tensor(xy, device=self.dev)
+            self.centres[key] = (d[:WW], d[WW:])
+        return self.centres[key]
+
+    def _score_parts(self, Z, level, gsd_l, score, st, ref, val, cxs, cys):
+        """The score by its separate kernels, into the given outputs."""
+        t, V, opt = self.t, len(self.views), self.opt
+        smp = []
+        for k, v in enumerate(self.views):
+            out, _ = sample_view(v.pyr[min(level, len(v.pyr) - 1)], v.cam(level), t.X0, t.Y0, gsd_l, Z, valid=val[k])
+            smp.append(out[..., 0])
+        S = torch.stack(smp)
+        boxes = box(torch.cat([S, S * S, val.to(torch.float32), S[self.ia] * S[self.ib]]), opt.window)
         a = L.HeightScoreArgs()
-        a.V, a.D, a.H, a.W, a.topk = V, int(np.prod(lead)) if lead else 1, HH, WW, self.topk
+        a.V, a.D, a.H, a.W, a.topk = V, score.numel() // (score.shape[-2] * score.shape[-1]), *score.shape[-2:], self.topk
         a.full, a.min_texture, a.full_texture = 1.0 - 1e-6, float(opt.min_texture), float(opt.full_texture)
         a.M, a.S2, a.VA, a.PP = (boxes[:V].data_ptr(), boxes[V:2 * V].data_ptr(), boxes[2 * V:3 * V].data_ptr(),
                                  boxes[3 * V:].data_ptr())
         a.cxs, a.cys, a.cam_xy, a.score = cxs.data_ptr(), cys.data_ptr(), L.host_ptr(self.cam_xy), score.data_ptr()
-        a.st, a.ref = (st.data_ptr(), ref.data_ptr()) if detail else (0, 0)
+        a.st, a.ref = (0, 0) if st is None else (st.data_ptr(), ref.data_ptr())
         L.check(L.load().mvs_height_score(ctypes.addressof(a), L.stream_handle()), "height score")
-        return (score, st, val, ref.to(torch.int64)) if detail else score
 
     def coarse(self, level, zlo, zhi):
         """Every height from zlo to zhi in steps of one cell, 64 at a time; cost 1 - score,
@@ -314,11 +360,11 @@ class _TileSweep:
         t, dev = self.t, self.dev
         s = 2 ** level
         HH, WW, gsd_l = (t.PH + s - 1) // s, (t.PW + s - 1) // s, self.gsd * s
-        zs = np.arange(zlo, zhi + gsd_l, gsd_l).astype(np.float32)
-        vol = torch.cat([self.score(torch.as_tensor(zs[c:c + 64], device=dev)[:, None, None].expand(-1, HH, WW)
-                                    .contiguous(), level, gsd_l) for c in range(0, len(zs), 64)])
+        zs = torch.as_tensor(np.arange(zlo, zhi + gsd_l, gsd_l).astype(np.float32), device=dev)
+        vol = torch.cat([self.score(zs[c:c + 64, None, None].expand(-1, HH, WW), level, gsd_l)
+                         for c in range(0, len(zs), 64)])
         agg = sgm((1.0 - torch.clamp(vol, -1.0, 1.0)).contiguous(), self.opt.sgm_p1, self.opt.sgm_p2)
-        return torch.as_tensor(zs, device=dev)[torch.argmin(agg, dim=0)]
+        return zs[torch.argmin(agg, dim=0)]
 
     def refine(self, Zc, level):
         """+-refine_steps cells around the upsampled coarser surface; cells whose best score is
@@ -326,47 +372,45 @@ class _TileSweep:
         t, opt, dev = self.t, self.opt, self.dev
         s = 2 ** level
         HH, WW, gsd_l = (t.PH + s - 1) // s, (t.PW + s - 1) // s, self.gsd * s
-        up = Zc.repeat_interleave(2, 0).repeat_interleave(2, 1)[:HH, :WW]
-        if tuple(up.shape) != (HH, WW):
-            up = torch.nn.functional.pad(up[None, None], (0, WW - up.shape[1], 0, HH - up.shape[0]),
-                                         mode="replicate")[0, 0]
         n = opt.refine_steps
         offs = torch.as_tensor((np.arange(-n, n + 1) * gsd_l).astype(np.float32), device=dev)
-        sc = self.score((up[None] + offs[:, None, None]).to(torch.float32), level, gsd_l)
-        bi = torch.argmax(sc, dim=0)
-        pick = lambda i: torch.gather(sc, 0, i[None])[0]
-        bi = torch.where(pick(bi) < np.float32(opt.refine_min_score), torch.full_like(bi, n), bi)
-        best = pick(bi)
-        frac = torch.zeros_like(best)
-        if level == 0:
-            s_lo, s_hi = pick(torch.clamp(bi - 1, 0, 2 * n)), pick(torch.clamp(bi + 1, 0, 2 * n))
-            den = s_lo - 2 * best + s_hi
-            ok = (den < np.float32(-1e-6)) & (bi > 0) & (bi < 2 * n)
-            den = torch.where(ok, den, torch.full_like(den, -1.0))
-            frac = torch.where(ok, torch.clamp(0.5 * (s_lo - s_hi) / den, -0.5, 0.5), torch.zeros_like(den))
-        return up + offs[bi] + frac * np.float32(gsd_l)
+        Zc = Zc.contiguous()
+        up = torch.empty((HH, WW), dtype=torch.float32, device=dev)
+        stack = torch.empty((2 * n + 1, HH, WW), dtype=torch.float32, device=dev)
+        lib, sh = L.load(), L.stream_handle()
+        L.check(lib.mvs_height_stack(HH, WW, int(Zc.shape[0]), int(Zc.shape[1]), Zc.data_ptr(), 2 * n + 1, offs.data_ptr(),
+                                     up.data_ptr(), stack.data_ptr(), sh), "height stack")
+        sc = self.score(stack, level, gsd_l)
+        out = torch.empty_like(up)
+        L.check(lib.mvs_height_pick(HH, WW, 2 * n + 1, sc.data_ptr(), up.data_ptr(), offs.data_ptr(),
+                                    float(np.float32(opt.refine_min_score)), 1 if level == 0 else 0,
+                                    float(np.float32(gsd_l)), out.data_ptr(), sh), "height pick")
+        return out
 
     def colour(self, Z, st, ref):
         """True-ortho colour at the chosen heights: feather^2 x agreement with the cell's reference
         x validity x cos(incidence)^power weighted mean of the views' RGB."""
-        t, dev = self.t, self.dev
-        cx = torch.as_tensor((t.X0 + (np.arange(t.PW) + 0.5) * self.gsd).astype(np.float32), device=dev)
-        cy = torch.as_tensor((t.Y0 - (np.arange(t.PH) + 0.5) * self.gsd).astype(np.float32), device=dev)
+        t, dev, V = self.t, self.dev, len(self.views)
+        cx, cy = self._centres(t.PH, t.PW, self.gsd)
         p = float(self.opt.view_angle_power)
+        rgbw = torch.empty((V,) + tuple(Z.shape) + (4,), dtype=torch.float32, device=dev)
+        ok = torch.empty((V,) + tuple(Z.shape), dtype=torch.uint8, device=dev)
+        for k, v in enumerate(self.views):
+            sample_view(v.rgbw, v.cam(0), t.X0, t.Y0, self.gsd, Z, out=rgbw[k], valid=ok[k])
+        ids = torch.arange(V, device=dev)[:, None, None]
+        agree = torch.where(ref[None] == ids, torch.ones_like(st),
+                            torch.clamp((st + np.float32(0.2)) / np.float32(0.6), 0.0, 1.0))
+        C = torch.as_tensor(np.array(self.cams).astype(np.float32), device=dev)
+        dz = C[:, 2, None, None] - Z[None]
+        dx = cx[None, None, :] - C[:, 0, None, None]
+        dy = cy[None, :, None] - C[:, 1, None, None]
+        cos_inc = torch.clamp(dz / torch.sqrt(dx * dx + dy * dy + dz * dz + np.float32(1e-6)), 0.0, 1.0)
+        w = rgbw[..., 3] ** 2 * agree * ok.to(torch.float32) * cos_inc ** p
         acc = torch.zeros(tuple(Z.shape) + (3,), dtype=torch.float32, device=dev)
         wsum = torch.zeros(tuple(Z.shape), dtype=torch.float32, device=dev)
-        for vi, v in enumerate(self.views):
-            rgbw, ok = sample_view(v.rgbw, v.cam(0), t.X0, t.Y0, self.gsd, Z)
-            agree = torch.where(ref == vi, torch.ones_like(st[vi]),
-                                torch.clamp((st[vi] + np.float32(0.2)) / np.float32(0.6), 0.0, 1.0))
-            C = self.cams[vi]
-            dz = np.float32(C[2]) - Z
-            dx = cx[None, :] - np.float32(C[0])
-            dy = cy[:, None] - np.float32(C[1])
-            cos_inc = torch.clamp(dz / torch.sqrt(dx * dx + dy * dy + dz * dz + np.float32(1e-6)), 0.0, 1.0)
-            w = rgbw[..., 3] ** 2 * agree * ok.to(torch.float32) * cos_inc ** p
-            acc = acc + rgbw[..., :3] * w[..., None]
-            wsum = wsum + w
+        for vi in range(V):
+            acc = acc + rgbw[vi, ..., :3] * w[vi, ..., None]
+            wsum = wsum + w[vi]
         return acc / torch.clamp(wsum, min=1e-6)[..., None]
 
 
@@ -413,7 +457,7 @@ def dense_reconstruct(ar, rec, gains: dict, native_gsd: float, opt: DenseOptions
             Z = _median3(Z.to(torch.float32)) if level > 0 else Z.to(torch.float32)
         score, st, valids, ref = sw.score(Z, 0, g.gsd, detail=True)
         colour = sw.colour(Z, st, ref)
-        nvalid = sum(v.to(torch.int32) for v in valids)
+        nvalid = valids.sum(0, dtype=torch.int32)
         # heights leave the tile with an overlap margin, blended by a linear ramp
         e = (max(0, tx - ov), max(0, ty - ov), min(g.W, tx + tw + ov), min(g.H, ty + th + ov))
         ry, rx = np.arange(e[1], e[3]), np.arange(e[0], e[2])

@@ -421,6 +421,25 @@ typedef struct mvs_fuse_args {
  * after another in the reference's order (sorted view index) on one stream. Bit-exact. */
 mvs_status mvs_fuse_view(const mvs_fuse_args* args, void* stream);
 
+/* Appends the points that a mvs_fuse_view call kept, in row-major order, to growing output arrays: the
+ * number of points stays on the device from view to view, so that the host reads it once for many
+ * views. The arrays hold at least rows[0] + the view's stride-grid pixels. */
+typedef struct mvs_fuse_append_args {
+    int32_t H, W, point_stride, owner;     /* owner: the view's id                               */
+    const uint8_t* keep;                   /* mvs_fuse_args' outputs                            */
+    const double* xyz;
+    const int32_t* count;
+    const uint8_t* rgb;                    /* (H, W, 3) the view's colours                      */
+    int64_t* rows;                         /* DEVICE (2): in/out number of points; work word     */
+    double* out_xyz;                       /* (capacity, 3)                                     */
+    uint8_t* out_rgb;                      /* (capacity, 3)                                     */
+    uint8_t* out_views;                    /* (capacity) min(count, 255)                        */
+    int32_t* out_owner;                    /* (capacity)                                        */
+    void* scratch;                         /* mvs_fuse_append_scratch_bytes                     */
+} mvs_fuse_append_args;
+size_t mvs_fuse_append_scratch_bytes(int32_t H, int32_t W, int32_t point_stride);
+mvs_status mvs_fuse_append(const mvs_fuse_append_args* args, void* stream);
+
 /* ---------------------------------------------------------------- legacy height sweep (mvs.py) */
 
 typedef struct mvs_sample_view_args {

@@ -73,6 +73,12 @@ class FuseArgs(C.Structure):
                 ("count", vp)]
 
 
+class FuseAppendArgs(C.Structure):
+    _fields_ = [("H", i32), ("W", i32), ("point_stride", i32), ("owner", i32), ("keep", vp), ("xyz", vp), ("count", vp),
+                ("rgb", vp), ("rows", vp), ("out_xyz", vp), ("out_rgb", vp), ("out_views", vp), ("out_owner", vp),
+                ("scratch", vp)]
+
+
 class SampleViewArgs(C.Structure):
     _fields_ = [("h", i32), ("w", i32), ("nch", i32), ("img", vp), ("cam", vp), ("X0", C.c_double),
                 ("Y0", C.c_double), ("gsd", C.c_double), ("D", i32), ("H", i32), ("W", i32), ("Z", vp),
@@ -145,6 +151,8 @@ SIGNATURES = {
     "mvs_depth_band_scratch_bytes": (C.c_size_t, [vp]),
     "mvs_depth_band_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_box_sat_mean": (i32, [i32, i32, i32, vp, i32, vp, vp]),
+    "mvs_fuse_append": (i32, [vp, vp]),
+    "mvs_fuse_append_scratch_bytes": (C.c_size_t, [i32, i32, i32]),
     "mvs_pm_scratch_bytes": (C.c_size_t, [vp]),
     "mvs_pm_refine_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_height_score": (i32, [vp, vp]),

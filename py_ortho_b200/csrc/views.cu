@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(256) init_normals_kernel(int H, int W, const f
 // to the pixel's own (acc starts at X, cnt at 1), kept when cnt >= min_views, and the agreeing
 // neighbours' stride-grid pixels marked as used. Views run one launch after another (the marks
 // of a view gate the candidates of the later ones); within a launch only other views' masks are
-// written, and only with 1.
+// written, and only with 1. One thread per stride-grid pixel (the other pixels emit nothing; the
+// launcher clears their keep and count): a thread per pixel left 3 of 4 lanes idle at stride 2.
 struct FuseParams {
     int H, W, n_nb, min_views, stride;
     double px_tol;
@@ -222,14 +223,13 @@ struct FuseParams {
 
 __global__ void __launch_bounds__(256) fuse_kernel(const __grid_constant__ FuseParams c) {
     const long long HW = (long long)c.H * c.W;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= HW) return;
-    const int y = (int)(idx / c.W), x = (int)(idx - (long long)y * c.W);
-    const int st = c.stride;
+    const int st = c.stride, gw = (c.W + st - 1) / st;
+    const long long cand = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = (int)(cand / gw) * st, x = (int)(cand % gw) * st;
+    if (y >= c.H) return;
+    const long long idx = (long long)y * c.W + x;
     const float Dv = c.depth[idx];
-    c.keep[idx] = 0;
-    c.count[idx] = 0;
-    if (!isfinite(Dv) || c.used[idx] || (st > 1 && (y % st != 0 || x % st != 0))) return;
+    if (!isfinite(Dv) || c.used[idx]) return;
     const double* R = c.cam;
     const double* C = c.cam + 9;
     const double d = (double)Dv;
@@ -293,6 +293,97 @@ __global__ void __launch_bounds__(256) fuse_kernel(const __grid_constant__ FuseP
     c.xyz[2 * HW + idx] = __ddiv_rn(a2, dc);
     for (int j = 0; j < c.n_nb; ++j)
         if (okbits & (1u << j)) c.nb_used[j][mark[j]] = 1;
+}
+
+// ---- the kept points of one fused view, appended in row-major order (mvs_fuse_append)
+struct AppendParams {
+    int H, W, stride, owner;
+    const unsigned char* keep;
+    const double* xyz;
+    const int* count;
+    const unsigned char* rgb;              // (H, W, 3)
+    unsigned* bsum;
+    long long* rows;                       // running number of points
+    double* o_xyz;                         // (capacity, 3)
+    unsigned char* o_rgb;                  // (capacity, 3)
+    unsigned char* o_views;                // (capacity)
+    int* o_owner;                          // (capacity)
+};
+constexpr int APPEND_BLOCK = 1024;
+
+__device__ __forceinline__ bool append_kept(const AppendParams& c, long long cand, long long& idx) {
+    const int gw = (c.W + c.stride - 1) / c.stride;
+    const long long y = cand / gw * c.stride, x = cand % gw * c.stride;
+    if (y >= c.H) return false;
+    idx = y * c.W + x;
+    return c.keep[idx] != 0;
+}
+
+__global__ void __launch_bounds__(APPEND_BLOCK) append_count_kernel(const __grid_constant__ AppendParams c) {
+    long long idx;
+    const int n = __syncthreads_count(append_kept(c, (long long)blockIdx.x * APPEND_BLOCK + threadIdx.x, idx));
+    if (threadIdx.x == 0) c.bsum[blockIdx.x] = (unsigned)n;
+}
+
+// Exclusive prefix over the block's threads (32 warps); total = the block's sum.
+__device__ __forceinline__ unsigned append_scan(unsigned v, unsigned& total) {
+    __shared__ unsigned part[33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) part[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+        unsigned s = part[lane];
+        const unsigned own = s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        part[lane] = s - own;
+        if (lane == 31) part[32] = s;
+    }
+    __syncthreads();
+    total = part[32];
+    return part[w] + inc - v;
+}
+
+// One block: block counts -> exclusive offsets in place; the running number of points moves on, its
+// value before goes to rows[1].
+__global__ void __launch_bounds__(APPEND_BLOCK) append_offsets_kernel(unsigned* bsum, int nb, long long* rows) {
+    const int per = (nb + APPEND_BLOCK - 1) / APPEND_BLOCK;
+    const int beg = min(nb, (int)threadIdx.x * per), end = min(nb, beg + per);
+    unsigned s = 0, total;
+    for (int i = beg; i < end; ++i) s += bsum[i];
+    unsigned run = append_scan(s, total);
+    for (int i = beg; i < end; ++i) {
+        const unsigned v = bsum[i];
+        bsum[i] = run;
+        run += v;
+    }
+    if (threadIdx.x == 0) {
+        rows[1] = rows[0];
+        rows[0] += total;
+    }
+}
+
+__global__ void __launch_bounds__(APPEND_BLOCK) append_points_kernel(const __grid_constant__ AppendParams c) {
+    const long long HW = (long long)c.H * c.W;
+    long long idx = 0;
+    const bool kept = append_kept(c, (long long)blockIdx.x * APPEND_BLOCK + threadIdx.x, idx);
+    unsigned total;
+    const unsigned at = append_scan(kept ? 1u : 0u, total);
+    if (!kept) return;
+    const long long o = c.rows[1] + c.bsum[blockIdx.x] + at;
+    for (int k = 0; k < 3; ++k) {
+        c.o_xyz[3 * o + k] = c.xyz[k * HW + idx];
+        c.o_rgb[3 * o + k] = c.rgb[3 * idx + k];
+    }
+    c.o_views[o] = (unsigned char)min(c.count[idx], 255);
+    c.o_owner[o] = c.owner;
 }
 
 static bool is_pinhole(const double* row) { return row[13] == 0.0 && row[14] == 0.0 && row[15] == 0.0; }
@@ -379,6 +470,40 @@ extern "C" mvs_status mvs_fuse_view(const mvs_fuse_args* a, void* stream) {
         p.rel_tol[j] = a->rel_tol[j];
     }
     const long long HW = (long long)a->H * a->W;
-    fuse_kernel<<<(unsigned)((HW + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    MVS_CUDA(cudaMemsetAsync(p.keep, 0, (size_t)HW, st), "fuse: clear keep");
+    MVS_CUDA(cudaMemsetAsync(p.count, 0, (size_t)HW * sizeof(int), st), "fuse: clear count");
+    const long long cand = (long long)((a->H + p.stride - 1) / p.stride) * ((a->W + p.stride - 1) / p.stride);
+    fuse_kernel<<<(unsigned)((cand + 255) / 256), 256, 0, st>>>(p);
     return check_launch("fuse kernel");
+}
+
+extern "C" size_t mvs_fuse_append_scratch_bytes(int32_t H, int32_t W, int32_t point_stride) {
+    if (H < 1 || W < 1) return 0;
+    const int s = point_stride > 1 ? point_stride : 1;
+    const long long cand = (long long)((H + s - 1) / s) * ((W + s - 1) / s);
+    return (size_t)((cand + APPEND_BLOCK - 1) / APPEND_BLOCK) * sizeof(unsigned);
+}
+
+extern "C" mvs_status mvs_fuse_append(const mvs_fuse_append_args* a, void* stream) {
+    clear_error();
+    if (!a) return fail(MVS_ERR_VALUE, "fuse_append: null arguments");
+    if (a->H < 0 || a->W < 0) return fail(MVS_ERR_VALUE, "fuse_append: negative shape");
+    if (a->H == 0 || a->W == 0) return MVS_OK;
+    if (!a->keep || !a->xyz || !a->count || !a->rgb || !a->rows || !a->out_xyz || !a->out_rgb || !a->out_views ||
+        !a->out_owner || !a->scratch)
+        return fail(MVS_ERR_VALUE, "fuse_append: null pointer");
+    AppendParams p;
+    memset(&p, 0, sizeof(p));
+    p.H = a->H; p.W = a->W; p.stride = a->point_stride > 1 ? a->point_stride : 1; p.owner = a->owner;
+    p.keep = a->keep; p.xyz = a->xyz; p.count = a->count; p.rgb = a->rgb;
+    p.bsum = reinterpret_cast<unsigned*>(a->scratch);
+    p.rows = reinterpret_cast<long long*>(a->rows);
+    p.o_xyz = a->out_xyz; p.o_rgb = a->out_rgb; p.o_views = a->out_views; p.o_owner = a->out_owner;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const int nb = (int)(mvs_fuse_append_scratch_bytes(a->H, a->W, p.stride) / sizeof(unsigned));
+    append_count_kernel<<<nb, APPEND_BLOCK, 0, st>>>(p);
+    append_offsets_kernel<<<1, APPEND_BLOCK, 0, st>>>(p.bsum, nb, p.rows);
+    append_points_kernel<<<nb, APPEND_BLOCK, 0, st>>>(p);
+    return check_launch("fuse append");
 }

@@ -184,6 +184,9 @@ def repair(k: int, raw: Dict[int, torch.Tensor], score: torch.Tensor, low: torch
 
 
 # ------------------------------------------------------------------ pass 3: point fusion
+FUSE_GROUP_ROWS = 1 << 24        # candidate pixels per group of views (32 bytes each: 0.5 GB of output space)
+
+
 def fuse(order: Sequence[int], maps: Dict[int, object], cams, nbrs, rel_tols, px_tol: float, min_views: int,
          point_stride: int, rgbs):
     """Point fusion of the final depth maps (densify._fuse, densify.py:676-762) on the device:
@@ -197,39 +200,78 @@ def fuse(order: Sequence[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
     lib = L.load()
     D = {k: _dev32(m, dev) for k, m in maps.items()}
     used = {k: torch.zeros(tuple(D[k].shape), dtype=torch.uint8, device=dev) for k in D}
-    pts, cols, nv, owner = [], [], [], []
+    st = max(int(point_stride), 1)
+    cand = {k: -(-int(d.shape[0]) // st) * -(-int(d.shape[1]) // st) for k, d in D.items()}
     sh = L.stream_handle()
-    for k in order:
-        if k not in D:
-            continue
-        H, W = (int(v) for v in D[k].shape)
-        nb = [j for j in nbrs[k] if j in D and j != k]
-        if len(nb) > L.MAX_SOURCES:
-            raise ValueError(f"fuse: view {k} has {len(nb)} neighbours (at most {L.MAX_SOURCES})")
-        cam = L.host_f64(cam_row(cams[k]))
-        nb_cam = L.host_f64(np.array([cam_row(cams[j]) for j in nb], np.float64).reshape(-1) if nb else np.zeros(1))
-        tol = L.host_f64(np.array([rel_tols[k][j] for j in nb], np.float64) if nb else np.zeros(1))
-        keep = torch.empty((H, W), dtype=torch.uint8, device=dev)
-        xyz = torch.empty((3, H, W), dtype=torch.float64, device=dev)
-        cnt = torch.empty((H, W), dtype=torch.int32, device=dev)
-        a = L.FuseArgs()
-        a.H, a.W, a.depth, a.used, a.cam = H, W, D[k].data_ptr(), used[k].data_ptr(), L.host_ptr(cam)
-        a.n_nb, a.point_stride = len(nb), int(point_stride)
-        for i, j in enumerate(nb):
-            a.nb_depth[i], a.nb_used[i] = D[j].data_ptr(), used[j].data_ptr()
-            a.nb_h[i], a.nb_w[i] = int(D[j].shape[0]), int(D[j].shape[1])
-        a.nb_cam, a.rel_tol, a.px_tol, a.min_views = L.host_ptr(nb_cam), L.host_ptr(tol), float(px_tol), int(min_views)
-        a.keep, a.xyz, a.count = keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr()
-        L.check(lib.mvs_fuse_view(ctypes.addressof(a), sh), "fuse")
-        sel = torch.nonzero(keep.view(-1)).squeeze(1)          # row-major, as np.nonzero
-        if sel.numel() == 0:
-            continue
-        pts.append(xyz.view(3, -1)[:, sel].T)
+
+    def dev_rgb(k):
         rgb = torch.as_tensor(np.ascontiguousarray(rgbs[k]), device=dev) if not isinstance(rgbs[k], torch.Tensor) \
             else rgbs[k].to(dev)
-        cols.append(rgb.reshape(-1, 3)[sel])
-        nv.append(cnt.view(-1)[sel].clamp(max=255).to(torch.uint8))
-        owner.append(torch.full((sel.numel(),), k, dtype=torch.int32, device=dev))
+        return rgb.reshape(-1, 3)
+
+    def uint8_rgb(k):
+        try:
+            c = rgbs[k]
+        except (KeyError, IndexError):
+            return False
+        c = c if isinstance(c, torch.Tensor) else np.asarray(c)
+        return c.dtype in (torch.uint8, np.uint8) and int(np.prod(c.shape)) == 3 * int(D[k].numel())
+
+    # colours of another type, or of some views only, are picked by torch, view by view
+    plain = all(uint8_rgb(k) for k in order if k in D)
+    other: list = []
+    parts: List[tuple] = []
+    todo = [k for k in order if k in D]
+    while todo:
+        # the views of a group append to one set of arrays, and the host waits once for their number
+        # of points (a wait per view left the device idle between views)
+        group, rows = [], 0
+        while todo and (not group or rows + cand[todo[0]] <= FUSE_GROUP_ROWS):
+            group.append(todo.pop(0))
+            rows += cand[group[-1]]
+        px = max(int(D[k].numel()) for k in group)
+        keep = torch.empty(px, dtype=torch.uint8, device=dev)
+        xyz = torch.empty(3 * px, dtype=torch.float64, device=dev)
+        cnt = torch.empty(px, dtype=torch.int32, device=dev)
+        n_rows = torch.zeros(2, dtype=torch.int64, device=dev)
+        out = (torch.empty((rows, 3), dtype=torch.float64, device=dev), torch.empty((rows, 3), dtype=torch.uint8, device=dev),
+               torch.empty(rows, dtype=torch.uint8, device=dev), torch.empty(rows, dtype=torch.int32, device=dev))
+        ws = torch.empty(max(lib.mvs_fuse_append_scratch_bytes(*(int(v) for v in D[k].shape), st) for k in group) or 1,
+                         dtype=torch.uint8, device=dev)
+        for k in group:
+            H, W = (int(v) for v in D[k].shape)
+            nb = [j for j in nbrs[k] if j in D and j != k]
+            if len(nb) > L.MAX_SOURCES:
+                raise ValueError(f"fuse: view {k} has {len(nb)} neighbours (at most {L.MAX_SOURCES})")
+            cam = L.host_f64(cam_row(cams[k]))
+            nb_cam = L.host_f64(np.array([cam_row(cams[j]) for j in nb], np.float64).reshape(-1) if nb else np.zeros(1))
+            tol = L.host_f64(np.array([rel_tols[k][j] for j in nb], np.float64) if nb else np.zeros(1))
+            a = L.FuseArgs()
+            a.H, a.W, a.depth, a.used, a.cam = H, W, D[k].data_ptr(), used[k].data_ptr(), L.host_ptr(cam)
+            a.n_nb, a.point_stride = len(nb), int(point_stride)
+            for i, j in enumerate(nb):
+                a.nb_depth[i], a.nb_used[i] = D[j].data_ptr(), used[j].data_ptr()
+                a.nb_h[i], a.nb_w[i] = int(D[j].shape[0]), int(D[j].shape[1])
+            a.nb_cam, a.rel_tol, a.px_tol, a.min_views = L.host_ptr(nb_cam), L.host_ptr(tol), float(px_tol), int(min_views)
+            a.keep, a.xyz, a.count = keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr()
+            L.check(lib.mvs_fuse_view(ctypes.addressof(a), sh), "fuse")
+            rgb = dev_rgb(k).contiguous() if plain else torch.zeros(3 * H * W, dtype=torch.uint8, device=dev)
+            b = L.FuseAppendArgs()
+            b.H, b.W, b.point_stride, b.owner = H, W, st, int(k)
+            b.keep, b.xyz, b.count, b.rgb, b.rows = (keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr(), rgb.data_ptr(),
+                                                     n_rows.data_ptr())
+            b.out_xyz, b.out_rgb, b.out_views, b.out_owner = (t.data_ptr() for t in out)
+            b.scratch = ws.data_ptr()
+            L.check(lib.mvs_fuse_append(ctypes.addressof(b), sh), "fuse append")
+            if not plain:
+                sel = torch.nonzero(keep[:H * W]).squeeze(1)
+                if sel.numel():
+                    other.append(dev_rgb(k)[sel])
+        n = int(n_rows[0].item())
+        if n:
+            parts.append(tuple(t[:n].clone() if todo or parts else t[:n] for t in out))
+    pts, cols, nv, owner = ([p[q] for p in parts] for q in range(4))
+    cols = cols if plain else other
 
     def cat(a, shape, dt):
         return torch.cat(a) if a else torch.zeros(shape, dtype=dt, device=dev)

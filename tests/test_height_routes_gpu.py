@@ -1,6 +1,6 @@
 """The height sweep's fused kernels against its separate ones and the oracle, bit for bit: the score
 evaluation, the 8-direction aggregation at every register layout, the refinement's stack, choice and
-median."""
+median; and the fused points of a flight by group."""
 from types import SimpleNamespace
 
 import numpy as np
@@ -95,3 +95,27 @@ def test_refinement_steps(hc, wc, HH, WW, level):
     p = np.pad(want, 1, mode="edge")
     med = np.sort(np.stack([p[y:y + HH, x:x + WW] for y in range(3) for x in range(3)]), axis=0)[4]
     assert same_bits(Hs._median3(g_out).cpu().numpy(), med)
+
+
+@pytest.mark.parametrize("stride,rows", [(1, 1 << 24), (2, 700), (3, 1)])
+def test_fusion_in_groups_and_with_other_colours(stride, rows, monkeypatch):
+    """The fused points of a small flight do not depend on how views are grouped; colours of another
+    type come through the picking route with the same points."""
+    from py_ortho_b200 import views as V
+    rng = np.random.default_rng(stride)
+    H, W, n = 37, 52, 4
+    cams = [SimpleNamespace(R=np.diag([1.0, -1.0, -1.0]), C=np.array([2.0 * k, 0.5 * k, 40.0]), f=60.0, k1=0.0, k2=0.0,
+                            k3=0.0, cx=(W - 1) / 2, cy=(H - 1) / 2, w=W, h=H) for k in range(n)]
+    maps = {k: np.where(rng.random((H, W)) < 0.05, np.nan, 40 + rng.normal(0, 0.02, (H, W))).astype(np.float32) for k in range(n)}
+    nbrs = {k: [j for j in range(n) if j != k] for k in range(n)}
+    tols = {k: {j: 0.01 for j in nbrs[k]} for k in nbrs}
+    rgbs = {k: rng.integers(0, 256, (H, W, 3)).astype(np.uint8) for k in range(n)}
+    want = O.fuse(list(range(n)), maps, cams, nbrs, tols, 1.5, 2, stride, rgbs)
+    monkeypatch.setattr(V, "FUSE_GROUP_ROWS", rows)
+    xyz, cols, nv, owner, _ = V.fuse(range(n), maps, cams, nbrs, tols, 1.5, 2, stride, rgbs)
+    assert same_bits(xyz.cpu().numpy(), want[0]) and np.array_equal(cols.cpu().numpy(), want[1])
+    assert np.array_equal(nv.cpu().numpy(), want[2]) and np.array_equal(owner.cpu().numpy(), want[3])
+    grey = {k: v.astype(np.float32) for k, v in rgbs.items()}
+    x2, c2, n2, o2, _ = V.fuse(range(n), maps, cams, nbrs, tols, 1.5, 2, stride, grey)
+    assert torch.equal(x2, xyz) and torch.equal(n2, nv) and torch.equal(o2, owner)
+    assert c2.dtype == torch.float32 and torch.equal(c2.to(torch.uint8), cols)

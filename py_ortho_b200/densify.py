@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from . import fast
+from . import fast, staging
 from .dense import C_addr, Hypotheses, finalize, new_state, sweep
 
 
@@ -91,7 +91,7 @@ def _dev(a, dtype=torch.float32) -> torch.Tensor:
     dev = L.require_cuda()
     if isinstance(a, torch.Tensor):
         return a.to(device=dev, dtype=dtype).contiguous()
-    return torch.from_numpy(np.ascontiguousarray(np.asarray(a), dtype=torch.empty((), dtype=dtype).numpy().dtype)).to(dev)
+    return staging.to_device(np.ascontiguousarray(np.asarray(a), dtype=torch.empty((), dtype=dtype).numpy().dtype), dev)
 
 
 def _box(a, r: int):
@@ -162,7 +162,7 @@ def _sweep(ref, cam_r, srcs, cams_s, inv_list, opt, ray=None):
         depth, best, sd = _sweep_maps(ref, cam_r, srcs, cams_s, inv_list, opt, ray)
     if host:
         torch.cuda.current_stream().synchronize()
-        return depth.cpu().numpy(), best.cpu().numpy(), sd.cpu().numpy()
+        return staging.to_host(depth), staging.to_host(best), staging.to_host(sd)
     return depth, best, sd
 
 
@@ -287,7 +287,7 @@ def depth_map(k, nbrs, rec, views, opt: DepthOptions):
     depth, score, low = out
     torch.cuda.current_stream().synchronize()
     L.check_device_faults()
-    return depth.cpu().numpy(), score.cpu().numpy(), low.cpu().numpy()
+    return staging.to_host(depth), staging.to_host(score), staging.to_host(low)
 
 
 def depth_map_device(k, nbrs, rec, views, opt: DepthOptions):
@@ -302,12 +302,12 @@ def _depth_map_device(k, nbrs, rec, views, opt: DepthOptions):
     if rng is None or not nbrs:
         return None
     ref, _, cam_r = views(k)
-    ref = np.asarray(ref, np.float32)
-    ref_mask = ~np.isfinite(ref)
-    ref = np.ascontiguousarray(np.where(ref_mask, 0.0, ref), np.float32)
+    raw = _dev(np.asarray(ref, np.float32))
+    mask = ~torch.isfinite(raw)
+    ref = torch.where(mask, torch.zeros_like(raw), raw)
     src = [views(j) for j in nbrs]
     lv = 2
-    pyr_r, pyr_c = [_dev(ref)], [cam_r]
+    pyr_r, pyr_c = [ref], [cam_r]
     pyr_s, pyr_cs = [[_dev(s[0]) for s in src]], [[s[2] for s in src]]
     for _ in range(lv):
         r_ = fast.half(pyr_r[-1])
@@ -316,7 +316,7 @@ def _depth_map_device(k, nbrs, rec, views, opt: DepthOptions):
         s_ = [fast.half(x) for x in pyr_s[-1]]
         pyr_s.append(s_)
         pyr_cs.append([c.scaled(0.5, x.shape[1], x.shape[0]) for c, x in zip(pyr_cs[-1], s_)])
-    rays = [fast.rays_world(ref.shape, cam_r)]
+    rays = [fast.rays_world(tuple(ref.shape), cam_r)]
     for lvl in range(1, lv + 1):
         h, w = pyr_r[lvl].shape
         rays.append(fast.half(rays[-1][:, :2 * h, :2 * w].contiguous()))
@@ -339,7 +339,6 @@ def _depth_map_device(k, nbrs, rec, views, opt: DepthOptions):
                                            Hypotheses.refine(iu, dstep, opt.refine_steps), opt, rays[lvl],
                                            precision=_per_pixel_precision(opt))
         dstep = dstep / 2
-    mask = torch.from_numpy(ref_mask).to(d.device)
     depth = torch.where(mask | (d < rng[0]) | (d > rng[1]), torch.full_like(d, float("nan")), d)
     low_texture = (sd * 64.0) < opt.min_texture
     return depth, score, low_texture

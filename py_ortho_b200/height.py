@@ -25,6 +25,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
+from . import fast, staging
 
 
 @dataclass
@@ -163,13 +164,6 @@ def grid_extent(rec, gsd: float, native_gsd: float, max_cells: float = 40e6, tri
     return Grid(x0, y1, int(round((x1 - x0) / gsd)), int(round((y1 - y0) / gsd)), gsd, min(1.0, native_gsd / gsd))
 
 
-def _halve(g: np.ndarray) -> np.ndarray:
-    """One 2x2-mean pyramid step of an (h, w, 1) float32 image (odd edges dropped)."""
-    h, w = g.shape[0] // 2 * 2, g.shape[1] // 2 * 2
-    q = g[:h, :w, 0]
-    return ((q[0::2, 0::2] + q[1::2, 0::2] + q[0::2, 1::2] + q[1::2, 1::2]) * 0.25)[..., None].astype(np.float32)
-
-
 def _feather(h: int, w: int) -> np.ndarray:
     """Colour weight: distance to the nearest image border over half the short side, clipped to 1."""
     s = 0.5 * min(h, w)
@@ -191,24 +185,28 @@ class _View:
         return self.R, self.C, self.f * s, self.k1, self.k2, self.k3, (self.cx + 0.5) * s - 0.5, (self.cy + 0.5) * s - 0.5
 
 
-def _make_view(rec, k, frame, rgb_u8, gains, biases, levels, dev) -> _View:
-    """The view of used camera k: gains / offsets, BT.601 grey, pyramid, feather channel."""
+def _make_view(rec, k, frame, rgb_u8, gains, biases, levels, dev, feathers) -> _View:
+    """The view of used camera k: gains / offsets, BT.601 grey, pyramid, feather channel, formed on
+    the device in NumPy's float32 order. feathers: the call's feather maps by image shape."""
     i = rec.used[k]
-    rgb = rgb_u8.astype(np.float32)
+    host = np.asarray(rgb_u8)
+    host = np.ascontiguousarray(host if host.dtype == np.uint8 else host.astype(np.float32))
+    rgb = staging.to_device(host, dev).to(torch.float32)
     if gains.get(i) is not None:
-        rgb *= np.asarray(gains[i], np.float32)
+        rgb = rgb * torch.as_tensor(np.asarray(gains[i], np.float32), device=dev)
     if biases is not None and biases.get(i) is not None:
-        rgb += np.asarray(biases[i], np.float32)
-    grey = np.ascontiguousarray((0.299 * rgb[..., 0] + 0.587 * rgb[..., 1] + 0.114 * rgb[..., 2])[..., None], np.float32)
-    pyr = [grey]
+        rgb = rgb + torch.as_tensor(np.asarray(biases[i], np.float32), device=dev)
+    pyr = [(0.299 * rgb[..., 0] + 0.587 * rgb[..., 1] + 0.114 * rgb[..., 2]).contiguous()]
     while len(pyr) < levels:
-        pyr.append(np.ascontiguousarray(_halve(pyr[-1])))
-    rgbw = np.ascontiguousarray(np.dstack([rgb, _feather(*rgb.shape[:2])]))
+        pyr.append(fast.half(pyr[-1]))
+    shape = tuple(int(v) for v in rgb.shape[:2])
+    if shape not in feathers:
+        feathers[shape] = torch.as_tensor(_feather(*shape), device=dev)[..., None]
+    rgbw = torch.cat([rgb, feathers[shape]], dim=-1).contiguous()
     it = rec.intr[rec.cam_group[k]]
-    sx = rgb.shape[1] / frame.width
-    return _View([torch.from_numpy(p).to(dev) for p in pyr], torch.from_numpy(rgbw).to(dev),
-                 np.ascontiguousarray(rec.R[k]), np.ascontiguousarray(rec.C[k]), it.f * sx, it.k1, it.k2, it.k3,
-                 (it.cx + 0.5) * sx - 0.5, (it.cy + 0.5) * sx - 0.5)
+    sx = shape[1] / frame.width
+    return _View([q[..., None] for q in pyr], rgbw, np.ascontiguousarray(rec.R[k]), np.ascontiguousarray(rec.C[k]),
+                 it.f * sx, it.k1, it.k2, it.k3, (it.cx + 0.5) * sx - 0.5, (it.cy + 0.5) * sx - 0.5)
 
 
 @dataclass
@@ -436,12 +434,12 @@ def dense_reconstruct(ar, rec, gains: dict, native_gsd: float, opt: DenseOptions
     Wacc = np.zeros((g.H, g.W), np.float32)
     out = DenseResult(None, np.full((g.H, g.W), -1.0, np.float32), np.zeros((g.H, g.W, 3), np.uint8),
                       np.zeros((g.H, g.W), bool), g.minX, g.maxY, g.gsd)
-    views = {}
+    views, feathers = {}, {}
 
     def view(k):
         if k not in views:
             fr = ar.frames[rec.used[k]]
-            views[k] = _make_view(rec, k, fr, load_rgb(fr, g.img_scale), gains, biases, levels, dev)
+            views[k] = _make_view(rec, k, fr, load_rgb(fr, g.img_scale), gains, biases, levels, dev, feathers)
         return views[k]
 
     T = opt.tile

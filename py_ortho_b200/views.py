@@ -28,7 +28,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from . import dense, fast
+from . import dense, fast, staging
 from .densify import DepthOptions, _depth_range, depth_map_device
 
 
@@ -41,7 +41,7 @@ def cam_row(cam) -> np.ndarray:
 def _dev32(a, device) -> torch.Tensor:
     if isinstance(a, torch.Tensor):
         return a.to(device=device, dtype=torch.float32).contiguous()
-    return torch.from_numpy(np.ascontiguousarray(a, np.float32)).to(device)
+    return staging.to_device(np.ascontiguousarray(a, np.float32), device)
 
 
 def consistency(D, cam_r, nb_maps: Sequence, nb_cams: Sequence, px_tol: float, rel_tol: Sequence[float],
@@ -397,6 +397,6 @@ def densify_views(rec, views, opt: DepthOptions, nbrs: Optional[List[List[int]]]
             D, ch, na = repair(k, maps, score, low, views, nbrs[k], rec, settings, opt)
         torch.cuda.current_stream().synchronize()
         L.check_device_faults()      # a sweep tile of pass 1 or 2 that gave up raises here
-        return D.cpu().numpy(), ch, na
+        return staging.to_host(D), ch, na
 
     return run_passes(N, nbrs, costs, shapes, pass1, pass2, group=group, device=dev)

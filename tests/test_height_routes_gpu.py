@@ -1,6 +1,6 @@
 """The height sweep's fused kernels against its separate ones and the oracle, bit for bit: the score
 evaluation, the 8-direction aggregation at every register layout, the refinement's stack, choice and
-median; and the fused points of a flight by group."""
+median; and the staged host copies."""
 from types import SimpleNamespace
 
 import numpy as np
@@ -95,6 +95,19 @@ def test_refinement_steps(hc, wc, HH, WW, level):
     p = np.pad(want, 1, mode="edge")
     med = np.sort(np.stack([p[y:y + HH, x:x + WW] for y in range(3) for x in range(3)]), axis=0)[4]
     assert same_bits(Hs._median3(g_out).cpu().numpy(), med)
+
+
+@pytest.mark.parametrize("n,dtype", [(1, np.float32), (1 << 20, np.float32), ((1 << 21) + 3, np.float32),
+                                     (5_000_001, np.float32), (9_000_001, np.bool_)])
+def test_staged_copies(n, dtype):
+    """Around one piece, two and an uneven number of pieces; on another stream."""
+    from py_ortho_b200 import staging
+    rng = np.random.default_rng(n)
+    a = rng.integers(0, 2, n).astype(dtype) if dtype is np.bool_ else rng.normal(0, 1, n).astype(dtype)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        t = staging.to_device(a, torch.device("cuda", 0))
+        back = staging.to_host(t)
+    assert np.array_equal(back, a) and back.dtype == a.dtype
 
 
 @pytest.mark.parametrize("stride,rows", [(1, 1 << 24), (2, 700), (3, 1)])

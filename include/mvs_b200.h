@@ -487,25 +487,6 @@ typedef struct mvs_height_score_args {
  * order), times the reference's texture weight. */
 mvs_status mvs_height_score(const mvs_height_score_args* args, void* stream);
 
-/* Semi-global aggregation of a (D, H, W) float32 cost volume along 8 directions, summed in the
- * reference's direction order. Replaces _mvs.sgm (_mvs.pyx:98-251); bit-exact. */
-mvs_status mvs_sgm(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
-                   void* stream);
-
-/* ---------------------------------------------------------------- misc */
-
-/* Device-side waits that gave up since the last call (the sweep's TMA copy of the reference
- * tile waits on an mbarrier with an iteration limit; a tile whose copy never completes leaves its
- * state untouched and is counted here). Synchronises with the device; clears the count.
- * Returns MVS_ERR_TIMEOUT when the count was non-zero. No counterpart in the reference. */
-mvs_status mvs_device_faults(uint32_t* count);
-
-/* Iterations of the sweep's bounded wait for its reference-tile copy (default 2^20 try_wait
- * iterations, far above a copy's latency); returns the previous value. For tests of the give-up
- * path: with 0 every tile gives up at once - it counts a fault, waits (with the default bound)
- * for its copy in flight to land and returns with its state untouched. Applies to calls made
- * after it, from any thread. No counterpart in the reference. */
-uint32_t mvs_set_wait_limit(uint32_t iterations);
 /* One photo-consistency evaluation of a height stack: every view's samples (mvs_sample_view on
  * one-channel images), all window means (mvs_box_sat_mean of the samples, their squares, the valid
  * masks and the pair products) and mvs_height_score, in three launches and with their values. The grid
@@ -540,14 +521,33 @@ mvs_status mvs_height_pick(int32_t H, int32_t W, int32_t K, const float* score, 
                            float weak, int32_t parabola, float cell, float* out, void* stream);
 mvs_status mvs_median3(int32_t H, int32_t W, const float* a, float* out, void* stream);
 
-
-/* Bounds-checked debug build only (libmvs_b200_debug.so, compiled with MVS_DEBUG_BOUNDS): the
- * number of shared-memory and global indices the tile engine, the batched kernels and PatchMatch
- * used outside their buffers since the last call (synchronises; clears the counts). Release
+/* Semi-global aggregation of a (D, H, W) float32 cost volume along 8 directions, summed in the
+ * reference's direction order. Replaces _mvs.sgm (_mvs.pyx:98-251); bit-exact. */
+mvs_status mvs_sgm(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
+                   void* stream);
 /* mvs_sgm with its scratch given by the caller (8 volumes up to 256 hypotheses, else one). */
 size_t mvs_sgm_scratch_bytes(int32_t D, int32_t H, int32_t W);
 mvs_status mvs_sgm_ws(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
                       void* scratch, size_t scratch_bytes, void* stream);
+
+/* ---------------------------------------------------------------- misc */
+
+/* Device-side waits that gave up since the last call (the sweep's TMA copy of the reference
+ * tile waits on an mbarrier with an iteration limit; a tile whose copy never completes leaves its
+ * state untouched and is counted here). Synchronises with the device; clears the count.
+ * Returns MVS_ERR_TIMEOUT when the count was non-zero. No counterpart in the reference. */
+mvs_status mvs_device_faults(uint32_t* count);
+
+/* Iterations of the sweep's bounded wait for its reference-tile copy (default 2^20 try_wait
+ * iterations, far above a copy's latency); returns the previous value. For tests of the give-up
+ * path: with 0 every tile gives up at once - it counts a fault, waits (with the default bound)
+ * for its copy in flight to land and returns with its state untouched. Applies to calls made
+ * after it, from any thread. No counterpart in the reference. */
+uint32_t mvs_set_wait_limit(uint32_t iterations);
+
+/* Bounds-checked debug build only (libmvs_b200_debug.so, compiled with MVS_DEBUG_BOUNDS): the
+ * number of shared-memory and global indices the tile engine, the batched kernels and PatchMatch
+ * used outside their buffers since the last call (synchronises; clears the counts). Release
  * builds return MVS_ERR_UNSUPPORTED. No counterpart in the reference (its Cython kernels are
  * compiled with boundscheck=False). */
 mvs_status mvs_debug_bound_violations(uint32_t* count);

@@ -98,12 +98,6 @@ class DepthBandArgs(C.Structure):
                 ("inv_hi", vp)]
 
 
-class BatchJob(C.Structure):
-    _fields_ = [("sweep", SweepArgs), ("depth", vp)]
-
-
-class BatchTuning(C.Structure):
-    _fields_ = [("plane_chunk", i32), ("ctas_per_sm", i32), ("tile_h", i32)]
 class HeightEvalArgs(C.Structure):
     _fields_ = [("V", i32), ("D", i32), ("H", i32), ("W", i32), ("r", i32), ("topk", i32), ("X0", C.c_double),
                 ("Y0", C.c_double), ("gsd", C.c_double), ("img", vp * MAX_SOURCES), ("img_h", i32 * MAX_SOURCES),
@@ -112,12 +106,21 @@ class HeightEvalArgs(C.Structure):
                 ("ref", vp)]
 
 
+class BatchJob(C.Structure):
+    _fields_ = [("sweep", SweepArgs), ("depth", vp)]
+
+
+class BatchTuning(C.Structure):
+    _fields_ = [("plane_chunk", i32), ("ctas_per_sm", i32), ("tile_h", i32)]
 
 
 # name -> (restype, argtypes); every symbol the header declares
 SIGNATURES = {
     "mvs_sweep": (i32, [vp, vp]),
     "mvs_sweep_noalloc": (i32, [vp, vp]),
+    "mvs_sweep_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_sweep_state_init": (i32, [i32, i32, vp, vp, vp, vp, vp, vp]),
+    "mvs_sweep_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_sweep_hypothesis": (i32, [i32, i32, vp, vp, vp, i32, vp, vp, vp, vp, vp, vp, i32, i32, i32,
                                    vp, vp, vp, vp, vp, vp]),
     "mvs_sweep_finalize": (i32, [i32, i32, vp, vp, vp, vp, vp, vp, vp]),
@@ -131,10 +134,11 @@ SIGNATURES = {
     "mvs_to_fp16": (i32, [i64, vp, vp, vp]),
     "mvs_tie_depths": (i32, [i32, vp, vp, i32, i32, vp, vp]),
     "mvs_depth_band": (i32, [vp, vp]),
+    "mvs_depth_band_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_depth_band_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_pm_refine": (i32, [vp, vp]),
-    "mvs_sweep_scratch_bytes": (C.c_size_t, [vp]),
-    "mvs_sweep_state_init": (i32, [i32, i32, vp, vp, vp, vp, vp, vp]),
-    "mvs_sweep_ws": (i32, [vp, vp, C.c_size_t, vp]),
+    "mvs_pm_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_pm_refine_ws": (i32, [vp, vp, C.c_size_t, vp]),
     "mvs_pm_stream_advance": (C.c_uint32, [C.c_uint32, C.c_uint64]),
     "mvs_batch_create": (i32, [vp, i32, vp, vp]),
     "mvs_batch_run": (i32, [vp, i32, vp]),
@@ -147,16 +151,19 @@ SIGNATURES = {
     "mvs_consistency": (i32, [vp, vp]),
     "mvs_init_normals": (i32, [i32, i32, vp, vp, vp, vp]),
     "mvs_fuse_view": (i32, [vp, vp]),
-    "mvs_sample_view": (i32, [vp, vp]),
-    "mvs_depth_band_scratch_bytes": (C.c_size_t, [vp]),
-    "mvs_depth_band_ws": (i32, [vp, vp, C.c_size_t, vp]),
-    "mvs_box_sat_mean": (i32, [i32, i32, i32, vp, i32, vp, vp]),
     "mvs_fuse_append": (i32, [vp, vp]),
     "mvs_fuse_append_scratch_bytes": (C.c_size_t, [i32, i32, i32]),
-    "mvs_pm_scratch_bytes": (C.c_size_t, [vp]),
-    "mvs_pm_refine_ws": (i32, [vp, vp, C.c_size_t, vp]),
+    "mvs_sample_view": (i32, [vp, vp]),
+    "mvs_box_sat_mean": (i32, [i32, i32, i32, vp, i32, vp, vp]),
     "mvs_height_score": (i32, [vp, vp]),
+    "mvs_height_eval_scratch_bytes": (C.c_size_t, [vp]),
+    "mvs_height_eval": (i32, [vp, vp, C.c_size_t, vp]),
+    "mvs_height_stack": (i32, [i32, i32, i32, i32, vp, i32, vp, vp, vp, vp]),
+    "mvs_height_pick": (i32, [i32, i32, i32, vp, vp, vp, C.c_float, i32, C.c_float, vp, vp]),
+    "mvs_median3": (i32, [i32, i32, vp, vp, vp]),
     "mvs_sgm": (i32, [i32, i32, i32, vp, C.c_float, C.c_float, vp, vp]),
+    "mvs_sgm_scratch_bytes": (C.c_size_t, [i32, i32, i32]),
+    "mvs_sgm_ws": (i32, [i32, i32, i32, vp, C.c_float, C.c_float, vp, vp, C.c_size_t, vp]),
     "mvs_last_error": (C.c_size_t, [C.c_char_p, C.c_size_t]),
     "mvs_device_faults": (i32, [vp]),
     "mvs_set_wait_limit": (C.c_uint32, [C.c_uint32]),
@@ -164,14 +171,7 @@ SIGNATURES = {
     "mvs_version": (C.c_char_p, []),
 }
 
-    "mvs_height_eval_scratch_bytes": (C.c_size_t, [vp]),
-    "mvs_height_eval": (i32, [vp, vp, C.c_size_t, vp]),
-    "mvs_height_stack": (i32, [i32, i32, i32, i32, vp, i32, vp, vp, vp, vp]),
-    "mvs_height_pick": (i32, [i32, i32, i32, vp, vp, vp, C.c_float, i32, C.c_float, vp, vp]),
-    "mvs_median3": (i32, [i32, i32, vp, vp, vp]),
 _lib = None
-    "mvs_sgm_scratch_bytes": (C.c_size_t, [i32, i32, i32]),
-    "mvs_sgm_ws": (i32, [i32, i32, i32, vp, C.c_float, C.c_float, vp, vp, C.c_size_t, vp]),
 _lock = threading.Lock()
 
 
@@ -246,22 +246,6 @@ def stream_handle(stream=None) -> int:
     return int(s.cuda_stream)
 
 
-def require_cuda() -> torch.device:
-    if not torch.cuda.is_available():
-        raise RuntimeError("py_ortho_b200 runs on a CUDA device (sm_100a); no CUDA device is visible")
-    return torch.device("cuda", torch.cuda.current_device())
-
-
-def ptr(t) -> int:
-    return 0 if t is None else int(t.data_ptr())
-
-
-def host_f64(a) -> np.ndarray:
-    return np.ascontiguousarray(np.asarray(a, np.float64))
-
-
-def host_ptr(a: np.ndarray) -> int:
-    return int(a.ctypes.data)
 def call_with_scratch(name: str, args: int, device, stream=None) -> int:
     """Status of the entry point `name` on `args` (a struct's address), its scratch taken from torch's
     caching allocator on the stream that the call uses: the driver's stream-ordered pool gives its
@@ -281,3 +265,19 @@ def call_with_scratch(name: str, args: int, device, stream=None) -> int:
     return getattr(lib, name)(args, sh)
 
 
+def require_cuda() -> torch.device:
+    if not torch.cuda.is_available():
+        raise RuntimeError("py_ortho_b200 runs on a CUDA device (sm_100a); no CUDA device is visible")
+    return torch.device("cuda", torch.cuda.current_device())
+
+
+def ptr(t) -> int:
+    return 0 if t is None else int(t.data_ptr())
+
+
+def host_f64(a) -> np.ndarray:
+    return np.ascontiguousarray(np.asarray(a, np.float64))
+
+
+def host_ptr(a: np.ndarray) -> int:
+    return int(a.ctypes.data)

@@ -280,9 +280,11 @@ struct EvalPlane {
 // row totals, and a ring of 32 + k table rows in shared memory feeds the four corners, so the table
 // (16 bytes a cell, written and read twice) never leaves the SM. Every sum runs in the order of the
 // separate passes. Needs the ring in shared memory (height_box_smem); wider grids take the passes.
-// Over a 9-view flight's 80 evaluations 7.4 ms, as the three passes took, but without the stacked, squared,
-// gathered and multiplied copies that fed them (~4 ms) and their launches.
-constexpr int HB_ROWS = 32;
+// Bound by the serial float64 sums and, before, by integer divisions around them: over a 9-view flight's
+// 80 evaluations 4.9 ms (7.4 ms with a slot by modulo, a cell by division and the mean by a float64
+// division), where the three passes took 7.4 ms and ~4 ms for the stacked, squared, gathered and
+// multiplied copies that fed them.
+constexpr int HB_ROWS = 32, HB_AHEAD = 8;      // rows per step; rows whose loads are in flight together
 static size_t height_box_smem(int W, int r) { return (size_t)(HB_ROWS + 2 * r + 1) * (W + 1) * sizeof(double); }
 
 __global__ void __launch_bounds__(256) height_box_kernel(const __grid_constant__ EvalParams p, int r,
@@ -311,35 +313,49 @@ __global__ void __launch_bounds__(256) height_box_kernel(const __grid_constant__
         pl.b = p.S + (a + 1 + e) * DHW + d * HW;
     }
     float* o = out + ((long long)q * p.D + d) * HW;
-    const double kk = (double)k * (double)k;
-    // table row i (1 .. H + 2r + 1 padded; row 0 .. r are zeros) lives in ring slot i % RING; column sums
-    // of each thread's columns stay in registers from row to row
+    const double kk = (double)k * (double)k, rk = 1.0 / kk;
+    // table row i (0 .. H + 2 r, padded; the first r + 1 are zeros) lives in ring slot i mod RING; column
+    // sums of each thread's columns stay in registers from row to row
     constexpr int MAXC = 4;                       // columns per thread (W <= 4 * 256)
     double col[MAXC];
 #pragma unroll
     for (int m = 0; m < MAXC; ++m) col[m] = 0.0;
     const int PH = H + k;
+    int base = 0;                                 // slot of row i0
+    auto slot = [&](int ahead) {                  // of row i0 + ahead, -RING <= ahead < RING
+        const int q = base + ahead;
+        return q >= RING ? q - RING : (q < 0 ? q + RING : q);
+    };
     for (int i0 = 0; i0 < PH; i0 += HB_ROWS) {
-        const int i1 = min(i0 + HB_ROWS, PH);
-        // column sums of rows i0 .. i1 - 1 (padded row i is image row i - r - 1)
+        const int rows = min(HB_ROWS, PH - i0);
+        // column sums of rows i0 .. i0 + rows - 1 (padded row i is image row i - r - 1)
 #pragma unroll
         for (int m = 0; m < MAXC; ++m) {
             const int x = threadIdx.x + m * 256;
             if (x < W) {
                 double c = col[m];
-                for (int i = i0; i < i1; ++i) {
-                    const int ay = i - r - 1;
-                    const double val = (ay >= 0 && ay < H) ? pl.at((long long)ay * W + x) : 0.0;
-                    c = c + val;
-                    hb_ring[(i % RING) * pitch + x] = c;
+                for (int a = 0; a < rows; a += HB_AHEAD) {
+                    // (rows past the image are read at its edge and count as 0)
+                    double v[HB_AHEAD];
+#pragma unroll
+                    for (int u = 0; u < HB_AHEAD; ++u)
+                        v[u] = pl.at((long long)min(max(i0 + a + u - r - 1, 0), H - 1) * W + x);
+#pragma unroll
+                    for (int u = 0; u < HB_AHEAD; ++u) {
+                        const int ay = i0 + a + u - r - 1;
+                        if (a + u < rows) {
+                            c = c + ((ay >= 0 && ay < H) ? v[u] : 0.0);
+                            hb_ring[slot(a + u) * pitch + x] = c;
+                        }
+                    }
                 }
                 col[m] = c;
             }
         }
         __syncthreads();
         // running totals along the rows, in place: lane = row
-        if (threadIdx.x < 32 && i0 + (int)threadIdx.x < i1) {
-            double* row = hb_ring + ((i0 + threadIdx.x) % RING) * pitch;
+        if ((int)threadIdx.x < rows) {
+            double* row = hb_ring + slot(threadIdx.x) * pitch;
             double total = 0.0;
             int x = 0;
             for (; x + 8 <= W; x += 8) {
@@ -358,25 +374,25 @@ __global__ void __launch_bounds__(256) height_box_kernel(const __grid_constant__
             }
         }
         __syncthreads();
-        // the means whose lower table row is one of these: y = i - k
-        const int y0 = max(i0 - k, 0), y1 = min(i1 - k, H);
-        for (int e = threadIdx.x; e < max(y1 - y0, 0) * W; e += 256) {
-            const int y = y0 + e / W, x = e % W;
-            const double* cur = hb_ring + ((y + k) % RING) * pitch;
-            const double* old = hb_ring + (y % RING) * pitch;
-            // padded column j holds the total up to image column j - r - 1 (0 before it, the last after)
-            const int jl = x - r - 1, jr = min(x + r, W - 1);
-            double val = cur[jr] - old[jr];
-            if (jl >= 0) {
-                val = val - cur[jl];
-                val = val + old[jl];
-            } else {
-                val = val - 0.0;
-                val = val + 0.0;
+        // the means whose lower table row is one of these, y = i - k: 4 rows of 64 threads at a time
+        for (int a = threadIdx.x >> 6; a < rows; a += 4) {
+            const int y = i0 + a - k;
+            if (y < 0) continue;
+            const double* cur = hb_ring + slot(a) * pitch;
+            const double* old = hb_ring + slot(a - k) * pitch;
+            for (int x = threadIdx.x & 63; x < W; x += 64) {
+                // padded column j holds the total up to image column j - r - 1 (0 before it, the last after)
+                const int jl = x - r - 1, jr = min(x + r, W - 1);
+                double val = cur[jr] - old[jr];
+                val = val - (jl >= 0 ? cur[jl] : 0.0);
+                val = val + (jl >= 0 ? old[jl] : 0.0);
+                // val / kk: the quotient's remainder is exact in one fused operation (Markstein)
+                const double t = val * rk;
+                o[(long long)y * W + x] = (float)(isfinite(t) ? __fma_rn(__fma_rn(-t, kk, val), rk, t) : t);
             }
-            o[(long long)y * W + x] = (float)(val / kk);
         }
         __syncthreads();
+        base = slot(HB_ROWS);                     // (HB_ROWS < RING)
     }
 }
 

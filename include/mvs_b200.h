@@ -525,7 +525,8 @@ mvs_status mvs_median3(int32_t H, int32_t W, const float* a, float* out, void* s
  * reference's direction order. Replaces _mvs.sgm (_mvs.pyx:98-251); bit-exact. */
 mvs_status mvs_sgm(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
                    void* stream);
-/* mvs_sgm with its scratch given by the caller (8 volumes up to 256 hypotheses, else one). */
+/* mvs_sgm with its scratch given by the caller: mvs_sgm_scratch_bytes (8 volumes up to 256 hypotheses,
+ * else one), or one volume (D * H * W floats) at the least: then one direction at a time. */
 size_t mvs_sgm_scratch_bytes(int32_t D, int32_t H, int32_t W);
 mvs_status mvs_sgm_ws(int32_t D, int32_t H, int32_t W, const float* cost, float P1, float P2, float* agg,
                       void* scratch, size_t scratch_bytes, void* stream);

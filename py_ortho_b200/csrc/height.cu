@@ -717,7 +717,7 @@ extern "C" mvs_status mvs_height_score(const mvs_height_score_args* a, void* str
 }
 
 // Volumes of scratch that mvs_sgm keeps: one per direction, or one for the direction at a time when D
-// is above 32 lanes' registers.
+// is above 32 lanes' registers (or there is no room for eight).
 static int sgm_volumes(int D) { return D <= 256 ? 8 : 1; }
 
 extern "C" size_t mvs_sgm_scratch_bytes(int32_t D, int32_t H, int32_t W) {
@@ -731,10 +731,10 @@ extern "C" mvs_status mvs_sgm_ws(int32_t D, int32_t H, int32_t W, const float* c
     const long long n = (long long)D * H * W;
     if (n == 0) return MVS_OK;
     if (!cost || !agg) return fail(MVS_ERR_VALUE, "sgm: null pointer");
-    if (!scratch || scratch_bytes < mvs_sgm_scratch_bytes(D, H, W)) return fail(MVS_ERR_VALUE, "sgm: scratch too small");
+    if (!scratch || scratch_bytes < sizeof(float) * (size_t)n) return fail(MVS_ERR_VALUE, "sgm: scratch too small");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     float* L = reinterpret_cast<float*>(scratch);
-    if (sgm_volumes(D) == 8) {
+    if (sgm_volumes(D) == 8 && scratch_bytes >= mvs_sgm_scratch_bytes(D, H, W)) {
         SgmDirs dirs;
         const int lines[8] = {H, H, W, W, H + W - 1, H + W - 1, H + W - 1, H + W - 1};
         dirs.line0[0] = 0;
@@ -764,9 +764,17 @@ extern "C" mvs_status mvs_sgm(int32_t D, int32_t H, int32_t W, const float* cost
                               void* stream) {
     clear_error();
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const size_t need = mvs_sgm_scratch_bytes(D, H, W);
+    size_t need = mvs_sgm_scratch_bytes(D, H, W);
     void* ws = nullptr;
-    if (need && cost && agg) MVS_CUDA(cudaMallocAsync(&ws, need, st), "sgm: scratch");
+    if (need && cost && agg) {
+        cudaError_t e = cudaMallocAsync(&ws, need, st);
+        if (e == cudaErrorMemoryAllocation && sgm_volumes(D) > 1) {   // no room: one direction at a time
+            cudaGetLastError();
+            need /= sgm_volumes(D);
+            e = cudaMallocAsync(&ws, need, st);
+        }
+        MVS_CUDA(e, "sgm: scratch");
+    }
     const mvs_status s = mvs_sgm_ws(D, H, W, cost, P1, P2, agg, ws, need, stream);
     if (ws) cudaFreeAsync(ws, st);
     return s;

@@ -110,7 +110,11 @@ def sgm(cost: torch.Tensor, P1: float, P2: float) -> torch.Tensor:
     agg = torch.empty_like(cost)
     lib = L.load()
     need = lib.mvs_sgm_scratch_bytes(D, H, W)
-    ws = torch.empty(need, dtype=torch.uint8, device=cost.device)
+    try:
+        ws = torch.empty(need, dtype=torch.uint8, device=cost.device)
+    except torch.cuda.OutOfMemoryError:                       # one direction at a time
+        need = 4 * D * H * W
+        ws = torch.empty(need, dtype=torch.uint8, device=cost.device)
     L.check(lib.mvs_sgm_ws(D, H, W, cost.data_ptr(), float(P1), float(P2), agg.data_ptr(), ws.data_ptr(), need,
                            L.stream_handle()), "sgm")
     return agg

@@ -61,6 +61,18 @@ def test_sgm_at_every_layout(D, H, W):
     assert same_bits(got, O.sgm(cost, np.float32(0.05), np.float32(0.6)))
 
 
+@pytest.mark.parametrize("D,H,W", [(1, 5, 9), (33, 21, 34), (256, 7, 12)])
+def test_sgm_one_direction_at_a_time(D, H, W):
+    """With room for one volume of scratch only."""
+    from py_ortho_b200 import _lib as L
+    cost = np.random.default_rng(D + 1).uniform(0, 2, (D, H, W)).astype(np.float32)
+    c = torch.from_numpy(cost).cuda()
+    agg, ws = torch.empty_like(c), torch.empty_like(c)
+    L.check(L.load().mvs_sgm_ws(D, H, W, c.data_ptr(), 0.05, 0.6, agg.data_ptr(), ws.data_ptr(), 4 * c.numel(),
+                                L.stream_handle()))
+    assert same_bits(agg.cpu().numpy(), O.sgm(cost, np.float32(0.05), np.float32(0.6)))
+
+
 @pytest.mark.parametrize("hc,wc,HH,WW,level", [(1, 1, 2, 1, 0), (5, 7, 10, 14, 0), (5, 7, 9, 13, 1), (6, 4, 13, 9, 0),
                                                (23, 40, 46, 79, 1)])
 def test_refinement_steps(hc, wc, HH, WW, level):

@@ -913,8 +913,9 @@ __global__ void __launch_bounds__(256) pm_quad_kernel(const float* __restrict__ 
 
 // Resident blocks of 256 threads per SM for the lane kernel (propagation; trials). Propagation of 4
 // iterations at 4000 x 3000, 8 sources, 7 x 7: 252 ms with single samples at 5 blocks (48 registers), in
-// pairs 239 ms at 5, 232 ms at 4 (64 registers), 248 ms at 3. What bounds it is latency at that
-// occupancy: issue slots alone would take ~100 ms, the footprints' L1 wavefronts ~50 ms.
+// pairs of a row 239 ms at 5, 232 ms at 4 (64 registers), 248 ms at 3, in pairs of the whole window and
+// with a shorter unit set-up 217 ms at 4. What bounds it is latency at that occupancy: issue slots alone
+// would take ~100 ms, the footprints' L1 wavefronts ~50 ms.
 #ifndef PM_LANE_MIN_BLOCKS
 #define PM_LANE_MIN_BLOCKS 4
 #endif
@@ -948,11 +949,24 @@ __device__ __forceinline__ float pm_rcp_ftz(float x) {
     return r;
 }
 
+// The smaller (larger) of a and b, NaN when either is.
+__device__ __forceinline__ float pm_min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float pm_max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // A pixel's window as the cost code reads it: sample (row, k) = e-th of the window as
 // (ray_q - ray_p, I_q - mI) with I = NaN where there is no sample (outside the image or a
 // non-finite reference value), and the ray offsets of the clipped window's four corners. PAIRS:
-// samples (row, 2 m) and (row, 2 m + 1) come as packed pairs of each component, for the packed
-// arithmetic of pm_window_sums (an odd side's last pair has a surplus second sample).
+// neighbouring samples come as packed pairs of each component, for the packed arithmetic of
+// pm_window_sums: samples e and e + 1 of the whole window (FLAT: only the last pair of an odd window
+// has a surplus second sample), or of a row (then every row of an odd side has one).
 //   PMWinStaged: staged once per visit in shared memory by the pixel's lane group;
 //   PMWinPairs:  the same for a side known at compile time, pair by pair (32 bytes: x x y y z z I I);
 //   PMWinTile:   read from the warp's shared tile of raw rays and reference values (one lane per
@@ -961,7 +975,7 @@ __device__ __forceinline__ float pm_rcp_ftz(float x) {
 //                operations, so the same values (positions outside the image hold masked samples
 //                either way). PAIRS at step 1, where a lane's columns start on an even one.
 struct PMWinStaged {
-    static constexpr bool PAIRS = false;
+    static constexpr bool PAIRS = false, FLAT = false;
     const float4* w;      // NW samples, then the 4 corners
     __device__ __forceinline__ float4 at(int, int, int e) const { return w[e]; }
     __device__ __forceinline__ float4 corner(int k4, int nw) const { return w[nw + k4]; }
@@ -969,20 +983,20 @@ struct PMWinStaged {
 };
 template <int NSIDE>
 struct PMWinPairs {
-    static constexpr bool PAIRS = true;
-    static constexpr int NP = (NSIDE + 1) / 2;                 // pairs per row
+    static constexpr bool PAIRS = true, FLAT = true;
+    static constexpr int NW = NSIDE * NSIDE, NP = (NW + 1) / 2;   // samples, pairs
     // float4 entries per pixel: the pairs, the 4 corners, one more (an odd number of 16-byte units
     // puts the 4 pixels of a warp on different banks)
-    static constexpr int ENTRIES = 2 * NSIDE * NP + 4 + 1;
+    static constexpr int ENTRIES = 2 * NP + 4 + 1;
     const float4* w;
-    static __device__ __forceinline__ int slot(int row, int k) { return (row * NP + (k >> 1)) * 8 + (k & 1); }
-    __device__ __forceinline__ float4 at(int row, int k, int) const {
-        const float* f = reinterpret_cast<const float*>(w) + slot(row, k);
+    static __device__ __forceinline__ int slot(int e) { return (e >> 1) * 8 + (e & 1); }
+    __device__ __forceinline__ float4 at(int, int, int e) const {
+        const float* f = reinterpret_cast<const float*>(w) + slot(e);
         return make_float4(f[0], f[2], f[4], f[6]);
     }
-    __device__ __forceinline__ float4 corner(int k4, int) const { return w[2 * NSIDE * NP + k4]; }
-    __device__ __forceinline__ void pair(int row, int m, float2& x, float2& y, float2& z, float2& i) const {
-        const float4 a = w[2 * (row * NP + m)], b = w[2 * (row * NP + m) + 1];
+    __device__ __forceinline__ float4 corner(int k4, int) const { return w[2 * NP + k4]; }
+    __device__ __forceinline__ void pair(int, int m, float2& x, float2& y, float2& z, float2& i) const {
+        const float4 a = w[2 * m], b = w[2 * m + 1];
         x = make_float2(a.x, a.y);
         y = make_float2(a.z, a.w);
         z = make_float2(b.x, b.y);
@@ -991,7 +1005,7 @@ struct PMWinPairs {
 };
 template <bool STEP1>
 struct PMWinTile {
-    static constexpr bool PAIRS = STEP1;
+    static constexpr bool PAIRS = STEP1, FLAT = false;
     const float* t;       // x plane at the window's first sample (row y - r, column x - r)
     int plane;            // entries of one plane (x, y, z, I)
     int rs, cs;           // tile offsets of one window row and one window column
@@ -1024,6 +1038,11 @@ struct PMWinT {
     bool allfin;          // every sample has a finite reference value inside the image
 };
 
+// Pairs of a flat window in flight (24 full pairs at 7 x 7, 12 at 5 x 5); propagation of 4 iterations at
+// 4000 x 3000, 8 sources: 2 / 3 / 4 pairs 223.0 / 216.7 / 223.6 ms; row by row (28 pairs, 4 in
+// flight) 232 ms.
+constexpr int PM_FLAT_AHEAD = 3;
+
 // One source's window sums. CHECKED: every sample tested as in the reference (camera depth,
 // source bounds, finite value) and the reference sums formed per source; otherwise (the whole
 // window maps inside the source, no sample near a test) only the three source sums are formed.
@@ -1044,41 +1063,49 @@ __device__ __forceinline__ void pm_window_sums(const Acc& win, int side_rt, cons
         const float2 B0 = pm_dup(B[0]), B1 = pm_dup(B[1]), B2 = pm_dup(B[2]), b0p = pm_dup(b0);
         const float2 C0 = pm_dup(C[0]), C1 = pm_dup(C[1]), C2 = pm_dup(C[2]), c0p = pm_dup(c0);
         const float2 bias = pm_dup(12582912.0f), nbias = pm_dup(-12582912.0f);
-#pragma unroll 1
-        for (int row = 0; row < NSIDE; ++row)
+        auto two = [&](int row, int m, bool both) {
+            float2 x, y, z, iv;
+            win.pair(row, m, x, y, z, iv);
+            const float2 cq = __ffma2_rn(C0, x, __ffma2_rn(C1, y, __ffma2_rn(C2, z, c0p)));
+            const float2 aq = __ffma2_rn(A0, x, __ffma2_rn(A1, y, __ffma2_rn(A2, z, a0p)));
+            const float2 bq = __ffma2_rn(B0, x, __ffma2_rn(B1, y, __ffma2_rn(B2, z, b0p)));
+            const float2 rc = make_float2(pm_rcp_ftz(cq.x), pm_rcp_ftz(cq.y));
+            const float2 ul = __fmul2_rn(aq, rc), vl = __fmul2_rn(bq, rc);
+            const float2 tu = __fadd2_rd(ul, bias), tv = __fadd2_rd(vl, bias);
+            const float2 fx = pm_sub2(ul, __fadd2_rn(tu, nbias)), fy = pm_sub2(vl, __fadd2_rn(tv, nbias));
 #pragma unroll
-            for (int m = 0; m < (NSIDE + 1) / 2; ++m) {
-                float2 x, y, z, iv;
-                win.pair(row, m, x, y, z, iv);
-                const float2 cq = __ffma2_rn(C0, x, __ffma2_rn(C1, y, __ffma2_rn(C2, z, c0p)));
-                const float2 aq = __ffma2_rn(A0, x, __ffma2_rn(A1, y, __ffma2_rn(A2, z, a0p)));
-                const float2 bq = __ffma2_rn(B0, x, __ffma2_rn(B1, y, __ffma2_rn(B2, z, b0p)));
-                const float2 rc = make_float2(pm_rcp_ftz(cq.x), pm_rcp_ftz(cq.y));
-                const float2 ul = __fmul2_rn(aq, rc), vl = __fmul2_rn(bq, rc);
-                const float2 tu = __fadd2_rd(ul, bias), tv = __fadd2_rd(vl, bias);
-                const float2 fx = pm_sub2(ul, __fadd2_rn(tu, nbias)), fy = pm_sub2(vl, __fadd2_rn(tv, nbias));
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    if (2 * m + q >= NSIDE) continue;
-                    // tap offset (floor(v) + V0) sw + floor(u) + U0 as below
-                    const unsigned xb = __float_as_uint(q ? tu.y : tu.x), yb = __float_as_uint(q ? tv.y : tv.x);
-                    const unsigned o = min(yb * (unsigned)sw + xb + kb, last);
-                    MVS_BOUND(o <= last);
-                    const float4 t = __ldg(qd + o);
-                    const float2 lo = make_float2(t.x, t.y), hi = make_float2(t.z, t.w);
-                    const float2 tb = __ffma2_rn(pm_dup(q ? fx.y : fx.x), pm_sub2(hi, lo), lo);   // (top, bottom)
-                    const float J = fmaf(q ? fy.y : fy.x, tb.y - tb.x, tb.x);
-                    float Jp = J - mJ, Iv = q ? iv.y : iv.x;
-                    if (!ALLFIN) {
-                        const bool ok = Iv == Iv;
-                        Jp = ok ? Jp : 0.f;
-                        Iv = ok ? Iv : 0.f;
-                    }
-                    T1 += Jp;
-                    T2 = fmaf(Jp, Jp, T2);
-                    X = fmaf(Iv, Jp, X);
+            for (int q = 0; q < 2; ++q) {
+                if (q == 1 && !both) continue;
+                // tap offset (floor(v) + V0) sw + floor(u) + U0 as below
+                const unsigned xb = __float_as_uint(q ? tu.y : tu.x), yb = __float_as_uint(q ? tv.y : tv.x);
+                const unsigned o = min(yb * (unsigned)sw + xb + kb, last);
+                MVS_BOUND(o <= last);
+                const float4 t = __ldg(qd + o);
+                const float2 lo = make_float2(t.x, t.y), hi = make_float2(t.z, t.w);
+                const float2 tb = __ffma2_rn(pm_dup(q ? fx.y : fx.x), pm_sub2(hi, lo), lo);   // (top, bottom)
+                const float J = fmaf(q ? fy.y : fy.x, tb.y - tb.x, tb.x);
+                float Jp = J - mJ, Iv = q ? iv.y : iv.x;
+                if (!ALLFIN) {
+                    const bool ok = Iv == Iv;
+                    Jp = ok ? Jp : 0.f;
+                    Iv = ok ? Iv : 0.f;
                 }
+                T1 += Jp;
+                T2 = fmaf(Jp, Jp, T2);
+                X = fmaf(Iv, Jp, X);
             }
+        };
+        if constexpr (Acc::FLAT) {
+            constexpr int FULL = NSIDE * NSIDE / 2;
+#pragma unroll PM_FLAT_AHEAD
+            for (int m = 0; m < FULL; ++m) two(0, m, true);
+            if (NSIDE % 2) two(0, FULL, false);
+        } else {
+#pragma unroll 1
+            for (int row = 0; row < NSIDE; ++row)
+#pragma unroll
+                for (int m = 0; m < (NSIDE + 1) / 2; ++m) two(row, m, 2 * m + 1 < NSIDE);
+        }
         return;
     }
     // rows rolled, the samples of a row unrolled when the side is known (the checked form, rare,
@@ -1148,6 +1175,7 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
     // rows of M (which only multiply ray_q - ray_p) in float32.
     const double* p = c.par + 18 * sl;
     const double* bs = c.bsrc + 3 * sl;
+    const float *pf = c.parf + 18 * sl, *bsf = c.bsf + 3 * sl;   // their float32 values
     const double rp[3] = {rpx, rpy, rpz};
     double cen[3];
 #pragma unroll
@@ -1159,8 +1187,8 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
     const double f = p[12], pcx = p[16], pcy = p[17];
     // the centre's camera depth is zp / ndr: in front of the source needs zp < 0
     const bool front = zp < 0.0;
-    const float ff = (float)f, rzf = front ? __fdividef(1.0f, (float)zp) : 0.f;
-    const float ucf = fmaf(ff, (float)xp * rzf, (float)pcx), vcf = fmaf(ff, (float)yp * rzf, (float)pcy);
+    const float ff = pf[12], rzf = front ? __fdividef(1.0f, (float)zp) : 0.f;
+    const float ucf = fmaf(ff, (float)xp * rzf, pf[16]), vcf = fmaf(ff, (float)yp * rzf, pf[17]);
     const float Uf = fminf(fmaxf(floorf(ucf), -1048576.f), 1048576.f);
     const float Vf = fminf(fmaxf(floorf(vcf), -1048576.f), 1048576.f);
     const bool anchor = front && Uf == Uf && Vf == Vf;
@@ -1172,9 +1200,9 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
         const float nj = j == 0 ? n0 : (j == 1 ? n1 : n2);
-        const float mx = fmaf((float)bs[0], nj, numf * (float)p[j]);
-        const float my = fmaf((float)bs[1], nj, numf * (float)p[3 + j]);
-        const float mz = fmaf((float)bs[2], nj, numf * (float)p[6 + j]);
+        const float mx = fmaf(bsf[0], nj, numf * pf[j]);
+        const float my = fmaf(bsf[1], nj, numf * pf[3 + j]);
+        const float mz = fmaf(bsf[2], nj, numf * pf[6 + j]);
         A[j] = fmaf(ff, mx, auf * mz);
         B[j] = fmaf(ff, my, avf * mz);
         C[j] = mz;
@@ -1188,9 +1216,10 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
     // the window sums' tap offset: yb sw + xb + kb for floor bits xb, yb (unsigned, wrapping)
     const unsigned kb = (unsigned)vb * (unsigned)sw + (unsigned)ub;
     const float4* qd = c.quad[sl];
-    // ---- corners: the whole window in front and inside (outside) the source
-    bool den_ok = true, inside = anchor, front_all = true;
-    int out_lo_u = 0, out_hi_u = 0, out_lo_v = 0, out_hi_v = 0;
+    // ---- corners: the whole window in front and inside (outside) the source (by the extremes: four
+    // comparisons a unit in place of eight a corner)
+    bool den_ok = true, front_all = true;
+    float ul0 = 0.f, ul1 = 0.f, vl0 = 0.f, vl1 = 0.f;        // extremes over the corners, NaN if one is
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const float4 w = win.corner(k, NW);
@@ -1202,15 +1231,14 @@ __device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>
         const float ul = aq * rc, vl = bq * rc;
         den_ok = den_ok && den < -1e-3f;
         front_all = front_all && cq < 1e-2f * den;
-        inside = inside && ul >= lou + 1.f && ul <= hiu - 1.f && vl >= lov + 1.f && vl <= hiv - 1.f;
-        out_lo_u += ul < lou - 1.f;
-        out_hi_u += ul > hiu + 1.f;
-        out_lo_v += vl < lov - 1.f;
-        out_hi_v += vl > hiv + 1.f;
+        ul0 = k ? pm_min_nan(ul0, ul) : ul;
+        ul1 = k ? pm_max_nan(ul1, ul) : ul;
+        vl0 = k ? pm_min_nan(vl0, vl) : vl;
+        vl1 = k ? pm_max_nan(vl1, vl) : vl;
     }
-    inside = inside && den_ok && front_all;
-    const bool outside = den_ok && front_all && anchor &&
-                         (out_lo_u == 4 || out_hi_u == 4 || out_lo_v == 4 || out_hi_v == 4);
+    const bool known = den_ok && front_all && anchor;
+    const bool inside = known && ul0 >= lou + 1.f && ul1 <= hiu - 1.f && vl0 >= lov + 1.f && vl1 <= hiv - 1.f;
+    const bool outside = known && (ul1 < lou - 1.f || ul0 > hiu + 1.f || vl1 < lov - 1.f || vl0 > hiv + 1.f);
     // ---- source shift: the source at the window centre (the anchor), else 0
     float mJ = 0.f;
     if (anchor && !outside) {
@@ -1375,7 +1403,7 @@ struct PMLaneWin<0> {
 };
 // float4 entries of one pixel's staged window (nside: the compile-time side or 0; nw: its samples)
 __host__ __device__ constexpr int pm_lane_entries(int nside, int nw) {
-    return nside > 0 ? 2 * nside * ((nside + 1) / 2) + 5 : nw + 4;
+    return nside > 0 ? 2 * ((nside * nside + 1) / 2) + 5 : nw + 4;
 }
 
 // PHASE 0: current plane and propagation; PHASE 1: the random trials.
@@ -1446,21 +1474,21 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
             }
             if constexpr (NSIDE > 0) {
                 if (e < nw) {
-                    float* f = reinterpret_cast<float*>(win) + Acc::slot(e / NSIDE, e % NSIDE);
+                    float* f = reinterpret_cast<float*>(win) + Acc::slot(e);
                     f[0] = v.x;
                     f[2] = v.y;
                     f[4] = v.z;
                     f[6] = v.w;
                 } else {
-                    win[2 * NSIDE * Acc::NP + e - nw] = v;
+                    win[2 * Acc::NP + e - nw] = v;
                 }
             } else {
                 win[e] = v;
             }
         }
-        if constexpr (NSIDE % 2 == 1 && NSIDE > 0) {   // the surplus sample of a row's last pair: the centre ray
-            for (int e = lane; e < NSIDE; e += L) {
-                float* f = reinterpret_cast<float*>(win) + Acc::slot(e, NSIDE);
+        if constexpr (NSIDE % 2 == 1 && NSIDE > 0) {   // the surplus sample of the last pair: the centre ray
+            if (lane == 0) {
+                float* f = reinterpret_cast<float*>(win) + Acc::slot(NSIDE * NSIDE);
                 f[0] = f[2] = f[4] = f[6] = 0.f;
             }
         }
@@ -1474,7 +1502,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
         float si = 0.f, sii = 0.f;
         for (int e = lane; e < nw; e += L) {
             float* f;
-            if constexpr (NSIDE > 0) f = reinterpret_cast<float*>(win) + Acc::slot(e / NSIDE, e % NSIDE) + 6;
+            if constexpr (NSIDE > 0) f = reinterpret_cast<float*>(win) + Acc::slot(e) + 6;
             else f = &win[e].w;
             const float I = *f;
             if (I == I) {
@@ -1624,7 +1652,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
 // sums add the same terms in another order).
 // Blocks of 4 warps; the trials of 4 iterations at 4000 x 3000, 8 sources: single samples from a tile of
 // 16-byte entries (half of its wavefronts bank conflicts) 88.0 ms at 4 blocks per SM; pairs from
-// planes 84.3 ms at 3 (168 registers), 89.7 ms at 4 (128, spills).
+// planes 84.3 ms at 3 (168 registers; 82.7 with the shorter unit set-up), 89.7 ms at 4 (128, spills).
 constexpr int PM_TRIAL_WARPS = 4;   // warps per block
 #ifndef PM_TRIAL_MIN_BLOCKS
 #define PM_TRIAL_MIN_BLOCKS 3

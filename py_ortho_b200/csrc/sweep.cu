@@ -374,7 +374,16 @@ extern "C" mvs_status mvs_sweep(const mvs_sweep_args* a, void* stream) {
     int nch = 1;
     const size_t need = sweep_scratch_bytes(a, &nch);
     void* ws = nullptr;
-    if (need) MVS_CUDA(cudaMallocAsync(&ws, need, st), "sweep: chunk-record scratch");
+    if (need) {
+        const cudaError_t e = cudaMallocAsync(&ws, need, st);
+        if (e == cudaErrorMemoryAllocation && a->plane_chunks <= 0) {   // no room: the same result in one chunk
+            cudaGetLastError();
+            mvs_sweep_args one = *a;
+            one.plane_chunks = 1;
+            return sweep_with_scratch(&one, nullptr, 0, st);
+        }
+        MVS_CUDA(e, "sweep: chunk-record scratch");
+    }
     mvs_status s = sweep_with_scratch(a, ws, need, st);
     if (ws) cudaFreeAsync(ws, st);
     return s;

@@ -331,7 +331,7 @@ def run_ours(a):
                    "evals_per_s": pm_evals / (ms_pm / 1e3),
                    "ms": round(ms_pm, 3), "share_of_step": round(ms_pm / (ms_pm + ms_sweep), 4),
                    "ncu_profile": PM_PROFILE[a.pm_precision],
-                   "issue_active_ncu": ({"propagation": 0.668, "trials": 0.505} if a.pm_precision == "fp32"
+                   "issue_active_ncu": ({"propagation": 0.605, "trials": 0.406} if a.pm_precision == "fp32"
                                         else 0.667),
                    "note": "not a contraction and not HBM-bound (DRAM < 2 %): propagation is bound by SIMT "
                            "issue, the trials by latency at low occupancy; issue_active is the fraction of SM "
@@ -385,14 +385,13 @@ def run_ours(a):
     L.check_device_faults()        # a sweep tile that gave up its bounded wait makes the run fail
     dominant = "pm" if ms_pm > ms_sweep else "sweep"
     # our kernels per step: the sweep (+ the ordered chunk merge when its planes are split over
-    # CTAs: mvs_sweep's automatic rule, tiles below 6 CTAs per SM), finalize, and per PatchMatch
-    # call the stream start, the float32 mode's footprint images (one launch per source) and, per
-    # colour pass, propagation, count, scan, stream states, trials
-    th_ = a.tile_h or 32
-    tiles = ((W + 63) // 64) * ((H + th_ - 1) // th_)
-    sweep_launches = 1 if tiles >= 6 * torch.cuda.get_device_properties(dev).multi_processor_count else 2
-    fp_launches = nsrc if a.pm_precision == "fp32" else 0
-    launches = sweep_launches + 1 + ((1 + fp_launches + 10 * iters) if iters else 0)
+    # CTAs: then it needs scratch), finalize, and per PatchMatch call the stream start, the float32
+    # mode's footprint images (one launch per source) or the float64 mode's image bounds and active
+    # lists, and, per colour pass, (current planes in float64,) propagation, count, scan, stream
+    # states, trials
+    sweep_launches = 1 + int(lib.mvs_sweep_scratch_bytes(ctypes.addressof(a_sw)) > 0)
+    pm_launches = (1 + nsrc + 10 * iters) if a.pm_precision == "fp32" else (1 + 2 + nsrc + 6 + 12 * iters)
+    launches = sweep_launches + 1 + (pm_launches if iters else 0)
     line = {
         "metric": "ZNCC evaluations/s (pixel x plane x view), sweep + PatchMatch",
         "value": value / 1e9, "unit": "Gpix.plane.view/s", "n_gpus": world, "steps": a.steps,
@@ -625,10 +624,10 @@ def cpu_baseline(cfg, nplanes, iters, device="cpu"):
 
 
 CHECK_ROWS = 64        # rows of the timed step's sweep that --check validates
-# thread instructions per evaluation of the FP32 plane sweep (smsp__thread_inst_executed.sum of
-# one launch at 3000 x 2250, 8 sources, r = 3: 157.8 at 16 planes, 157.0 at 64;
-# profiles/sweep_kernel_3000x2250_8src_16planes.md)
-SWEEP_INST_PER_EVAL = 157.0
+# thread instructions per evaluation of the FP32 plane sweep, sources outside a tile skipped and
+# samples in packed pairs (smsp__thread_inst_executed.sum of one launch at 3000 x 2250, 8 sources,
+# r = 3, 16 planes; profiles/sweep_kernel_3000x2250_8src_16planes.md)
+SWEEP_INST_PER_EVAL = 72.3
 
 
 def reference_band_check(sc, ref_h, srcs_h, geo, planes, r, top_k, band):

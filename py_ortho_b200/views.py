@@ -22,7 +22,7 @@ reference's pass 2 reads it).
 from __future__ import annotations
 
 import ctypes
-from typing import Callable, Dict, List, Optional, Sequence
+from typing import Callable, Dict, Iterable, List, Optional, Sequence
 
 import numpy as np
 import torch
@@ -187,41 +187,32 @@ def repair(k: int, raw: Dict[int, torch.Tensor], score: torch.Tensor, low: torch
 FUSE_GROUP_ROWS = 1 << 24        # candidate pixels per group of views (32 bytes each: 0.5 GB of output space)
 
 
-def fuse(order: Sequence[int], maps: Dict[int, object], cams, nbrs, rel_tols, px_tol: float, min_views: int,
+def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px_tol: float, min_views: int,
          point_stride: int, rgbs):
     """Point fusion of the final depth maps (densify._fuse, densify.py:676-762) on the device:
     views in `order` (the reference fuses sorted(have)), one ``mvs_fuse_view`` launch each, the
     used masks carried from view to view on the device. maps[k]: (H, W) depth (NaN = none);
-    nbrs[k]: neighbour ids; rel_tols[k][j]: relative depth tolerance; rgbs[k]: (H, W, 3) uint8.
+    nbrs[k]: neighbour ids; rel_tols[k][j]: relative depth tolerance; rgbs[k]: (H, W, 3) uint8, read
+    once per view, when its turn comes.
     Returns (xyz float64 (n, 3), colours uint8 (n, 3), views uint8 (n,), owner int32 (n,)) as
     torch CUDA tensors in the reference's order (views in order, pixels row-major), and the
     used masks {k: bool tensor}."""
     dev = L.require_cuda()
     lib = L.load()
+    order = [k for k in order if k in maps]          # taken once: any iterable
     D = {k: _dev32(m, dev) for k, m in maps.items()}
     used = {k: torch.zeros(tuple(D[k].shape), dtype=torch.uint8, device=dev) for k in D}
     st = max(int(point_stride), 1)
     cand = {k: -(-int(d.shape[0]) // st) * -(-int(d.shape[1]) // st) for k, d in D.items()}
     sh = L.stream_handle()
 
-    def dev_rgb(k):
-        rgb = torch.as_tensor(np.ascontiguousarray(rgbs[k]), device=dev) if not isinstance(rgbs[k], torch.Tensor) \
-            else rgbs[k].to(dev)
-        return rgb.reshape(-1, 3)
+    def colours(k):
+        c = rgbs[k]
+        c = c.to(dev) if isinstance(c, torch.Tensor) else torch.as_tensor(np.ascontiguousarray(c), device=dev)
+        return c.reshape(-1, 3)
 
-    def uint8_rgb(k):
-        try:
-            c = rgbs[k]
-        except (KeyError, IndexError):
-            return False
-        c = c if isinstance(c, torch.Tensor) else np.asarray(c)
-        return c.dtype in (torch.uint8, np.uint8) and int(np.prod(c.shape)) == 3 * int(D[k].numel())
-
-    # colours of another type, or of some views only, are picked by torch, view by view
-    plain = all(uint8_rgb(k) for k in order if k in D)
-    other: list = []
-    parts: List[tuple] = []
-    todo = [k for k in order if k in D]
+    pts, cols, nv, owner = [], [], [], []
+    todo = list(order)
     while todo:
         # the views of a group append to one set of arrays, and the host waits once for their number
         # of points (a wait per view left the device idle between views)
@@ -238,6 +229,7 @@ def fuse(order: Sequence[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
                torch.empty(rows, dtype=torch.uint8, device=dev), torch.empty(rows, dtype=torch.int32, device=dev))
         ws = torch.empty(max(lib.mvs_fuse_append_scratch_bytes(*(int(v) for v in D[k].shape), st) for k in group) or 1,
                          dtype=torch.uint8, device=dev)
+        picked = []                  # (first row, end row, colours) of the views whose colours torch picks
         for k in group:
             H, W = (int(v) for v in D[k].shape)
             nb = [j for j in nbrs[k] if j in D and j != k]
@@ -255,23 +247,41 @@ def fuse(order: Sequence[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
             a.nb_cam, a.rel_tol, a.px_tol, a.min_views = L.host_ptr(nb_cam), L.host_ptr(tol), float(px_tol), int(min_views)
             a.keep, a.xyz, a.count = keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr()
             L.check(lib.mvs_fuse_view(ctypes.addressof(a), sh), "fuse")
-            rgb = dev_rgb(k).contiguous() if plain else torch.zeros(3 * H * W, dtype=torch.uint8, device=dev)
+            rgb, missing = None, None
+            try:
+                rgb = colours(k)
+            except Exception as e:                       # raised below if the view keeps a point
+                missing = e
+            direct = rgb is not None and rgb.dtype == torch.uint8 and int(rgb.shape[0]) == H * W
+            rgb8 = rgb.contiguous() if direct else torch.empty(3 * H * W, dtype=torch.uint8, device=dev)
             b = L.FuseAppendArgs()
             b.H, b.W, b.point_stride, b.owner = H, W, st, int(k)
-            b.keep, b.xyz, b.count, b.rgb, b.rows = (keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr(), rgb.data_ptr(),
+            b.keep, b.xyz, b.count, b.rgb, b.rows = (keep.data_ptr(), xyz.data_ptr(), cnt.data_ptr(), rgb8.data_ptr(),
                                                      n_rows.data_ptr())
             b.out_xyz, b.out_rgb, b.out_views, b.out_owner = (t.data_ptr() for t in out)
             b.scratch = ws.data_ptr()
             L.check(lib.mvs_fuse_append(ctypes.addressof(b), sh), "fuse append")
-            if not plain:
+            if not direct:                               # another type or size, or none
                 sel = torch.nonzero(keep[:H * W]).squeeze(1)
                 if sel.numel():
-                    other.append(dev_rgb(k)[sel])
+                    if missing is not None:
+                        raise missing
+                    if int(sel[-1]) >= int(rgb.shape[0]):
+                        raise IndexError(f"fuse: view {k} has {int(rgb.shape[0])} colours for its {H} x {W} pixels")
+                    at = int(n_rows[1].item())
+                    picked.append((at, at + int(sel.numel()), rgb[sel]))
         n = int(n_rows[0].item())
         if n:
-            parts.append(tuple(t[:n].clone() if todo or parts else t[:n] for t in out))
-    pts, cols, nv, owner = ([p[q] for p in parts] for q in range(4))
-    cols = cols if plain else other
+            own = (lambda t: t.clone()) if todo or pts else (lambda t: t)    # gives the group's arrays back
+            for dst, t in zip((pts, nv, owner), (out[0], out[2], out[3])):
+                dst.append(own(t[:n]))
+            at = 0
+            for lo, hi, c in picked + [(n, n, None)]:
+                if lo > at:
+                    cols.append(own(out[1][at:lo]))
+                if c is not None:
+                    cols.append(c)
+                at = hi
 
     def cat(a, shape, dt):
         return torch.cat(a) if a else torch.zeros(shape, dtype=dt, device=dev)

@@ -212,12 +212,12 @@ def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
         return c.reshape(-1, 3)
 
     pts, cols, nv, owner = [], [], [], []
-    todo = list(order)
+    todo, limit = list(order), FUSE_GROUP_ROWS
     while todo:
         # the views of a group append to one set of arrays, and the host waits once for their number
         # of points (a wait per view left the device idle between views)
         group, rows = [], 0
-        while todo and (not group or rows + cand[todo[0]] <= FUSE_GROUP_ROWS):
+        while todo and (not group or rows + cand[todo[0]] <= limit):
             group.append(todo.pop(0))
             rows += cand[group[-1]]
         px = max(int(D[k].numel()) for k in group)
@@ -225,8 +225,17 @@ def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
         xyz = torch.empty(3 * px, dtype=torch.float64, device=dev)
         cnt = torch.empty(px, dtype=torch.int32, device=dev)
         n_rows = torch.zeros(2, dtype=torch.int64, device=dev)
-        out = (torch.empty((rows, 3), dtype=torch.float64, device=dev), torch.empty((rows, 3), dtype=torch.uint8, device=dev),
-               torch.empty(rows, dtype=torch.uint8, device=dev), torch.empty(rows, dtype=torch.int32, device=dev))
+        try:
+            out = (torch.empty((rows, 3), dtype=torch.float64, device=dev),
+                   torch.empty((rows, 3), dtype=torch.uint8, device=dev),
+                   torch.empty(rows, dtype=torch.uint8, device=dev), torch.empty(rows, dtype=torch.int32, device=dev))
+        except torch.cuda.OutOfMemoryError:
+            # no room for a place per candidate: views one by one, and then only the kept points' places
+            limit = 0
+            if len(group) > 1:
+                todo, keep, xyz, cnt = group + todo, None, None, None
+                continue
+            out = None
         ws = torch.empty(max(lib.mvs_fuse_append_scratch_bytes(*(int(v) for v in D[k].shape), st) for k in group) or 1,
                          dtype=torch.uint8, device=dev)
         picked = []                  # (first row, end row, colours) of the views whose colours torch picks
@@ -252,7 +261,20 @@ def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
                 rgb = colours(k)
             except Exception as e:                       # raised below if the view keeps a point
                 missing = e
-            direct = rgb is not None and rgb.dtype == torch.uint8 and int(rgb.shape[0]) == H * W
+            direct = out is not None and rgb is not None and rgb.dtype == torch.uint8 and int(rgb.shape[0]) == H * W
+            if not direct:
+                sel = torch.nonzero(keep[:H * W]).squeeze(1)
+                if sel.numel() and missing is not None:
+                    raise missing
+                if sel.numel() and int(sel[-1]) >= int(rgb.shape[0]):
+                    raise IndexError(f"fuse: view {k} has {int(rgb.shape[0])} colours for its {H} x {W} pixels")
+                if out is None:
+                    if sel.numel():
+                        pts.append(xyz[:3 * H * W].view(3, -1)[:, sel].T)
+                        cols.append(rgb[sel])
+                        nv.append(cnt[sel].clamp(max=255).to(torch.uint8))
+                        owner.append(torch.full((sel.numel(),), int(k), dtype=torch.int32, device=dev))
+                    continue
             rgb8 = rgb.contiguous() if direct else torch.empty(3 * H * W, dtype=torch.uint8, device=dev)
             b = L.FuseAppendArgs()
             b.H, b.W, b.point_stride, b.owner = H, W, st, int(k)
@@ -261,15 +283,9 @@ def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
             b.out_xyz, b.out_rgb, b.out_views, b.out_owner = (t.data_ptr() for t in out)
             b.scratch = ws.data_ptr()
             L.check(lib.mvs_fuse_append(ctypes.addressof(b), sh), "fuse append")
-            if not direct:                               # another type or size, or none
-                sel = torch.nonzero(keep[:H * W]).squeeze(1)
-                if sel.numel():
-                    if missing is not None:
-                        raise missing
-                    if int(sel[-1]) >= int(rgb.shape[0]):
-                        raise IndexError(f"fuse: view {k} has {int(rgb.shape[0])} colours for its {H} x {W} pixels")
-                    at = int(n_rows[1].item())
-                    picked.append((at, at + int(sel.numel()), rgb[sel]))
+            if not direct and sel.numel():               # colours of another type or size
+                at = int(n_rows[1].item())
+                picked.append((at, at + int(sel.numel()), rgb[sel]))
         n = int(n_rows[0].item())
         if n:
             own = (lambda t: t.clone()) if todo or pts else (lambda t: t)    # gives the group's arrays back
@@ -282,6 +298,7 @@ def fuse(order: Iterable[int], maps: Dict[int, object], cams, nbrs, rel_tols, px
                 if c is not None:
                     cols.append(c)
                 at = hi
+        keep, xyz, cnt, out = None, None, None, None
 
     def cat(a, shape, dt):
         return torch.cat(a) if a else torch.zeros(shape, dtype=dt, device=dev)

@@ -75,3 +75,33 @@ def test_colours_of_mixed_types(rows, monkeypatch):
     del mixed[1]
     with pytest.raises(KeyError):
         V.fuse(range(5), maps, cams, nbrs, tols, 1.5, 2, 1, mixed)
+
+
+@pytest.mark.parametrize("room", [64 << 10, 24 << 10])
+def test_without_room_for_every_candidate(room, monkeypatch):
+    """Allocations above `room` bytes fail once the first has: 5 x 1924 candidates take 231 KB, one view's 46 KB
+    (views one by one), and with less room than that only the kept points' places are taken."""
+    from py_ortho_b200 import views as V
+    maps, cams, nbrs, tols, rgbs = _flight(seed=3)
+    want = O.fuse(range(5), maps, cams, nbrs, tols, 1.5, 2, 1, rgbs)
+    empty, refused = torch.empty, []
+
+    def limited(*a, **kw):
+        t = empty(*a, **kw)
+        # the (candidates, 3) arrays of points; the views' own arrays are flat
+        if kw.get("dtype") is torch.float64 and t.ndim == 2 and t.numel() * 8 > room:
+            refused.append(t.numel())
+            raise torch.cuda.OutOfMemoryError("no room")
+        return t
+    monkeypatch.setattr(torch, "empty", limited)
+    got = V.fuse(iter(range(5)), maps, cams, nbrs, tols, 1.5, 2, 1, rgbs)
+    monkeypatch.undo()
+    _same(got, want)
+    assert len(refused) == (1 if room > 46176 else 6)
+    mixed = dict(rgbs)
+    mixed[1] = rgbs[1].astype(np.float32)
+    monkeypatch.setattr(torch, "empty", limited)
+    got = V.fuse(range(5), maps, cams, nbrs, tols, 1.5, 2, 1, mixed)
+    monkeypatch.undo()
+    assert got[1].dtype == torch.float32
+    _same((got[0], got[1].to(torch.uint8), got[2], got[3]), want)

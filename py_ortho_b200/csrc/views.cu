@@ -197,6 +197,9 @@ __global__ void __launch_bounds__(256) init_normals_kernel(int H, int W, const f
 }
 
 
+// Stride-grid positions 0, st, 2 st, ... < n, for n >= 1 and any st >= 1 (n + st may pass 2^31).
+__host__ __device__ inline int stride_cells(int n, int st) { return (n - 1) / st + 1; }
+
 // Fusion of one reference image (densify._fuse_loop, densify.py:688-762): the forward-backward
 // check of consistency_kernel for every neighbour in order, the agreeing neighbours' points added
 // to the pixel's own (acc starts at X, cnt at 1), kept when cnt >= min_views, and the agreeing
@@ -223,10 +226,10 @@ struct FuseParams {
 
 __global__ void __launch_bounds__(256) fuse_kernel(const __grid_constant__ FuseParams c) {
     const long long HW = (long long)c.H * c.W;
-    const int st = c.stride, gw = (c.W + st - 1) / st;
+    const int st = c.stride, gw = stride_cells(c.W, st);
     const long long cand = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (cand >= (long long)stride_cells(c.H, st) * gw) return;
     const int y = (int)(cand / gw) * st, x = (int)(cand % gw) * st;
-    if (y >= c.H) return;
     const long long idx = (long long)y * c.W + x;
     const float Dv = c.depth[idx];
     if (!isfinite(Dv) || c.used[idx]) return;
@@ -312,7 +315,7 @@ struct AppendParams {
 constexpr int APPEND_BLOCK = 1024;
 
 __device__ __forceinline__ bool append_kept(const AppendParams& c, long long cand, long long& idx) {
-    const int gw = (c.W + c.stride - 1) / c.stride;
+    const int gw = stride_cells(c.W, c.stride);
     const long long y = cand / gw * c.stride, x = cand % gw * c.stride;
     if (y >= c.H) return false;
     idx = y * c.W + x;
@@ -473,7 +476,7 @@ extern "C" mvs_status mvs_fuse_view(const mvs_fuse_args* a, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     MVS_CUDA(cudaMemsetAsync(p.keep, 0, (size_t)HW, st), "fuse: clear keep");
     MVS_CUDA(cudaMemsetAsync(p.count, 0, (size_t)HW * sizeof(int), st), "fuse: clear count");
-    const long long cand = (long long)((a->H + p.stride - 1) / p.stride) * ((a->W + p.stride - 1) / p.stride);
+    const long long cand = (long long)stride_cells(a->H, p.stride) * stride_cells(a->W, p.stride);
     fuse_kernel<<<(unsigned)((cand + 255) / 256), 256, 0, st>>>(p);
     return check_launch("fuse kernel");
 }
@@ -481,7 +484,7 @@ extern "C" mvs_status mvs_fuse_view(const mvs_fuse_args* a, void* stream) {
 extern "C" size_t mvs_fuse_append_scratch_bytes(int32_t H, int32_t W, int32_t point_stride) {
     if (H < 1 || W < 1) return 0;
     const int s = point_stride > 1 ? point_stride : 1;
-    const long long cand = (long long)((H + s - 1) / s) * ((W + s - 1) / s);
+    const long long cand = (long long)stride_cells(H, s) * stride_cells(W, s);
     return (size_t)((cand + APPEND_BLOCK - 1) / APPEND_BLOCK) * sizeof(unsigned);
 }
 

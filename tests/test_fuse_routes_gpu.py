@@ -105,3 +105,16 @@ def test_without_room_for_every_candidate(room, monkeypatch):
     monkeypatch.undo()
     assert got[1].dtype == torch.float32
     _same((got[0], got[1].to(torch.uint8), got[2], got[3]), want)
+
+
+@pytest.mark.parametrize("stride", [36, 37, 52, 53, 2**31 - 60, 2**31 - 1])
+def test_strides_around_and_far_beyond_the_image(stride):
+    """37 x 52 pixels: from 2 x 2 candidates to the first pixel alone."""
+    from py_ortho_b200 import _lib as L, views as V
+    maps, cams, nbrs, tols, rgbs = _flight(seed=4)
+    for m in maps.values():
+        m[0, 0] = 40.0
+    want = O.fuse(range(5), maps, cams, nbrs, tols, 1.5, 1, stride, rgbs)
+    assert len(want[0]) > 0
+    _same(V.fuse(range(5), maps, cams, nbrs, tols, 1.5, 1, stride, rgbs), want)
+    assert L.load().mvs_fuse_append_scratch_bytes(37, 52, stride) == 4

@@ -58,6 +58,19 @@ inline int num_sms() {
     return n;
 }
 
+// A launch's dynamic shared memory where its size depends on the call. The limit that a kernel may be
+// launched with is state of the function on its device, shared by every host thread, so it is always
+// set to the same value, the most a block can have (kernels with static shared memory: less): a limit
+// of this call's own size could be lowered by another thread between here and the launch.
+constexpr size_t MVS_SMEM_MAX = 227 * 1024;
+template <class K>
+inline mvs_status allow_smem(K kern, size_t smem, const char* what) {
+    if (smem > MVS_SMEM_MAX)
+        return fail(MVS_ERR_CUDA, "%s: %zu bytes of shared memory above the %zu of a block", what, smem, MVS_SMEM_MAX);
+    MVS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MVS_SMEM_MAX), what);
+    return MVS_OK;
+}
+
 // Bounds-checked debug build (nvcc -DMVS_DEBUG_BOUNDS; `python -m py_ortho_b200.build
 // --debug-bounds` writes libmvs_b200_debug.so): MVS_BOUND(cond) counts every shared-memory or
 // global index the instrumented kernels (tile engine, batched / server kernels, PatchMatch) would

@@ -858,8 +858,7 @@ extern "C" mvs_status mvs_height_eval(const mvs_height_eval_args* a, void* scrat
     MVS_TRY(check_launch("height samples"));
     float* box = reinterpret_cast<float*>(ws + l.o_box);
     const size_t smem = height_box_smem(a->W, a->r);
-    MVS_CUDA(cudaFuncSetAttribute(height_box_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-             "height box: shared memory attribute");
+    MVS_TRY(allow_smem(height_box_kernel, smem, "height box: shared memory attribute"));
     height_box_kernel<<<dim3(l.planes, a->D), 256, smem, st>>>(p, a->r, box);
     MVS_TRY(check_launch("height box"));
     q.V = a->V; q.D = a->D; q.H = a->H; q.W = a->W; q.topk = a->topk;

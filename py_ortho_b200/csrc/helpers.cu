@@ -225,10 +225,7 @@ static mvs_status box_rows(int H, int W, int r, float* io0, float* io1, cudaStre
 
 static mvs_status box_rows_wide(int H, int W, int r, float* io, cudaStream_t st) {
     const size_t smem = (size_t)2 * W * sizeof(float);
-    if (smem > 48 * 1024) {
-        MVS_CUDA(cudaFuncSetAttribute(box_row_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                 "box: shared memory attribute");
-    }
+    if (smem > 48 * 1024) MVS_TRY(allow_smem(box_row_wide_kernel, smem, "box: shared memory attribute"));
     box_row_wide_kernel<<<H, 128, smem, st>>>(H, W, r, box_scale(r), io);
     return check_launch("box row pass");
 }

@@ -2040,10 +2040,8 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
         else if (lanes == 8) { PM_PICK(8, 0) PM_PICK(8, 1) }
         else { PM_PICK(16, 0) PM_PICK(16, 1) }
 #undef PM_PICK
-        for (int ph = 0; ph < 2 && status == MVS_OK; ++ph) {
-            if (cudaFuncSetAttribute(lane_kernel[ph], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-                status = fail(MVS_ERR_CUDA, "pm_refine: shared-memory carve-out");
-        }
+        for (int ph = 0; ph < 2 && status == MVS_OK; ++ph)
+            status = allow_smem(lane_kernel[ph], smem, "pm_refine: shared-memory carve-out");
     }
     // the trials: one lane per pixel (pm_trial_kernel) when the warps' tiles fit in shared memory,
     // else the lane groups' kernel
@@ -2052,7 +2050,7 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
     const int wpr = (int)(((a->W + 1) / 2 + 31) / 32);
     const unsigned grid_trial = (unsigned)(((long long)a->H * wpr + PM_TRIAL_WARPS - 1) / PM_TRIAL_WARPS);
 #if !PM_TRIAL_LANE_GROUPS
-    if (fast && status == MVS_OK && smem_trial <= 227 * 1024) {
+    if (fast && status == MVS_OK && smem_trial <= MVS_SMEM_MAX) {
 #define PM_PICK_TRIAL(LN)                                                                        \
     trial_kernel = side == 7 && a->step == 1   ? pm_trial_kernel<LN, 7, true>                       \
                    : side == 5 && a->step == 1 ? pm_trial_kernel<LN, 5, true>                       \
@@ -2063,9 +2061,9 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
         else if (lanes == 8) { PM_PICK_TRIAL(8) }
         else { PM_PICK_TRIAL(16) }
 #undef PM_PICK_TRIAL
-        if (cudaFuncSetAttribute(trial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_trial) !=
-            cudaSuccess) {
+        if (allow_smem(trial_kernel, smem_trial, "pm_refine: trials") != MVS_OK) {
             cudaGetLastError();
+            clear_error();
             trial_kernel = nullptr;
         }
     }

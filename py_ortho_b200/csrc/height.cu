@@ -285,7 +285,9 @@ struct EvalPlane {
 // division), where the three passes took 7.4 ms and ~4 ms for the stacked, squared, gathered and
 // multiplied copies that fed them.
 constexpr int HB_ROWS = 32, HB_AHEAD = 8;      // rows per step; rows whose loads are in flight together
-static size_t height_box_smem(int W, int r) { return (size_t)(HB_ROWS + 2 * r + 1) * (W + 1) * sizeof(double); }
+static size_t height_box_smem(int W, int r) {      // (the factors as 64 bits: 2 r may pass 2^31)
+    return ((size_t)HB_ROWS + 2 * (size_t)r + 1) * ((size_t)W + 1) * sizeof(double);
+}
 
 __global__ void __launch_bounds__(256) height_box_kernel(const __grid_constant__ EvalParams p, int r,
                                                          float* __restrict__ out) {

@@ -407,25 +407,25 @@ __global__ void __launch_bounds__(256) height_box_kernel(const __grid_constant__
 __global__ void __launch_bounds__(256) height_stack_kernel(int H, int W, int hc, int wc, int K, const float* __restrict__ Zc,
                                                            const float* __restrict__ offs, float* __restrict__ up,
                                                            float* __restrict__ stack) {
-    const int HW = H * W, i = blockIdx.x * 256 + threadIdx.x;
+    const long long HW = (long long)H * W, i = blockIdx.x * 256LL + threadIdx.x;
     if (i >= HW) return;
-    const int y = i / W, x = i - y * W;
-    const float z = Zc[(long long)(min(y, 2 * hc - 1) >> 1) * wc + (min(x, 2 * wc - 1) >> 1)];
+    const int y = (int)i / W, x = (int)i - y * W;            // (H W < 2^31)
+    const float z = Zc[(long long)min(y >> 1, hc - 1) * wc + min(x >> 1, wc - 1)];
     up[i] = z;
-    for (int k = 0; k < K; ++k) stack[(long long)k * HW + i] = __fadd_rn(z, __ldg(offs + k));
+    for (int k = 0; k < K; ++k) stack[k * HW + i] = __fadd_rn(z, __ldg(offs + k));
 }
 
 // The first best score's hypothesis; a best score below `weak` keeps the middle one; `parabola`: the
 // vertex through its neighbours' scores. out = (up + offs[b]) + frac * cell.
-__global__ void __launch_bounds__(256) height_pick_kernel(int HW, int K, const float* __restrict__ sc,
+__global__ void __launch_bounds__(256) height_pick_kernel(long long HW, int K, const float* __restrict__ sc,
                                                           const float* __restrict__ up, const float* __restrict__ offs,
                                                           float weak, int parabola, float cell, float* __restrict__ out) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
+    const long long i = blockIdx.x * 256LL + threadIdx.x;
     if (i >= HW) return;
     int b = 0;
     float best = sc[i];
     for (int k = 1; k < K; ++k) {
-        const float v = sc[(long long)k * HW + i];
+        const float v = sc[k * HW + i];
         if (v > best || (v != v && best == best)) {      // a NaN counts as the largest, the first one wins
             best = v;
             b = k;
@@ -433,11 +433,11 @@ __global__ void __launch_bounds__(256) height_pick_kernel(int HW, int K, const f
     }
     if (best < weak) {
         b = K / 2;
-        best = sc[(long long)b * HW + i];
+        best = sc[b * HW + i];
     }
     float frac = 0.f;
     if (parabola) {
-        const float lo = sc[(long long)max(b - 1, 0) * HW + i], hi = sc[(long long)min(b + 1, K - 1) * HW + i];
+        const float lo = sc[max(b - 1, 0) * HW + i], hi = sc[min(b + 1, K - 1) * HW + i];
         const float den = __fadd_rn(__fsub_rn(lo, __fmul_rn(2.f, best)), hi);
         if (den < -1e-6f && b > 0 && b < K - 1) {
             const float f = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(lo, hi)), den);
@@ -449,13 +449,13 @@ __global__ void __launch_bounds__(256) height_pick_kernel(int HW, int K, const f
 
 // 3 x 3 median with edge padding; NaN sorts last.
 __global__ void __launch_bounds__(256) median3_kernel(int H, int W, const float* __restrict__ a, float* __restrict__ out) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= H * W) return;
-    const int y = i / W, x = i - y * W;
+    const long long i = blockIdx.x * 256LL + threadIdx.x;
+    if (i >= (long long)H * W) return;
+    const int y = (int)i / W, x = (int)i - y * W;            // (H W < 2^31)
     float v[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        v[k] = a[(long long)min(max(y + k / 3 - 1, 0), H - 1) * W + min(max(x + k % 3 - 1, 0), W - 1)];
+        v[k] = a[(long long)min(max(y + (k / 3 - 1), 0), H - 1) * W + min(max(x + (k % 3 - 1), 0), W - 1)];
 #pragma unroll
     for (int k = 0; k < 5; ++k)                          // the five smallest in order
 #pragma unroll
@@ -882,8 +882,8 @@ extern "C" mvs_status mvs_height_stack(int32_t H, int32_t W, int32_t hc, int32_t
     if ((long long)H * W >= (1LL << 31)) return fail(MVS_ERR_VALUE, "height_stack: grid too large");
     if (H == 0 || W == 0) return MVS_OK;
     if (!Zc || !offs || !up || !stack) return fail(MVS_ERR_VALUE, "height_stack: null pointer");
-    height_stack_kernel<<<(H * W + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(H, W, hc, wc, K, Zc, offs,
-                                                                                               up, stack);
+    height_stack_kernel<<<(unsigned)(((long long)H * W + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        H, W, hc, wc, K, Zc, offs, up, stack);
     return check_launch("height stack");
 }
 
@@ -895,8 +895,9 @@ extern "C" mvs_status mvs_height_pick(int32_t H, int32_t W, int32_t K, const flo
     if ((long long)H * W >= (1LL << 31)) return fail(MVS_ERR_VALUE, "height_pick: grid too large");
     if (H == 0 || W == 0) return MVS_OK;
     if (!score || !up || !offs || !out) return fail(MVS_ERR_VALUE, "height_pick: null pointer");
-    height_pick_kernel<<<(H * W + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(H * W, K, score, up, offs,
-                                                                                              weak, parabola, cell, out);
+    const long long HW = (long long)H * W;
+    height_pick_kernel<<<(unsigned)((HW + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        HW, K, score, up, offs, weak, parabola, cell, out);
     return check_launch("height pick");
 }
 
@@ -906,6 +907,7 @@ extern "C" mvs_status mvs_median3(int32_t H, int32_t W, const float* a, float* o
     if ((long long)H * W >= (1LL << 31)) return fail(MVS_ERR_VALUE, "median3: image too large");
     if (H == 0 || W == 0) return MVS_OK;
     if (!a || !out || a == out) return fail(MVS_ERR_VALUE, "median3: bad pointers");
-    median3_kernel<<<(H * W + 255) / 256, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(H, W, a, out);
+    median3_kernel<<<(unsigned)(((long long)H * W + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        H, W, a, out);
     return check_launch("median3");
 }

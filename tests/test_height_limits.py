@@ -2,6 +2,7 @@
 import ctypes
 
 import pytest
+import torch
 
 
 def _eval_args(L, W, r, H=8, D=1):
@@ -23,3 +24,29 @@ def test_the_fused_evaluation_takes_what_its_window_means_fit(W, r, fits):
     need = L.load().mvs_height_eval_scratch_bytes(ctypes.addressof(a))
     assert fits == ((32 + 2 * r + 1) * (W + 1) * 8 <= 200 * 1024)
     assert (need > 0) == fits
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,W", [(1, 2**31 - 2), (2**31 - 2, 1)])
+def test_refinement_steps_on_the_largest_grids(H, W):
+    """Within 256 cells of 2^31 (8.6 GB an array), checked in pieces."""
+    from py_ortho_b200 import _lib as L
+    lib, sh, n = L.load(), L.stream_handle(), H * W
+    z = torch.rand(n // 2, device="cuda")
+    up, out = torch.empty(n, device="cuda"), torch.empty(n, device="cuda")
+    off = torch.tensor([0.25], device="cuda")
+    hc, wc = (1, W // 2) if H == 1 else (H // 2, 1)
+    L.check(lib.mvs_height_stack(H, W, hc, wc, z.data_ptr(), 1, off.data_ptr(), up.data_ptr(), out.data_ptr(), sh))
+    for o in (0, n // 4 * 2, n - 600):
+        want = z[o // 2:o // 2 + 300].repeat_interleave(2)
+        assert torch.equal(up[o:o + 600], want) and torch.equal(out[o:o + 600], want + 0.25)
+    # a single score is its own best: up + offs[0]
+    L.check(lib.mvs_height_pick(H, W, 1, up.data_ptr(), up.data_ptr(), off.data_ptr(), 0.0, 1, 1.0, out.data_ptr(), sh))
+    assert torch.equal(out[-600:], up[-600:] + 0.25) and torch.equal(out[:600], up[:600] + 0.25)
+    L.check(lib.mvs_median3(H, W, up.data_ptr(), out.data_ptr(), sh))
+    for o in (0, n - 600):
+        v = up[o:o + 600]
+        lo, hi = torch.cat([v[:1], v[:-1]]), torch.cat([v[1:], v[-1:]])
+        want = torch.sort(torch.stack([lo, v, hi]), dim=0).values[1]       # three equal rows (columns): the middle of 3
+        s = slice(0, 599) if o == 0 else slice(1, 600)
+        assert torch.equal(out[o:o + 600][s], want[s])

@@ -34,6 +34,9 @@ struct PMStats;
 
 struct PMParams {
     int H, W, S, r, step, top_k, it, colour;
+    int last;                           // the window's last offset, -r + m step <= r
+    float r2;                           // r r
+    int few;                            // at most 400 samples in a window
     double cr0, cr1, cr2, geo_w, geo_tol, dmin, dmax, dd_scale, nn_scale;
     const float* ref;
     const float* ray;
@@ -620,16 +623,17 @@ __global__ void __launch_bounds__(128, PM_MIN_BLOCKS) pm_kernel(const __grid_con
     }
     {
         // the window clipped to the image, its corner rays and its reference sums
-        const int r = c.r, st = c.step, m = 2 * r / st;
-        px.a0 = y - r < 0 ? -r + (r - y + st - 1) / st * st : -r;
-        px.b0 = x - r < 0 ? -r + (r - x + st - 1) / st * st : -r;
-        px.a1 = min(-r + m * st, c.H - 1 - y);
-        px.b1 = min(-r + m * st, c.W - 1 - x);
+        // (the first offset inside the image lies within a step of it; its parts may pass 2^31)
+        const int r = c.r, st = c.step;
+        px.a0 = y < r ? (int)(((unsigned)(r - y - 1) / st + 1u) * st - r) : -r;
+        px.b0 = x < r ? (int)(((unsigned)(r - x - 1) / st + 1u) * st - r) : -r;
+        px.a1 = min(c.last, c.H - 1 - y);
+        px.b1 = min(c.last, c.W - 1 - x);
         const float rx = __ldg(c.ray + idx), ry = __ldg(c.ray + HW + idx), rz = __ldg(c.ray + 2 * HW + idx);
         px.rpx = rx; px.rpy = ry; px.rpz = rz;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int yy = k < 2 ? max(y - r, 0) : min(y + r, c.H - 1), xx = (k & 1) ? min(x + r, c.W - 1) : max(x - r, 0);
+            const int yy = k < 2 ? max(y - r, 0) : y + min(r, c.H - 1 - y), xx = (k & 1) ? x + min(r, c.W - 1 - x) : max(x - r, 0);
             const long long q = (long long)yy * c.W + xx;
             cor[3 * k][px.slot] = __ldg(c.ray + q) - rx;
             cor[3 * k + 1][px.slot] = __ldg(c.ray + HW + q) - ry;
@@ -648,8 +652,8 @@ __global__ void __launch_bounds__(128, PM_MIN_BLOCKS) pm_kernel(const __grid_con
             }
         // piecewise linear interpolation between points 2 r apart is off by at most r^2 / 2 second
         // differences per direction
-        px.dev = (float)(r * r) * __uint_as_float(c.stats->ray_bend);
-        px.prune = __uint_as_float(c.stats->max_abs) <= 6.f && (m + 1) * (m + 1) <= 400;
+        px.dev = c.r2 * __uint_as_float(c.stats->ray_bend);
+        px.prune = __uint_as_float(c.stats->max_abs) <= 6.f && c.few;
     }
     auto cost = [&](double d, const double* nb, double bound, double& ph) { return pm_cost(c, px, cor, d, nb, bound, ph); };
     const double inf = __longlong_as_double(0x7ff0000000000000LL);
@@ -1402,7 +1406,7 @@ struct PMLaneWin<0> {
     using Acc = PMWinStaged;
 };
 // float4 entries of one pixel's staged window (nside: the compile-time side or 0; nw: its samples)
-__host__ __device__ constexpr int pm_lane_entries(int nside, int nw) {
+__host__ __device__ constexpr size_t pm_lane_entries(int nside, size_t nw) {
     return nside > 0 ? 2 * ((nside * nside + 1) / 2) + 5 : nw + 4;
 }
 
@@ -1439,7 +1443,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
     const int side = NSIDE > 0 ? NSIDE : pm_side(c.r, c.step);
     const int nw = side * side;
     using Acc = typename PMLaneWin<NSIDE>::Acc;
-    const int entries = pm_lane_entries(NSIDE, nw);
+    const int entries = (int)pm_lane_entries(NSIDE, nw);
     float4* win = pm_win + (threadIdx.x / L) * entries;
     MVS_BOUND((threadIdx.x / L + 1) * entries * sizeof(float4) <= c.win_smem);
     const float rpx = __ldg(c.ray + idx), rpy = __ldg(c.ray + HW + idx), rpz = __ldg(c.ray + 2 * HW + idx);
@@ -1662,7 +1666,7 @@ constexpr int PM_TRIAL_WARPS = 4;   // warps per block
 #endif
 
 __host__ __device__ inline int pm_tile_pitch(int r) { return 64 + 2 * r; }
-__host__ __device__ inline size_t pm_tile_entries(int r) { return (size_t)(2 * r + 1) * pm_tile_pitch(r); }
+__host__ __device__ inline size_t pm_tile_entries(int r) { return (2 * (size_t)r + 1) * (64 + 2 * (size_t)r); }
 
 // Sums over the window's samples e = 0 .. nw - 1 as an L-lane group forms them: lane l adds
 // e = l, l + L, ... in order, then the xor butterfly (every lane ends with the same value).
@@ -1846,6 +1850,9 @@ namespace {
 
 size_t pm_align(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// The last of a window's offsets -r, -r + step, ... <= r.
+long long pm_last(int r, int step) { return -(long long)r + 2LL * r / step * step; }
+
 // MVS_OK and *work = false: nothing to do.
 mvs_status check_pm(const mvs_pm_args* a, bool* work) {
     *work = false;
@@ -1858,6 +1865,9 @@ mvs_status check_pm(const mvs_pm_args* a, bool* work) {
     if (a->H == 0 || a->W == 0 || a->iters <= 0) return MVS_OK;
     if (!a->ref || !a->ray || !a->Cr || !a->par || !a->depth || !a->normal || !a->score || !a->active)
         return fail(MVS_ERR_VALUE, "pm_refine: null pointer");
+    // the step past the window's last offset is formed as an int
+    if (pm_last(a->r, a->step) + a->step >= (1LL << 31))
+        return fail(MVS_ERR_VALUE, "pm_refine: a window of radius %d at step %d is too large", a->r, a->step);
     if ((long long)a->H * ((a->W + 1) / 2) >= (1LL << 31))
         return fail(MVS_ERR_VALUE, "pm_refine: image of %d x %d pixels is too large", a->W, a->H);
     for (int s = 0; s < a->S; ++s) {
@@ -1884,8 +1894,9 @@ struct PMLayout {
 
 PMLayout pm_layout(const mvs_pm_args* a) {
     PMLayout l;
-    // float32 evaluation needs pinhole sources (the local map is a homography)
-    l.fast = a->precision == MVS_PM_FP32;
+    // float32 evaluation needs pinhole sources (the local map is a homography) and window positions
+    // that are ints (the float64 kernel takes any)
+    l.fast = a->precision == MVS_PM_FP32 && std::max(a->H, a->W) + 2LL * a->r + 64 < (1LL << 31);
     for (int s = 0; s < a->S && l.fast; ++s) {
         const double* q = a->par + 18 * s;
         l.fast = q[13] == 0.0 && q[14] == 0.0 && q[15] == 0.0;
@@ -1943,6 +1954,9 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
     PMParams p;
     memset(&p, 0, sizeof(p));
     p.H = a->H; p.W = a->W; p.S = a->S; p.r = a->r; p.step = a->step; p.top_k = a->top_k;
+    p.last = (int)pm_last(a->r, a->step);
+    p.r2 = (float)a->r * (float)a->r;
+    p.few = 2LL * a->r / a->step + 1 <= 20;
     p.cr0 = a->Cr[0]; p.cr1 = a->Cr[1]; p.cr2 = a->Cr[2];
     p.geo_w = a->geo_w; p.geo_tol = a->geo_tol; p.dmin = a->dmin; p.dmax = a->dmax;
     p.ref = a->ref; p.ray = a->ray; p.depth = a->depth; p.normal = a->normal; p.score = a->score;
@@ -2023,8 +2037,8 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
     const PMJump& J = stream_tables().J;
     // float32 lanes: one per source; a block holds as many pixel groups as its staged windows fit
     const int lanes = a->S <= 4 ? 4 : (a->S <= 8 ? 8 : 16);
-    const int side = pm_side(a->r, a->step);
-    const size_t win_bytes = (size_t)pm_lane_entries(side == 7 || side == 5 ? side : 0, side * side) * sizeof(float4);
+    const int side = fast ? pm_side(a->r, a->step) : 0;
+    const size_t win_bytes = pm_lane_entries(side == 7 || side == 5 ? side : 0, (size_t)side * side) * sizeof(float4);
     int groups = 256 / lanes;
     while (groups > 1 && (size_t)groups * win_bytes > 96 * 1024) groups >>= 1;
     const int block = fast ? groups * lanes : 128;

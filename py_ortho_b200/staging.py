@@ -30,9 +30,18 @@ def _plain() -> bool:
     return torch.cuda.is_current_stream_capturing()
 
 
+class _Readable:
+    """An array's memory as torch.from_numpy takes it without a warning when the array is read-only."""
+
+    def __init__(self, a: np.ndarray):
+        self.array = a
+        self.__array_interface__ = {**a.__array_interface__, "data": (a.__array_interface__["data"][0], False)}
+
+
 def to_device(a: np.ndarray, device) -> torch.Tensor:
-    """torch.from_numpy(a).to(device) for a C-contiguous array."""
-    src = torch.from_numpy(a)
+    """torch.from_numpy(a).to(device) for a C-contiguous array, which is only read (a decoded image or a
+    mapped file may be read-only)."""
+    src = torch.from_numpy(a if a.flags.writeable else np.asarray(_Readable(a)))
     if a.nbytes < LARGE or _plain():
         return src.to(device)
     out = torch.empty(src.shape, dtype=src.dtype, device=device)

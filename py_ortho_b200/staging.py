@@ -25,6 +25,14 @@ class _Ring:
         self.done = [torch.cuda.Event() for _ in range(2)]
 
 
+def _ring(dtype: torch.dtype):
+    """A _Ring, or None where no memory can be pinned (a limit on locked pages): then the plain copy."""
+    try:
+        return _Ring(dtype)
+    except RuntimeError:
+        return None
+
+
 def _plain() -> bool:
     """Staging waits for its own copies: not possible while the stream is being captured."""
     return torch.cuda.is_current_stream_capturing()
@@ -44,9 +52,12 @@ def to_device(a: np.ndarray, device) -> torch.Tensor:
     src = torch.from_numpy(a if a.flags.writeable else np.asarray(_Readable(a)))
     if a.nbytes < LARGE or _plain():
         return src.to(device)
+    ring = _ring(src.dtype)
+    if ring is None:
+        return src.to(device)
     out = torch.empty(src.shape, dtype=src.dtype, device=device)
     with torch.cuda.device(out.device):
-        flat, dst, ring = src.reshape(-1), out.view(-1), _Ring(src.dtype)
+        flat, dst = src.reshape(-1), out.view(-1)
         for k, o in enumerate(range(0, flat.numel(), ring.n)):
             m, b = min(ring.n, flat.numel() - o), k & 1
             if k >= 2:
@@ -63,9 +74,12 @@ def to_host(t: torch.Tensor) -> np.ndarray:
     """t.cpu().numpy(): waits for the work before it on the current stream, as .cpu() does."""
     if t.device.type != "cuda" or not t.is_contiguous() or t.numel() * t.element_size() < LARGE:
         return t.cpu().numpy()
+    ring = _ring(t.dtype)
+    if ring is None:
+        return t.cpu().numpy()
     out = torch.empty(t.shape, dtype=t.dtype)
     with torch.cuda.device(t.device):
-        src, dst, ring = t.view(-1), out.view(-1), _Ring(t.dtype)
+        src, dst = t.view(-1), out.view(-1)
         pieces = [(o, min(ring.n, src.numel() - o)) for o in range(0, src.numel(), ring.n)]
 
         def fetch(k):

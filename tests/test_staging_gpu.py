@@ -36,3 +36,19 @@ def test_read_only_arrays_are_copied_without_a_warning(n, kind, always_warn, tmp
     t += 1
     assert np.array_equal(u.cpu().numpy()[0], want) and np.array_equal(a, want)
     assert np.array_equal((t - u[0]).cpu().numpy(), (want + np.float32(1)) - want)
+
+
+def test_without_pinned_memory_the_plain_copy_runs(monkeypatch):
+    from py_ortho_b200 import staging
+    a = np.random.default_rng(0).normal(0, 1, 5_000_001).astype(np.float32)
+    empty, refused = torch.empty, []
+
+    def pageable(*args, **kw):
+        if kw.get("pin_memory"):
+            refused.append(1)
+            raise RuntimeError("CUDA error: out of memory")
+        return empty(*args, **kw)
+    monkeypatch.setattr(torch, "empty", pageable)
+    t = staging.to_device(a, DEV)
+    back = staging.to_host(t)
+    assert len(refused) == 2 and np.array_equal(back, a)

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cudaTypedefs.h>
 #include <mutex>
+#include <utility>
 
 namespace mvs {
 
@@ -268,14 +269,22 @@ int pick_kmax(SweepParams& p) {
     return 8;
 }
 
-// CTAs of a tile shape that fit on one SM together: the kernels' launch bounds, and the shared
-// memory of Geom<r, th> (228 KB per SM, 1 KB of it reserved per CTA).
-static int resident_ctas(int r, int th, int kk) {
-    const size_t JP = TW + 2 * ((r + 3) & ~3) + 4, HR = th + 2 * r;
-    const size_t smem = HR * JP * 8 + HR * TW * 16 + (size_t)(th == TH_DEFAULT && kk <= 2 && (r == 4 || r == 5) ? 5 : 6) * th * TW * 4 +
-                        sizeof(Coef) * MVS_MAX_SOURCES + 1024;
-    const int fit = (int)((size_t)228 * 1024 / smem), bound = th == 16 ? 3 : (th == 32 ? 2 : 1);
+// CTAs of a tile shape that fit on one SM together: the kernels' launch bounds and their shared
+// memory (228 KB per SM, 1 KB of it reserved per CTA), for lists of kk = min(top_k, sources) entries.
+template <int TH, int KMAX, int... R>
+static size_t tile_smem(int r, std::integer_sequence<int, R...>) {
+    static constexpr size_t bytes[] = {Geom<R, TH>::smem_bytes(WinnerState<R, KMAX, TH>::PLANES)...};
+    return bytes[r];
+}
+template <int TH>
+static int resident_ctas(int r, int kk) {
+    const auto radii = std::make_integer_sequence<int, MVS_MAX_RADIUS + 1>{};
+    const size_t smem = (kk <= 2 ? tile_smem<TH, 2>(r, radii) : tile_smem<TH, 8>(r, radii)) + 1024;
+    const int fit = (int)((size_t)228 * 1024 / smem), bound = TileShape<TH>::MIN_CTAS;
     return fit < 1 ? 1 : (fit < bound ? fit : bound);
+}
+static int resident_ctas(int r, int th, int kk) {
+    return th == 16 ? resident_ctas<16>(r, kk) : th == 64 ? resident_ctas<64>(r, kk) : resident_ctas<TH_DEFAULT>(r, kk);
 }
 
 // Plane chunks of a launch: `tiles` x chunks CTAs of about equal work run `slots` at a time, so the
@@ -341,8 +350,9 @@ size_t sweep_scratch_bytes(const mvs_sweep_args* a, int* nchunks_out) {
     const int tiles = ((a->W + TW - 1) / TW) * ((a->H + th - 1) / th);
     const int nplanes = a->i1 - a->i0;
     const int per_call = nplanes < MVS_MAX_PLANES_PER_CALL ? nplanes : MVS_MAX_PLANES_PER_CALL;
+    const int kk = a->top_k < a->n_src ? a->top_k : a->n_src;
     int nch = a->plane_chunks > 0 ? a->plane_chunks
-                                 : auto_plane_chunks(tiles, per_call, num_sms() * resident_ctas(a->r, th, a->top_k));
+                                 : auto_plane_chunks(tiles, per_call, num_sms() * resident_ctas(a->r, th, kk));
     if (nch > per_call) nch = per_call < 1 ? 1 : per_call;
     *nchunks_out = nch;
     if (nch <= 1) return 0;

@@ -1,8 +1,11 @@
 """The height sweep's entry points at the edges of what they accept."""
 import ctypes
 
+import numpy as np
 import pytest
 import torch
+
+from conftest import same_bits
 
 
 def _eval_args(L, W, r, H=8, D=1):
@@ -50,3 +53,34 @@ def test_refinement_steps_on_the_largest_grids(H, W):
         want = torch.sort(torch.stack([lo, v, hi]), dim=0).values[1]       # three equal rows (columns): the middle of 3
         s = slice(0, 599) if o == 0 else slice(1, 600)
         assert torch.equal(out[o:o + 600][s], want[s])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,r", [(656, 3), (775, 0), (1024, 3), (1025, 3), (1500, 3)])
+def test_the_score_of_a_grid_too_wide_for_the_fused_evaluation(W, r):
+    """The fused call refuses it and writes nothing; its parts give, away from the crop's border, the fused
+    score of the grid's first 600 columns."""
+    from py_ortho_b200 import _lib as L, height as Hs
+    from test_height_routes_gpu import _sweep
+    H, C, V = 20, 600, 3
+    sw = _sweep(V, W, H, Hs.DenseOptions(window=r, min_texture=0.5), 5)
+    sw.t.X0, sw.t.Y0 = -14.0, 7.0                            # the views see the first columns
+    Z = torch.rand((2, H, W), device="cuda") * 6
+    outs = [torch.full((V, 2, H, W), 77, dtype=torch.uint8, device="cuda"), torch.full((2, H, W), 7.5, device="cuda")]
+    a = _eval_args(L, W, r, H, 2)
+    cams, img = np.zeros((2, 18)), sw.views[0].pyr[0]
+    a.cams, a.Z, a.valid, a.score = cams.ctypes.data, Z.data_ptr(), outs[0].data_ptr(), outs[1].data_ptr()
+    a.cxs, a.cys = (t.data_ptr() for t in sw._centres(H, W, 0.7))
+    for k in range(2):
+        a.img[k], a.img_h[k], a.img_w[k] = img.data_ptr(), int(img.shape[0]), int(img.shape[1])
+    ws = torch.empty(1 << 24, dtype=torch.uint8, device="cuda")
+    assert L.load().mvs_height_eval(ctypes.addressof(a), ws.data_ptr(), ws.numel(), L.stream_handle()) == L.ERR_UNSUPPORTED
+    torch.cuda.synchronize()
+    assert (outs[0] == 77).all() and (outs[1] == 7.5).all()
+    got = sw.score(Z, 0, 0.7, detail=True)
+    crop = _eval_args(L, C, r, H, 2)
+    assert L.load().mvs_height_eval_scratch_bytes(ctypes.addressof(crop)) > 0
+    want = sw.score(Z[:, :, :C].contiguous(), 0, 0.7, detail=True)
+    assert 0 < int(got[2].sum()) < got[2].numel() and (r == 0 or got[0].std() > 0)
+    for x, y in zip(got, want):
+        assert same_bits(x[..., :C - r].cpu().numpy(), y[..., :C - r].cpu().numpy())

@@ -246,8 +246,10 @@ mvs_status mvs_to_fp16(int64_t n, const float* in, void* out_half, void* stream)
 
 /* Arithmetic of the PatchMatch cost. */
 typedef enum mvs_pm_precision {
-    MVS_PM_FP64 = 0,     /* the reference's float64 cost, operation for operation: bit-identical
-                            results to a sequential evaluation with the same draws               */
+    MVS_PM_FP64 = 0,     /* the reference's float64 cost: every sum, product and comparison with its
+                            rounding, without the windows that cannot matter; quotients are
+                            correctly rounded unless one lies within 2^-50 ulp of the middle
+                            between two doubles. Bit-identical on every input tested             */
     MVS_PM_FP32 = 1      /* window samples and sums in float32, one float64-composed local
                             homography per candidate and source (pinhole sources; otherwise as
                             MVS_PM_FP64); the lanes of a pixel group evaluate its sources in
@@ -293,10 +295,12 @@ typedef struct mvs_pm_args {
  * finite after propagation takes 8 draws in raster order, colour pass after colour pass. Each
  * pass runs propagation for all its pixels in parallel, counts the drawing pixels (a prefix sum
  * in raster order) and jumps the stream to each pixel's offset (GF(2) matrix powers), then runs
- * the trials in parallel. With MVS_PM_FP64 the result is bit-identical to the reference's.
- * Scratch (about 21 bytes per pixel, 26 with MVS_PM_FP64, plus 16 per pixel when iters > 1, plus 16 per source pixel
- * with MVS_PM_FP32: each source's 2 x 2 bilinear footprints, one 16-byte load per sample) is
- * allocated stream-ordered per call. */
+ * the trials in parallel. With MVS_PM_FP64 the result is the reference's bits but for its
+ * quotients' exception (mvs_pm_precision). A window whose next step past its last offset is no
+ * int32 is refused; with MVS_PM_FP32, positions that are none run as MVS_PM_FP64.
+ * Scratch is allocated stream-ordered per call: 10.5 bytes per pixel with MVS_PM_FP32, 15 with
+ * MVS_PM_FP64, plus 16 per pixel when iters > 1, plus 16 per source pixel with MVS_PM_FP32 (each
+ * source's 2 x 2 bilinear footprints, one 16-byte load per sample). */
 mvs_status mvs_pm_refine(const mvs_pm_args* args, void* stream);
 
 /* mvs_pm_refine with its scratch given by the caller (256-byte aligned device memory, free to be used
@@ -552,6 +556,11 @@ uint32_t mvs_set_wait_limit(uint32_t iterations);
  * builds return MVS_ERR_UNSUPPORTED. No counterpart in the reference (its Cython kernels are
  * compiled with boundscheck=False). */
 mvs_status mvs_debug_bound_violations(uint32_t* count);
+
+/* quot[i] = a[i] / b[i] and rcp[i] = 1 / b[i] as the float64 PatchMatch and the per-pixel sweep
+ * form them on the device (tests compare them with the division; device pointers). */
+mvs_status mvs_debug_quotients(int64_t n, const double* a, const double* b, double* quot, double* rcp,
+                               void* stream);
 
 /* Message of this thread's last failing call ("" if none). Returns the message length. */
 size_t mvs_last_error(char* buf, size_t cap);

@@ -168,6 +168,7 @@ SIGNATURES = {
     "mvs_device_faults": (i32, [vp]),
     "mvs_set_wait_limit": (C.c_uint32, [C.c_uint32]),
     "mvs_debug_bound_violations": (i32, [vp]),
+    "mvs_debug_quotients": (i32, [i64, vp, vp, vp, vp, vp]),
     "mvs_version": (C.c_char_p, []),
 }
 

@@ -2,7 +2,8 @@
 //
 // This file is compiled with -fmad=false: every float64 expression below is evaluated with one
 // rounding per operation in the written order, which is how the reference's C (x86-64, no FMA)
-// evaluates it. The float64 mode is bit-identical to the reference's pm_refine.
+// evaluates it. The float64 mode gives the bits of the reference's pm_refine on every input tested (its
+// quotients have an exception, see pm_quot).
 //
 // Parallel schedule. The reference visits the pixels of one colour ((x + y) % 2) in raster order,
 // but every pixel reads only its own plane, pixels of the other colour (all 8 neighbour offsets,
@@ -138,9 +139,10 @@ __device__ __forceinline__ double pm_bil(const float* im, int w, int h, double u
 
 // ---------------------------------------------------------------- float64 evaluation (MVS_PM_FP64)
 //
-// _pm_cost (_dense.pyx:461-556), every value with the reference's bits. What bounds it is the float64
-// pipe (64 lanes a clock per SM), so the work that provably does not reach a result is left out and
-// what is shared is formed once:
+// _pm_cost (_dense.pyx:461-556): every sum, product and comparison that reaches a result is the
+// reference's, with its rounding; quotients have pm_quot's exception. What bounds it is the float64 pipe
+// (64 lanes a clock per SM), so the work that provably does not reach a result is left out and what is
+// shared is formed once:
 //   * the geometric term comes first: a candidate whose geometric term alone reaches the pixel's
 //     best cost cannot be accepted (the photo term is at least 1 - NCC, see PM_PRUNE), so its windows
 //     are not evaluated;
@@ -196,19 +198,11 @@ __global__ void __launch_bounds__(256) pm_bend_kernel(const float* __restrict__ 
     if ((threadIdx.x & 31) == 0) atomicMax(&st->ray_bend, __float_as_uint(m));
 }
 
-// 1 / z by two Newton-Raphson steps on the hardware's approximation, to the last bit or so.
-__device__ __forceinline__ double pm_rcp(double z) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));
-    double e = __fma_rn(-z, r, 1.0);
-    r = __fma_rn(r, e, r);
-    e = __fma_rn(-z, r, 1.0);
-    return __fma_rn(r, e, r);
-}
-
 // a / b from r ~ 1 / b: Markstein's correction (IBM J. Res. Dev. 34, 1990) - the remainder a - q b is
-// exact in one fused operation, so the result is the correctly rounded quotient except where a / b
-// lies within ~2^-50 ulp of the middle between two doubles. Several numerators share one reciprocal.
+// exact in one fused operation. With r within 2^-52 of 1 / b and q within 1.5 x 2^-52 of a / b, both
+// relative, q + (a - q b) r is off by 1.5 x 2^-104 before its one rounding, 1.5 x 2^-51 ulp: the result is
+// the correctly rounded quotient unless a / b lies within 2^-50 ulp of the middle between two doubles
+// (and is then one of the two). Several numerators share one reciprocal.
 __device__ __forceinline__ double pm_quot(double a, double b, double r) {
     const double q = __dmul_rn(a, r);
     return __fma_rn(__fma_rn(-q, b, a), r, q);
@@ -279,7 +273,7 @@ __device__ __forceinline__ void pm_sums64(const PMParams& c, const PMPix& px, co
             const double qx = __ldg(c.ray + q), qy = __ldg(c.ray + HW + q), qz = __ldg(c.ray + 2 * HW + q);
             const double den = n[0] * qx + n[1] * qy + n[2] * qz;
             if (CHECKED && den >= -1e-9) continue;
-            const double t = pm_quot(num, den, pm_rcp(den));
+            const double t = pm_quot(num, den, rcp_newton(den));
             const double X = c.cr0 + t * qx, Y = c.cr1 + t * qy, Z = c.cr2 + t * qz;
             ++ns;
             const double II = I * I;
@@ -294,7 +288,7 @@ __device__ __forceinline__ void pm_sums64(const PMParams& c, const PMPix& px, co
                 const double zc = p[6] * dx + p[7] * dy + p[8] * dz;
                 const bool front = !CHECKED || zc > 1e-6;
                 const double zq = front ? zc : 1.0;
-                const double rz = pm_rcp(zq);
+                const double rz = rcp_newton(zq);
                 const double nx = pm_quot(xc, zq, rz), ny = pm_quot(yc, zq, rz);
                 // pinhole source: the reference's factor f (1 + r2 (k1 + r2 (k2 + r2 k3)))
                 // evaluates to exactly f (r2 >= 0 finite, so every product with 0 is +0)
@@ -460,7 +454,7 @@ __device__ double pm_cost(const PMParams& c, const PMPix& px, const PMCorners& c
     }
     const double gterm = c.geo_w * pm_geo(c, d, px.rpx, px.rpy, px.rpz);
     // PM_PRUNE: the NCC of values up to 6 in magnitude exceeds 1 by less than 1e-3 through rounding
-    // (window sums of < 1000 samples carry < 1e-12; the variances are at least 1e-8), so the cost
+    // (window sums of at most 400 samples carry < 1e-12; the variances are at least 1e-8), so the cost
     // is at least gterm - 1e-3
     if (px.prune && gterm - 1e-3 >= best) {
         ncc_out = 0.0;
@@ -2125,6 +2119,26 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
             status = fail(MVS_ERR_CUDA, "pm_refine: stream state copy");
     }
     return status;
+}
+
+namespace mvs {
+__global__ void quotients_kernel(long long n, const double* a, const double* b, double* quot, double* rcp) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const double r = rcp_newton(b[i]);
+    rcp[i] = r;
+    quot[i] = pm_quot(a[i], b[i], r);
+}
+}  // namespace mvs
+
+extern "C" mvs_status mvs_debug_quotients(int64_t n, const double* a, const double* b, double* quot, double* rcp,
+                                          void* stream) {
+    clear_error();
+    if (n < 0) return fail(MVS_ERR_VALUE, "quotients: negative size");
+    if (n == 0) return MVS_OK;
+    if (!a || !b || !quot || !rcp) return fail(MVS_ERR_VALUE, "quotients: null pointer");
+    quotients_kernel<<<(unsigned)((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(n, a, b, quot, rcp);
+    return check_launch("quotients");
 }
 
 unsigned mvs::take_bound_violations_pm() { return take_bound_violations_here(); }

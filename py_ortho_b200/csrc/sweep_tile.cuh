@@ -298,17 +298,6 @@ __device__ __forceinline__ float2 sample_plane_inside2(const Coef& c, const void
 // inverse depth and the result), so the integer tap position comes from an addition rounded toward
 // -inf instead of two conversions, and the bounds are compared as integers.
 
-// 1 / z by two Newton-Raphson steps on the hardware's approximation (relative error ~2^-20 ->
-// 2^-40 -> the last bit or so). 0, inf and NaN give NaN.
-__device__ __forceinline__ double rcp_newton(double z) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(z));
-    double e = __fma_rn(-z, r, 1.0);
-    r = __fma_rn(r, e, r);
-    e = __fma_rn(-z, r, 1.0);
-    return __fma_rn(r, e, r);
-}
-
 // The source position of one sample: offset of the top-left tap (0 when invalid) and the fractions.
 struct RayTap {
     double fx, fy;

@@ -241,8 +241,9 @@ def pm_refine(ref, ray, Cr, srcs: Sequence, src_depths: Sequence, par, depth, no
     updated in place; returns the number of accepted hypothesis changes. The random trials draw
     from the reference's own xorshift32 stream (started at seed | 1), in its raster order.
 
-    precision: "fp64" evaluates the reference's float64 cost operation for operation (bit-identical
-    to the reference's pm_refine); "fp32" evaluates the windows in float32 from one
+    precision: "fp64" evaluates the reference's float64 cost (bit-identical to the reference's
+    pm_refine on every input tested; quotients within 2^-50 ulp of the middle between two doubles may
+    round the other way); "fp32" evaluates the windows in float32 from one
     float64-composed homography per candidate and source (costs within ~1e-6 of float64; near-ties
     may be decided differently).
 

@@ -155,9 +155,7 @@ __device__ __forceinline__ double pm_bil(const float* im, int w, int h, double u
 // Each of a source's sums still accumulates in window order.
 
 // Sources per pass over the window (PM_MIN_BLOCKS has the measurements).
-#ifndef PM_PASS
-#define PM_PASS 2
-#endif
+constexpr int PM_PASS = 2;
 
 // What mvs_pm_refine's preparation finds out about its inputs (float bit patterns, all >= 0).
 struct PMStats {
@@ -483,11 +481,6 @@ __device__ double pm_cost(const PMParams& c, const PMPix& px, const PMCorners& c
                 group |= list & (0u - list);
                 list &= list - 1;
             }
-#if PM_PASS >= 4
-            if (m == 4) pm_batch64<4>(c, px, group, checked, in, out, num, n, ncc);
-            else if (m == 3) pm_batch64<3>(c, px, group, checked, in, out, num, n, ncc);
-            else
-#endif
             if (m == 2) pm_batch64<2>(c, px, group, checked, in, out, num, n, ncc);
             else pm_batch64<1>(c, px, group, checked, in, out, num, n, ncc);
         }
@@ -515,9 +508,8 @@ __device__ double pm_cost(const PMParams& c, const PMPix& px, const PMCorners& c
 // pass with 5 blocks (96 registers) 8.0 / 24.7, 6 blocks 8.3 / 26.1, 8 blocks 7.7 / 27.2; 4 sources a
 // pass with 5 blocks 11.5 / 37.7 (spills), 4 blocks 12.5 / 38.7. One thread per pixel, all windows
 // and tests, three divisions a sample: 36.0 / 54.2.
-#ifndef PM_MIN_BLOCKS
-#define PM_MIN_BLOCKS 5
-#endif
+constexpr int PM_MIN_BLOCKS = 5;
+
 // Pixel of pass number t (raster order of the colour's pixels): false past the image.
 __device__ __forceinline__ bool pm_pixel(const PMParams& c, long long t, int& y, int& x) {
     const int half_w = (c.W + 1) / 2;
@@ -914,15 +906,7 @@ __global__ void __launch_bounds__(256) pm_quad_kernel(const float* __restrict__ 
 // pairs of a row 239 ms at 5, 232 ms at 4 (64 registers), 248 ms at 3, in pairs of the whole window and
 // with a shorter unit set-up 217 ms at 4. What bounds it is latency at that occupancy: issue slots alone
 // would take ~100 ms, the footprints' L1 wavefronts ~50 ms.
-#ifndef PM_LANE_MIN_BLOCKS
-#define PM_LANE_MIN_BLOCKS 4
-#endif
-#ifndef PM_LANE_MIN_BLOCKS_TRIALS
-#define PM_LANE_MIN_BLOCKS_TRIALS PM_LANE_MIN_BLOCKS
-#endif
-#ifndef PM_UNIT_INLINE
-#define PM_UNIT_INLINE __forceinline__
-#endif
+constexpr int PM_LANE_MIN_BLOCKS = 4;
 
 __device__ __forceinline__ int pmf_floor(float x, float& f) {   // |x| < 2^22
     const float t = __fadd_rd(x, 12582912.0f);
@@ -977,15 +961,11 @@ struct PMWinStaged {
     const float4* w;      // NW samples, then the 4 corners
     __device__ __forceinline__ float4 at(int, int, int e) const { return w[e]; }
     __device__ __forceinline__ float4 corner(int k4, int nw) const { return w[nw + k4]; }
-    __device__ __forceinline__ void pair(int, int, float2&, float2&, float2&, float2&) const {}
 };
 template <int NSIDE>
 struct PMWinPairs {
     static constexpr bool PAIRS = true, FLAT = true;
     static constexpr int NW = NSIDE * NSIDE, NP = (NW + 1) / 2;   // samples, pairs
-    // float4 entries per pixel: the pairs, the 4 corners, one more (an odd number of 16-byte units
-    // puts the 4 pixels of a warp on different banks)
-    static constexpr int ENTRIES = 2 * NP + 4 + 1;
     const float4* w;
     static __device__ __forceinline__ int slot(int e) { return (e >> 1) * 8 + (e & 1); }
     __device__ __forceinline__ float4 at(int, int, int e) const {
@@ -1161,7 +1141,7 @@ __device__ __forceinline__ void pm_window_sums(const Acc& win, int side_rt, cons
 // (s < S); n . ray_p = ndr < -1e-6. Follows _pm_cost: -1 below the count gate, 0 below the
 // variance floor.
 template <int NSIDE, class Acc>
-__device__ PM_UNIT_INLINE float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>& wn, float rpx, float rpy, float rpz,
+__device__ __forceinline__ float pm_unit_ncc(const PMParams& c, const PMWinT<Acc>& wn, float rpx, float rpy, float rpz,
                                             double d, const double* n, double ndr, int sl) {
     const double num = d * ndr;
     const float n0 = (float)n[0], n1 = (float)n[1], n2 = (float)n[2], denp = (float)ndr;
@@ -1399,14 +1379,16 @@ template <>
 struct PMLaneWin<0> {
     using Acc = PMWinStaged;
 };
-// float4 entries of one pixel's staged window (nside: the compile-time side or 0; nw: its samples)
+// float4 entries of one pixel's staged window (nside: the compile-time side or 0; nw: its samples).
+// Pairs: two entries each, the 4 corners and one more - an odd number of 16-byte units puts the
+// pixels of a warp on different banks.
 __host__ __device__ constexpr size_t pm_lane_entries(int nside, size_t nw) {
     return nside > 0 ? 2 * ((nside * nside + 1) / 2) + 5 : nw + 4;
 }
 
 // PHASE 0: current plane and propagation; PHASE 1: the random trials.
 template <int L, int NSIDE, int PHASE>
-__global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE_MIN_BLOCKS_TRIALS)
+__global__ void __launch_bounds__(256, PM_LANE_MIN_BLOCKS)
     pm_lane_kernel(const __grid_constant__ PMParams c) {
     extern __shared__ float4 pm_win[];
     const int H = c.H, W = c.W;
@@ -1652,12 +1634,7 @@ __global__ void __launch_bounds__(256, PHASE == 0 ? PM_LANE_MIN_BLOCKS : PM_LANE
 // 16-byte entries (half of its wavefronts bank conflicts) 88.0 ms at 4 blocks per SM; pairs from
 // planes 84.3 ms at 3 (168 registers; 82.7 with the shorter unit set-up), 89.7 ms at 4 (128, spills).
 constexpr int PM_TRIAL_WARPS = 4;   // warps per block
-#ifndef PM_TRIAL_MIN_BLOCKS
-#define PM_TRIAL_MIN_BLOCKS 3
-#endif
-#ifndef PM_TRIAL_LANE_GROUPS
-#define PM_TRIAL_LANE_GROUPS 0      // 1: the trials on the lane groups' kernel (comparisons)
-#endif
+constexpr int PM_TRIAL_MIN_BLOCKS = 3;
 
 __host__ __device__ inline int pm_tile_pitch(int r) { return 64 + 2 * r; }
 __host__ __device__ inline size_t pm_tile_entries(int r) { return (2 * (size_t)r + 1) * (64 + 2 * (size_t)r); }
@@ -2005,7 +1982,7 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
             p.quad[s] = q;
             off += pm_align((size_t)a->src_w[s] * a->src_h[s] * sizeof(float4));
             const long long ns = (long long)a->src_w[s] * a->src_h[s];
-            const int qb = (int)std::min<long long>((ns + 255) / 256, 148LL * 8);
+            const int qb = (int)std::min<long long>((ns + 255) / 256, num_sms() * 8LL);
             pm_quad_kernel<<<qb, 256, 0, st>>>(a->src[s], a->src_w[s], a->src_h[s], q);
         }
     }
@@ -2016,7 +1993,7 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
         PMStats* stats = reinterpret_cast<PMStats*>(rng + 8);
         cudaMemsetAsync(stats, 0, sizeof(PMStats), st);
         p.stats = stats;
-        const unsigned sb = 148 * 8;
+        const unsigned sb = num_sms() * 8;
         pm_bend_kernel<<<sb, 256, 0, st>>>(a->ray, a->H, a->W, stats);
         pm_stats_kernel<<<sb, 256, 0, st>>>(a->ref, HW, stats);
         for (int s = 0; s < a->S; ++s)
@@ -2057,7 +2034,6 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
     const size_t smem_trial = (size_t)PM_TRIAL_WARPS * pm_tile_entries(a->r) * sizeof(float4);
     const int wpr = (int)(((a->W + 1) / 2 + 31) / 32);
     const unsigned grid_trial = (unsigned)(((long long)a->H * wpr + PM_TRIAL_WARPS - 1) / PM_TRIAL_WARPS);
-#if !PM_TRIAL_LANE_GROUPS
     if (fast && status == MVS_OK && smem_trial <= MVS_SMEM_MAX) {
 #define PM_PICK_TRIAL(LN)                                                                        \
     trial_kernel = side == 7 && a->step == 1   ? pm_trial_kernel<LN, 7, true>                       \
@@ -2075,7 +2051,6 @@ extern "C" mvs_status mvs_pm_refine_ws(const mvs_pm_args* a, void* scratch_mem, 
             trial_kernel = nullptr;
         }
     }
-#endif
     const unsigned grid = fast ? (unsigned)((n * lanes + block - 1) / block) : (unsigned)((n + 127) / 128);
     if (status == MVS_OK) {
         pm_rng_init_kernel<<<1, 1, 0, st>>>(rng, a->rng_state, a->seed | 1u);

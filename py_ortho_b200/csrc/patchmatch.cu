@@ -243,6 +243,7 @@ struct PMPix {
     int nfin;
     int slot;                      // the pixel's place in the block (PMCorners)
     float dev;                     // bound of a ray's distance from the corners' bilinear interpolation
+    float wmax;                    // largest component of the corner offsets
     bool prune;
 };
 
@@ -339,13 +340,16 @@ __device__ __forceinline__ void pm_sums64(const PMParams& c, const PMPix& px, co
 // front, and counted), -1 every sample outside, 0 neither shown. The window's rays are within `dev` of
 // the bilinear interpolation of its corner rays and the plane's map is projective, so undistorted
 // image points lie in the box of the corners' points, widened by the effect of `dev` and of float32
-// rounding; a distorted source's factor 1 + r2 (..) is bounded by its terms' absolute values.
+// rounding; a distorted source's factor 1 + r2 (..) is bounded by its terms' absolute values. The bounds
+// hold for normals of any length and windows of any size: rounding is in proportion to the map's
+// coefficients times the offsets, not to the corners' sums, which cancel where a plane is seen edge-on.
 __device__ __forceinline__ int pm_where(const PMParams& c, const PMPix& px, const PMCorners& cor, int s, float num,
                                         float n0, float n1, float n2, float ndr) {
     const float* p = c.parf + 18 * s;
     const float* bs = c.bsf + 3 * s;
     const float rx = (float)px.rpx, ry = (float)px.rpy, rz = (float)px.rpz;
-    float M[3][3], cen[3], big = 0.f;
+    const float nl = fabsf(n0) + fabsf(n1) + fabsf(n2), den_max = -(1e-4f + 4.f * px.dev) * fmaxf(nl, 1.f);
+    float M[3][3], cen[3], bmax = 0.f;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const float b = bs[i], p0 = p[3 * i], p1 = p[3 * i + 1], p2 = p[3 * i + 2];
@@ -353,9 +357,10 @@ __device__ __forceinline__ int pm_where(const PMParams& c, const PMPix& px, cons
         M[i][1] = fmaf(b, n1, num * p1);
         M[i][2] = fmaf(b, n2, num * p2);
         cen[i] = fmaf(b, ndr, num * fmaf(p0, rx, fmaf(p1, ry, p2 * rz)));
-        big = fmaxf(big, fabsf(b * ndr));
+        bmax = fmaxf(bmax, fabsf(b));
     }
-    big += fabsf(num) * (fabsf(rx) + fabsf(ry) + fabsf(rz));
+    const float big = bmax * (fabsf(ndr) + nl * px.wmax) +
+                      fabsf(num) * (fabsf(rx) + fabsf(ry) + fabsf(rz) + 3.f * px.wmax);
     const float zc = cen[2];                              // camera depth is zc / ndr: < 0 in front
     if (!(zc < -1e-20f)) return 0;
     const float iz = __fdividef(1.0f, zc);
@@ -368,7 +373,7 @@ __device__ __forceinline__ int pm_where(const PMParams& c, const PMPix& px, cons
         const float v1 = fmaf(M[1][0], w0, fmaf(M[1][1], w1, fmaf(M[1][2], w2, cen[1])));
         const float v2 = fmaf(M[2][0], w0, fmaf(M[2][1], w1, fmaf(M[2][2], w2, cen[2])));
         const float den = fmaf(n0, w0, fmaf(n1, w1, fmaf(n2, w2, ndr)));
-        good = good && den < -1e-4f - 4.f * px.dev && v2 < 1e-2f * den && v2 < 0.5f * zc;
+        good = good && den < den_max && v2 < 1e-2f * den && v2 < 0.5f * zc;
         const float r = __fdividef(1.0f, v2);
         xlo = fminf(xlo, v0 * r);
         xhi = fmaxf(xhi, v0 * r);
@@ -617,14 +622,18 @@ __global__ void __launch_bounds__(128, PM_MIN_BLOCKS) pm_kernel(const __grid_con
         px.b1 = min(c.last, c.W - 1 - x);
         const float rx = __ldg(c.ray + idx), ry = __ldg(c.ray + HW + idx), rz = __ldg(c.ray + 2 * HW + idx);
         px.rpx = rx; px.rpy = ry; px.rpz = rz;
+        float wmax = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int yy = k < 2 ? max(y - r, 0) : y + min(r, c.H - 1 - y), xx = (k & 1) ? x + min(r, c.W - 1 - x) : max(x - r, 0);
             const long long q = (long long)yy * c.W + xx;
-            cor[3 * k][px.slot] = __ldg(c.ray + q) - rx;
-            cor[3 * k + 1][px.slot] = __ldg(c.ray + HW + q) - ry;
-            cor[3 * k + 2][px.slot] = __ldg(c.ray + 2 * HW + q) - rz;
+            const float w0 = __ldg(c.ray + q) - rx, w1 = __ldg(c.ray + HW + q) - ry, w2 = __ldg(c.ray + 2 * HW + q) - rz;
+            cor[3 * k][px.slot] = w0;
+            cor[3 * k + 1][px.slot] = w1;
+            cor[3 * k + 2][px.slot] = w2;
+            wmax = fmaxf(wmax, fmaxf(fabsf(w0), fmaxf(fabsf(w1), fabsf(w2))));
         }
+        px.wmax = wmax;
         px.si = px.sii = 0.0;
         px.nfin = 0;
         for (int a = px.a0; a <= px.a1; a += st)

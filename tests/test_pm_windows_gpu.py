@@ -60,3 +60,32 @@ def test_windows_that_are_refused(r, step, precision, error):
     from py_ortho_b200 import dense
     with pytest.raises(error):
         _refine(dense.pm_refine, r, step, precision=precision)
+
+
+@pytest.mark.parametrize("r,step,length,bend", [(3, 1, 1.0, 0.0), (3, 1, 1e5, 3e-4), (12, 4, 1e-3, 0.0), (12, 4, 1e3, 3e-4),
+                                               (30, 10, 1e5, 0.0)])
+def test_planes_seen_edge_on_bit_exact_vs_oracle(r, step, length, bend):
+    """Normals of any length, nearly perpendicular to their rays, on straight and on irregular ray grids: the
+    proofs that a window lies inside or outside a source hold where the plane's terms cancel. Every candidate
+    is outside the depth range, so the score map is the current planes' photo term."""
+    from py_ortho_b200 import dense, scene as S
+    W, H = 64, 48
+    sc = S.make_scene("c2", seed=5, width=W, height=H)
+    rng = np.random.default_rng(r + int(np.log10(length)) + int(bend * 1e5))
+    ref = sc.grey(sc.ref).astype(np.float32)
+    srcs = [sc.grey(s).astype(np.float32) for s in sc.srcs[:6]]
+    par = np.array([c.row() for c in sc.src_cams[:6]], np.float64)
+    ray = (O.rays_world((H, W), sc.ref_cam) + rng.normal(0, 1, (3, H, W)) * bend).astype(np.float32)
+    u = ray / np.linalg.norm(ray, axis=0)
+    t = np.cross(u, rng.normal(0, 1, (3, H, W)), axis=0)
+    t /= np.linalg.norm(t, axis=0)
+    eps = 10.0 ** rng.uniform(-5, -1, (H, W))
+    normal = ((t - eps * u) * length).astype(np.float32)
+    depth = (sc.depth_true * (1 + rng.normal(0, 0.01, (H, W)))).astype(np.float32)
+    act = np.ones((H, W), np.uint8)
+    out = []
+    for fn in (dense.pm_refine, O.pm_refine):
+        st = [depth.copy(), normal.copy(), np.zeros((H, W), np.float32)]
+        assert fn(ref, ray, sc.ref_cam.C, srcs, [None] * 6, par, *st, act, r, step, 3, 0.0, 0.02, 1, 1e9, 1e9 + 1, 5) == 0
+        out.append(st[2])
+    assert same_bits(*out)

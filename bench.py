@@ -30,7 +30,12 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 PM_HYPS = 11          # hypotheses per PatchMatch pixel-iteration (1 + 8 propagation + 2 random)
-PM_PROFILE = {"fp32": "profiles/pm_lane_kernel_1000x750_8src.md", "fp64": "profiles/pm_kernel_2000x1500_8src.md"}
+# fraction of the SM issue slots used by each PatchMatch kernel (ncu, one launch each of a colour pass
+# at 1000 x 750, 8 sources, 7 x 7)
+PM_ISSUE_ACTIVE = {"fp32": {"propagation": 0.605, "trials": 0.406},
+                   "fp64": {"current": 0.548, "propagation": 0.632, "trials": 0.473}}
+PM_BOUND = {"fp32": "latency of the footprint loads at 27 (propagation) and 9 (trials) warps per SM",
+            "fp64": "latency of float64 chains at 19 (propagation) and 17 (trials) warps per SM, FP64 pipe 53 % and 40 %"}
 
 
 def parse():
@@ -44,7 +49,7 @@ def parse():
                          "--mode depthmap only)")
     ap.add_argument("--pm-precision", choices=["fp32", "fp64"], default="fp32",
                     help="PatchMatch cost arithmetic: fp32 windows (float64-composed homographies) or the "
-                         "reference's float64 operation order (bit-exact)")
+                         "reference's float64 arithmetic")
     ap.add_argument("--config", default="c2")
     ap.add_argument("--width", type=int, default=0, help="override the image width (smaller test runs)")
     ap.add_argument("--height", type=int, default=0)
@@ -280,7 +285,7 @@ def run_ours(a):
     ms_sweep = acc["sweep"] / a.steps
     ms_pm = acc["pm"] / a.steps if iters else 0.0
     # the other PatchMatch arithmetic, timed once after the timed region on the same state: the
-    # float64 kernel (the reference's arithmetic, bit-exact) when the step ran float32, or vice versa
+    # float64 kernel (the reference's arithmetic) when the step ran float32, or vice versa
     pm_other = None
     if iters and world == 1:
         other = 0 if pm.precision == 1 else 1
@@ -316,7 +321,7 @@ def run_ours(a):
                   "evals_per_s": sweep_evals / (ms_sweep / 1e3), "ms": round(ms_sweep, 3)}
     # the roof that binds this kernel: SIMT issue. 128 FP32 lanes x SMs x the sampled SM clock
     # thread instructions per second, over the instructions per evaluation the committed ncu
-    # capture counts (profiles/sweep_kernel_3000x2250_8src_16planes.md)
+    # capture counts (SWEEP_INST_PER_EVAL)
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
     clk = clocks.summary().get("sm_mhz") or 1965.0
     issue_rate = 128.0 * n_sm * clk * 1e6
@@ -327,15 +332,13 @@ def run_ours(a):
     if iters:
         roof_pm = {"kernel": "pm_lane_kernel + pm_trial_kernel" if a.pm_precision == "fp32" else "pm_kernel",
                    "precision": a.pm_precision,
-                   "bound": "fp32-issue" if a.pm_precision == "fp32" else "fp64-issue",
+                   "bound": PM_BOUND[a.pm_precision],
                    "evals_per_s": pm_evals / (ms_pm / 1e3),
                    "ms": round(ms_pm, 3), "share_of_step": round(ms_pm / (ms_pm + ms_sweep), 4),
-                   "ncu_profile": PM_PROFILE[a.pm_precision],
-                   "issue_active_ncu": ({"propagation": 0.605, "trials": 0.406} if a.pm_precision == "fp32"
-                                        else 0.667),
-                   "note": "not a contraction and not HBM-bound (DRAM < 2 %): propagation is bound by SIMT "
-                           "issue, the trials by latency at low occupancy; issue_active is the fraction of SM "
-                           "issue slots used (ncu, see ncu_profile)"}
+                   "issue_active_ncu": PM_ISSUE_ACTIVE[a.pm_precision],
+                   "note": "not a contraction and not HBM-bound (DRAM < 2 %); issue_active_ncu is the fraction "
+                           "of the SM issue slots used (one launch of a colour pass at 1000 x 750, 8 sources, "
+                           "7 x 7)"}
     # the cost of the precision forms of the sweep, each timed once after the timed region on the
     # same view: compensated FP32 sums (config 3's form; FP16 sources), and the reference's float64
     # window sums
@@ -626,7 +629,7 @@ def cpu_baseline(cfg, nplanes, iters, device="cpu"):
 CHECK_ROWS = 64        # rows of the timed step's sweep that --check validates
 # thread instructions per evaluation of the FP32 plane sweep, sources outside a tile skipped and
 # samples in packed pairs (smsp__thread_inst_executed.sum of one launch at 3000 x 2250, 8 sources,
-# r = 3, 16 planes; profiles/sweep_kernel_3000x2250_8src_16planes.md)
+# r = 3, 16 planes)
 SWEEP_INST_PER_EVAL = 72.3
 
 

@@ -138,7 +138,9 @@ mvs_status mvs_sweep_noalloc(const mvs_sweep_args* args, void* stream);
 
 /* mvs_sweep with its plane-chunk scratch given by the caller (256-byte aligned device memory, free
  * to be used again by work that follows on `stream`): a host process with a caching allocator saves
- * the driver's allocation per call. mvs_sweep_scratch_bytes: the bytes these arguments need on the
+ * the driver's allocation per call. The scratch is 24 bytes per pixel and chunk; the automatic number
+ * of chunks keeps it within about 300 MB, and mvs_sweep, when it cannot have that, runs in one chunk,
+ * which needs none. mvs_sweep_scratch_bytes: the bytes these arguments need on the
  * current device (0: none, also for arguments that mvs_sweep rejects); fewer give MVS_ERR_VALUE. */
 size_t mvs_sweep_scratch_bytes(const mvs_sweep_args* args);
 /* The initial winner-take-all state (densify.py:331-335): -2 in the four score planes, idx -1. */

@@ -508,11 +508,14 @@ __device__ double pm_cost(const PMParams& c, const PMPix& px, const PMCorners& c
     return (1.0 - photo) + gterm;
 }
 
-// Resident blocks of 128 threads per SM. Propagation + trials of a 1600 x 1200 repair (4 sources, 5 x 5
-// samples, a third of the pixels active, geometric term) / of 5 views of 800 x 600 (ms): 2 sources a
-// pass with 5 blocks (96 registers) 8.0 / 24.7, 6 blocks 8.3 / 26.1, 8 blocks 7.7 / 27.2; 4 sources a
-// pass with 5 blocks 11.5 / 37.7 (spills), 4 blocks 12.5 / 38.7. One thread per pixel, all windows
-// and tests, three divisions a sample: 36.0 / 54.2.
+// Resident blocks of 128 threads per SM, 2 sources a pass (4 sources a pass spilled: 11.5 against 8.0 ms
+// with one thread walking a pixel's candidates). All of a call's launches with a lane per candidate, ms,
+// at 4 / 5 / 6 / 8 blocks (128 / 96 / 80 / 64 registers): a 1600 x 1200 repair (4 sources, 5 x 5 samples, a
+// third of the pixels active, geometric term) 6.07 / 6.23 / 6.27 / 5.84, 5 views of 800 x 600 15.7 / 16.6 /
+// 17.4 / 17.9, 2000 x 1500 with 8 sources, 7 x 7 samples and every pixel active 117.5 / 119.6 / 117.8 /
+// 116.3, 320 x 240 1.62 / 1.78 / 1.85 / 1.91: within 2 % on large views, where fewer registers pay for more
+// warps, and fewer blocks better by up to 9 % on small ones, whose pixels do not fill the chip; 5 lies
+// between. One thread per pixel, all windows and tests, three divisions a sample: 36.0 and 54.2 on the first two.
 constexpr int PM_MIN_BLOCKS = 5;
 
 // Pixel of pass number t (raster order of the colour's pixels): false past the image.
@@ -908,13 +911,13 @@ __global__ void __launch_bounds__(256) pm_quad_kernel(const float* __restrict__ 
 //   * the lanes of a pixel sort their NCCs with a shuffle network (top-k mean) and sum the
 //     geometric term; every lane follows the same candidate sequence and decision.
 // Float32 costs differ from the float64 ones by ~1e-7 (measured 99.9th percentile 2e-6), so the
-// strict '<' can decide near-ties differently; the float64 mode is the bit-exact reference.
+// strict '<' can decide near-ties differently; the float64 mode decides them as the reference does.
 
 // Resident blocks of 256 threads per SM for the lane kernel (propagation; trials). Propagation of 4
 // iterations at 4000 x 3000, 8 sources, 7 x 7: 252 ms with single samples at 5 blocks (48 registers), in
 // pairs of a row 239 ms at 5, 232 ms at 4 (64 registers), 248 ms at 3, in pairs of the whole window and
-// with a shorter unit set-up 217 ms at 4. What bounds it is latency at that occupancy: issue slots alone
-// would take ~100 ms, the footprints' L1 wavefronts ~50 ms.
+// with a shorter unit set-up 217 ms at 4. What bounds it is latency at that occupancy: 60 % of the issue
+// slots are used (~130 of the 217 ms), stalls are led by the footprint loads.
 constexpr int PM_LANE_MIN_BLOCKS = 4;
 
 __device__ __forceinline__ int pmf_floor(float x, float& f) {   // |x| < 2^22
